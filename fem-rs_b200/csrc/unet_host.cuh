@@ -17,6 +17,7 @@
 
 #include "unet_kernels.cuh"
 #include "unet_tc.cuh"
+#include "unet_wgrad.cuh"
 
 namespace fg {
 
@@ -284,35 +285,82 @@ static int unet_forward(fg_unet *u) {
     return FG_OK;
 }
 
-// gradient of one layer: weights/bias from (in, dy); optional input gradient din
-static int layer_bwd(fg_unet *u, int li, const TView &in, const Vol &V, const TView &dy, TView *din) {
+// input gradient of one layer: the convolution of dy with the flipped weights
+static int layer_dgrad(fg_unet *u, int li, const Vol &V, const TView &dy, const TView &din) {
     ConvLayer &l = u->L[li];
+    const size_t nf = (size_t)l.cin * l.kpt;
+    if (nf > u->wflip_n) {
+        if (u->wflip) cudaFree(u->wflip);
+        CK(cudaMalloc(&u->wflip, nf * sizeof(__nv_bfloat16)));
+        u->wflip_n = nf;
+    }
+    flip_weights_kernel<<<64, 256, 0, u->stream>>>(l.wb, l.cout, l.cin, l.kp, u->wflip, l.kpt);
+    return conv_fwd(u, l, dy, V, u->wflip, l.cout, l.cin, l.kpt, nullptr, din, 0);
+}
+
+// Weight and bias gradients of all layers (one launch and its reduction), after
+// the input gradients: every layer's input and output gradient stay in their
+// buffers until the next pass.
+struct WgItem {
+    int li;
+    TView in, dy;
+    Vol V;
+};
+static int unet_wgrad(fg_unet *u, const WgItem *items, int n) {
     UnetBufs &b = u->buf;
-    const int64_t nv = V.nvox();
-    const int chunk = 4096;
-    const int nchunks = (int)((nv + chunk - 1) / chunk);
-    const size_t need = (size_t)nchunks * l.cout * l.kp;
-    if (need > b.part_n) {
+    WgArgs A{};
+    A.n = n;
+    double work[WG_MAXL], sum = 0.0;
+    int smem = 0;
+    for (int k = 0; k < n; ++k) {
+        WgLayer &L = A.L[k];
+        const ConvLayer &l = u->L[items[k].li];
+        L.in = items[k].in;
+        L.dy = items[k].dy;
+        L.V = items[k].V;
+        L.cin = l.cin;
+        L.cout = l.cout;
+        L.kp = l.kp;
+        L.gw = l.gw;
+        L.gb = l.gb;
+        // patches of at most WG_TILE voxels, as wide in x as the volume allows up to 36
+        L.ntx = (L.V.X + 35) / 36;
+        L.TX = (L.V.X + L.ntx - 1) / L.ntx;
+        L.TY = std::max(1, std::min(L.V.Y, WG_TILE / L.TX));
+        L.nty = (L.V.Y + L.TY - 1) / L.TY;
+        L.ntiles = L.V.B * L.V.Z * L.nty * L.ntx;
+        const int nt = 9 * wg_c8(l.cin);
+        L.groups = (nt + 8 * WG_NPW - 1) / (8 * WG_NPW);
+        L.tpg = (nt + L.groups - 1) / L.groups;
+        smem = std::max(smem, 2 * 16 * wg_stage_units(L));
+        work[k] = (double)L.ntiles * (2 + nt / 8 * wg_co16(l.cout));
+        sum += work[k];
+    }
+    // voxel splits: two waves' worth of blocks over all layers, in proportion to their work
+    int64_t blocks = 0, part = 0, red = 0;
+    for (int k = 0; k < n; ++k) {
+        WgLayer &L = A.L[k];
+        const double want = 148.0 * 4 * work[k] / sum / (3 * L.groups);
+        L.splits = std::max(1, std::min(L.ntiles, (int)(want + 0.5)));
+        L.blk0 = (int)blocks;
+        L.part0 = part;
+        L.red0 = (int)red;
+        blocks += (int64_t)L.splits * 3 * L.groups;
+        part += (int64_t)L.splits * L.cout * (27 * L.cin + 1);
+        red += (int64_t)L.cout * (27 * L.cin + 1);
+    }
+    if ((size_t)part > b.part_n) {
         if (b.part) cudaFree(b.part);
-        CK(cudaMalloc(&b.part, need * sizeof(float)));
-        b.part_n = need;
+        b.part = nullptr;
+        b.part_n = 0;
+        CK(cudaMalloc(&b.part, part * sizeof(float)));
+        b.part_n = part;
     }
-    dim3 g((l.kp + 31) / 32, nchunks);
-    conv3_wgrad_kernel<<<g, 128, 0, u->stream>>>(in, V, l.cin, dy, l.cout, l.kp, chunk, b.part);
-    conv3_wgrad_reduce<<<64, 256, 0, u->stream>>>(b.part, nchunks, l.cout * l.kp, l.gw);
-    bias_grad_kernel<<<l.cout, 256, 0, u->stream>>>(dy, nv, l.gb);
+    A.part = b.part;
+    CK(cudaFuncSetAttribute(conv3_wgrad_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    conv3_wgrad_all_kernel<<<(unsigned)blocks, WG_THREADS, smem, u->stream>>>(A);
+    conv3_wgrad_all_reduce<<<(unsigned)((red + 255) / 256), 256, 0, u->stream>>>(A, (int)red);
     CK(cudaGetLastError());
-    if (din) {
-        const size_t nf = (size_t)l.cin * l.kpt;
-        if (nf > u->wflip_n) {
-            if (u->wflip) cudaFree(u->wflip);
-            CK(cudaMalloc(&u->wflip, nf * sizeof(__nv_bfloat16)));
-            u->wflip_n = nf;
-        }
-        flip_weights_kernel<<<64, 256, 0, u->stream>>>(l.wb, l.cout, l.cin, l.kp, u->wflip, l.kpt);
-        int rc = conv_fwd(u, l, dy, V, u->wflip, l.cout, l.cin, l.kpt, nullptr, *din, 0);
-        if (rc) return rc;
-    }
     return FG_OK;
 }
 
@@ -336,29 +384,30 @@ static int unet_backward(fg_unet *u) {
         dh0{b.dcat0, C1 + C0, C1}, dg1{b.dg1, C1, 0}, dcat1{b.dcat1, C2 + C1, 0}, dup1{b.dcat1, C2 + C1, 0},
         dh1{b.dcat1, C2 + C1, C2}, dh2{b.dh2, C2, 0}, da2{b.da2, C2, 0}, dx2{b.dx2, C1, 0},
         da1{b.da1, C1, 0}, dx1{b.dx1, C0, 0}, da0{b.da0, C0, 0};
-    if ((rc = layer_bwd(u, LOUT, g0, b.v0, dout, &dg0))) return rc;
+    if ((rc = layer_dgrad(u, LOUT, b.v0, dout, dg0))) return rc;
     if ((rc = relu_bwd(u, dg0, g0, b.v0, C0))) return rc;
-    if ((rc = layer_bwd(u, L0C, cat0, b.v0, dg0, &dcat0))) return rc;
+    if ((rc = layer_dgrad(u, L0C, b.v0, dg0, dcat0))) return rc;
     // P^T = 8 R : gradient of the level-1 output g1 from the prolongated channels
     launch_restrict(u, dup0, b.v0, dg1, b.v1, C1, 8.f);
     if ((rc = relu_bwd(u, dg1, g1, b.v1, C1))) return rc;
-    if ((rc = layer_bwd(u, L1C, cat1, b.v1, dg1, &dcat1))) return rc;
+    if ((rc = layer_dgrad(u, L1C, b.v1, dg1, dcat1))) return rc;
     launch_restrict(u, dup1, b.v1, dh2, b.v2, C2, 8.f);
     if ((rc = relu_bwd(u, dh2, h2, b.v2, C2))) return rc;
-    if ((rc = layer_bwd(u, L2B, a2, b.v2, dh2, &da2))) return rc;
+    if ((rc = layer_dgrad(u, L2B, b.v2, dh2, da2))) return rc;
     if ((rc = relu_bwd(u, da2, a2, b.v2, C2))) return rc;
-    if ((rc = layer_bwd(u, L2A, x2, b.v2, da2, &dx2))) return rc;
+    if ((rc = layer_dgrad(u, L2A, b.v2, da2, dx2))) return rc;
     // R^T = P / 8 : add the down-path gradient to the skip gradient of h1
     launch_prolong(u, dx2, b.v2, dh1, b.v1, C1, 0.125f, 1);
     if ((rc = relu_bwd(u, dh1, h1, b.v1, C1))) return rc;
-    if ((rc = layer_bwd(u, L1B, a1, b.v1, dh1, &da1))) return rc;
+    if ((rc = layer_dgrad(u, L1B, b.v1, dh1, da1))) return rc;
     if ((rc = relu_bwd(u, da1, a1, b.v1, C1))) return rc;
-    if ((rc = layer_bwd(u, L1A, x1, b.v1, da1, &dx1))) return rc;
+    if ((rc = layer_dgrad(u, L1A, b.v1, da1, dx1))) return rc;
     launch_prolong(u, dx1, b.v1, dh0, b.v0, C0, 0.125f, 1);
     if ((rc = relu_bwd(u, dh0, h0, b.v0, C0))) return rc;
-    if ((rc = layer_bwd(u, L0B, a0, b.v0, dh0, &da0))) return rc;
+    if ((rc = layer_dgrad(u, L0B, b.v0, dh0, da0))) return rc;
     if ((rc = relu_bwd(u, da0, a0, b.v0, C0))) return rc;
-    if ((rc = layer_bwd(u, L0A, x0, b.v0, da0, nullptr))) return rc;
+    const WgItem items[] = {{LOUT, g0, dout, b.v0}, {L0C, cat0, dg0, b.v0}, {L1C, cat1, dg1, b.v1}, {L2B, a2, dh2, b.v2}, {L2A, x2, da2, b.v2}, {L1B, a1, dh1, b.v1}, {L1A, x1, da1, b.v1}, {L0B, a0, dh0, b.v0}, {L0A, x0, da0, b.v0}};
+    if ((rc = unet_wgrad(u, items, NLAYERS))) return rc;
     CK(cudaGetLastError());
     return FG_OK;
 }

@@ -15,9 +15,7 @@
 // kernel applied to the output gradient with the flipped, transposed weights
 // W'[ci][tap][co] = W[co][26-tap][ci].
 //
-// conv3_wgrad_kernel: dW[co][k] = sum_v dY[v][co] A[v][k] as a GEMM with the
-// voxel dimension as K, split over voxel chunks; chunk partials are summed in
-// chunk order by conv3_wgrad_reduce (deterministic, no atomics).
+// The weight and bias gradients are in unet_wgrad.cuh.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -254,113 +252,6 @@ __global__ void __launch_bounds__(128) conv3_fwd16_kernel(const TView in, const 
         if (ok1)
             *reinterpret_cast<__nv_bfloat162 *>(out.p + v1 * out.cs + out.co + n) = __floats2bfloat162_rn(r2, r3);
     }
-}
-
-// Weight gradient partials: block (n-block of 32 columns, voxel chunk), warp =
-// m-tile of 16 output channels.  part[chunk][co][Kp] (FP32).
-__global__ void __launch_bounds__(128) conv3_wgrad_kernel(const TView in, const Vol V, int Cin,
-                                                          const TView dy, int Cout, int Kp, int chunk,
-                                                          float *__restrict__ part) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gid = lane >> 2, t4 = lane & 3;
-    const int K = 27 * Cin;
-    const int nb0 = blockIdx.x * 32;
-    const int mt = warp;  // 16 output channels per warp
-    if (mt * 16 >= Cout) return;
-    const int64_t nv = V.nvox();
-    const int64_t vbeg = (int64_t)blockIdx.y * chunk, vend = min(nv, vbeg + chunk);
-    float acc[4][4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    const int co0 = mt * 16 + gid, co1 = co0 + 8;
-    for (int64_t vs = vbeg; vs < vend; vs += 16) {
-        // A (16 co x 16 voxels): a0 = (co0, v = vs + 2 t4 + {0,1}), a1 = (co1, ...), a2/a3: voxels + 8
-        uint32_t a[4];
-        __nv_bfloat16 e[8];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int64_t v = vs + t4 * 2 + q + h * 8;
-                const bool ok = v < vend;
-                e[h * 4 + q] = (ok && co0 < Cout) ? dy.p[v * dy.cs + dy.co + co0] : __float2bfloat16(0.f);
-                e[h * 4 + 2 + q] = (ok && co1 < Cout) ? dy.p[v * dy.cs + dy.co + co1] : __float2bfloat16(0.f);
-            }
-        a[0] = (uint32_t)__bfloat16_as_ushort(e[0]) | ((uint32_t)__bfloat16_as_ushort(e[1]) << 16);
-        a[1] = (uint32_t)__bfloat16_as_ushort(e[2]) | ((uint32_t)__bfloat16_as_ushort(e[3]) << 16);
-        a[2] = (uint32_t)__bfloat16_as_ushort(e[4]) | ((uint32_t)__bfloat16_as_ushort(e[5]) << 16);
-        a[3] = (uint32_t)__bfloat16_as_ushort(e[6]) | ((uint32_t)__bfloat16_as_ushort(e[7]) << 16);
-        // B (16 voxels x 8 columns): b = (k = voxel vs + 2 t4 + {0,1} (+8), n = column nb + gid)
-        int vb[4], vz[4], vyy[4], vx[4];
-        bool vok[4];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int64_t v = vs + t4 * 2 + q + h * 8;
-                vok[h * 2 + q] = v < vend;
-                vox_coords(V, v < vend ? v : vbeg, vb[h * 2 + q], vz[h * 2 + q], vyy[h * 2 + q], vx[h * 2 + q]);
-            }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const KCol c = kcol(nb0 + j * 8 + gid, Cin, K);
-            uint16_t bv[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                __nv_bfloat16 val = __float2bfloat16(0.f);
-                if (vok[u] && c.ok) {
-                    const int zz = vz[u] + c.dz, yy = vyy[u] + c.dy, xx = vx[u] + c.dx;
-                    if (zz >= 0 && zz < V.Z && yy >= 0 && yy < V.Y && xx >= 0 && xx < V.X) {
-                        const int64_t vv = (((int64_t)vb[u] * V.Z + zz) * V.Y + yy) * V.X + xx;
-                        val = in.p[vv * in.cs + in.co + c.ci];
-                    }
-                }
-                bv[u] = __bfloat16_as_ushort(val);
-            }
-            const uint32_t b0 = (uint32_t)bv[0] | ((uint32_t)bv[1] << 16);
-            const uint32_t b1 = (uint32_t)bv[2] | ((uint32_t)bv[3] << 16);
-            mma_bf16_16816(acc[j], a, b0, b1);
-        }
-    }
-    float *pp = part + (int64_t)blockIdx.y * Cout * Kp;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int n = nb0 + j * 8 + t4 * 2;
-        if (n >= Kp) continue;
-        if (co0 < Cout) {
-            pp[(int64_t)co0 * Kp + n] = acc[j][0];
-            pp[(int64_t)co0 * Kp + n + 1] = acc[j][1];
-        }
-        if (co1 < Cout) {
-            pp[(int64_t)co1 * Kp + n] = acc[j][2];
-            pp[(int64_t)co1 * Kp + n + 1] = acc[j][3];
-        }
-    }
-}
-
-// dW[i] = sum_c part[c][i] in chunk order; db[co] = sum over voxels of dy (fixed order)
-__global__ void conv3_wgrad_reduce(const float *__restrict__ part, int nchunks, int n,
-                                   float *__restrict__ dw) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int c = 0; c < nchunks; ++c) s += part[(int64_t)c * n + i];
-        dw[i] = s;
-    }
-}
-
-// bias gradient: one block per output channel, fixed-order tree over voxels
-__global__ void __launch_bounds__(256) bias_grad_kernel(const TView dy, int64_t nv, float *__restrict__ db) {
-    __shared__ float sm[256];
-    const int co = blockIdx.x;
-    float s = 0.f;
-    for (int64_t v = threadIdx.x; v < nv; v += 256) s += __bfloat162float(dy.p[v * dy.cs + dy.co + co]);
-    sm[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) db[co] = sm[0];
 }
 
 // W'[ci][tap][co] = W[co][26 - tap][ci]  (input-gradient weights), padded rows

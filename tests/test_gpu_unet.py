@@ -59,6 +59,37 @@ def test_gradients_match_reference():
         o += nw + co
 
 
+@pytest.mark.parametrize("channels,shape", [
+    ((16, 32, 48), (1, 5, 5, 5)),      # a patch smaller than one k16 step per row, one-voxel-wide coarsest level
+    ((16, 32, 48), (1, 5, 5, 37)),     # two x patches, the second ragged
+    ((8, 8, 8), (2, 5, 13, 41)),       # 8-channel layers (half an m-tile), ragged y patches, two samples
+    ((16, 64, 16), (1, 9, 5, 9)),      # 64 output channels, four m-tiles
+])
+def test_weight_gradients_at_patch_edges(channels, shape):
+    """The weight and bias gradients of every layer at the patch and tile
+    edges of their kernel, against the NumPy reference with the bound of the
+    other gradient tests (BF16 storage): 5e-2 per layer.  Run twice: the sums
+    are in a fixed order, so the bits repeat."""
+    need_gpu()
+    net = femgpu.UNet(channels=channels, seed=13)
+    rng = np.random.default_rng(3)
+    inp = rng.standard_normal(shape + (2,)).astype(np.float32)
+    tgt = rng.standard_normal(shape).astype(np.float32)
+    net.loss_grad(inp, tgt)
+    g = net.get_grads()
+    net.loss_grad(inp, tgt)
+    assert np.array_equal(g, net.get_grads())
+    _, g_ref = R.loss_grad(net.get_params(), inp, tgt, channels)
+    c0, c1, c2 = channels
+    shapes = [(2, c0), (c0, c0), (c0, c1), (c1, c1), (c1, c2), (c2, c2), (c2 + c1, c1), (c1 + c0, c0), (c0, 8)]
+    o = 0
+    for li, (ci, co) in enumerate(shapes):
+        nw = co * 27 * ci
+        for part, sl in (("W", slice(o, o + nw)), ("b", slice(o + nw, o + nw + co))):
+            assert rel(g[sl], g_ref[sl]) <= 5e-2, (li, part, rel(g[sl], g_ref[sl]))
+        o += nw + co
+
+
 def test_training_reduces_loss():
     need_gpu()
     net = femgpu.UNet(seed=7)
