@@ -2038,6 +2038,36 @@ static std::vector<int2> largest_first_bmap(fg_op *const *ops, const std::vector
 
 static const int kTuneTZ[FG_TUNE_CANDIDATES] = {1, 2, 4, 8, 16};
 
+// Blocks of the batched fix-up: the shared-face rows of all instances, as many
+// per block as keep the launch at about 64 blocks per SM.
+static std::vector<FixBlk> fix_blocks(const std::vector<Grid> &g) {
+    int64_t total = 0;
+    for (const Grid &q : g) total += fixup_rows(q);
+    const int per = (int)std::max<int64_t>(1, (total + 148 * 64 - 1) / (148 * 64));
+    std::vector<FixBlk> m;
+    for (size_t i = 0; i < g.size(); ++i) {
+        const int rows = fixup_rows(g[i]);
+        for (int r = 0; r < rows; r += per) m.push_back(FixBlk{(int)i, r, std::min(per, rows - r)});
+    }
+    return m;
+}
+
+// Blocks of the batched vector kernels: about 16 per SM over all instances, in
+// proportion to their lengths (at least one, at most one per 256 groups of
+// four); first[i]: the first block of instance i.
+static std::vector<BatchBlk> vec_blocks(const std::vector<int64_t> &n, std::vector<int> &first) {
+    double total = 0.0;
+    for (int64_t v : n) total += (double)v;
+    std::vector<BatchBlk> m;
+    for (size_t i = 0; i < n.size(); ++i) {
+        const int most = (int)std::max<int64_t>(1, (n[i] / 4 + VEC_THREADS - 1) / VEC_THREADS);
+        const int nb = std::max(1, std::min(most, (int)(148.0 * 16.0 * (double)n[i] / total + 0.5)));
+        first.push_back((int)m.size());
+        for (int b = 0; b < nb; ++b) m.push_back(BatchBlk{(int)i, b, nb});
+    }
+    return m;
+}
+
 // time `reps` batched FP32 applies (apply + fix-up) of the instances `inst`
 // in their current tile shapes; microseconds per apply
 static int time_batched_apply(fg_op *const *ops, const std::vector<int> &inst, cudaStream_t bs, int reps,
@@ -2066,24 +2096,27 @@ static int time_batched_apply(fg_op *const *ops, const std::vector<int> &inst, c
     ApplyArgs<float> *d_a = nullptr;
     CUtensorMap *d_t = nullptr;
     FixArgs<float> *d_f = nullptr;
+    std::vector<Grid> fg(k);
+    for (int j = 0; j < k; ++j) fg[j] = f[j].g;
+    const std::vector<FixBlk> fm = fix_blocks(fg);
+    FixBlk *d_fm = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     auto cleanup = [&]() {
-        void *ptrs[] = {G.bmap, d_a, d_t, d_f};
+        void *ptrs[] = {G.bmap, d_a, d_t, d_f, d_fm};
         for (void *q : ptrs) if (q) cudaFree(q);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
     };
     struct Guard { std::function<void()> f; ~Guard() { f(); } } guard{cleanup};
     if ((rc = dev_upload(&G.bmap, m)) || (rc = dev_upload(&d_a, a)) || (rc = dev_upload(&d_t, t)) ||
-        (rc = dev_upload(&d_f, f)))
+        (rc = dev_upload(&d_f, f)) || (rc = dev_upload(&d_fm, fm)))
         return rc;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    const dim3 fgrid(64, k);
     auto once = [&]() -> int {
         int r2 = launch_batched<float>(bs, G, d_a, d_t, 1, 0);
         if (r2) return r2;
-        fixup_batched_kernel<float><<<fgrid, 128, 0, bs>>>(d_f, 1, 0);
+        if (!fm.empty()) fixup_batched_kernel<float><<<(unsigned)fm.size(), 128, 0, bs>>>(d_f, d_fm, 1, 0);
         CK(cudaGetLastError());
         return FG_OK;
     };
@@ -2315,7 +2348,6 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
     cudaStream_t bs;
     CK(cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking));
     // device tables
-    constexpr int VBX = 64;
     std::vector<ApplyArgs<float>> a32(2 * n);
     std::vector<ApplyArgs<double>> a64(n);
     std::vector<CUtensorMap> t32(2 * n), t64(n);
@@ -2325,7 +2357,16 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
     SolverState *d_st = nullptr;
     double *d_part = nullptr;
     CK(cudaMalloc(&d_st, sizeof(SolverState) * n));
-    CK(cudaMalloc(&d_part, sizeof(double) * 2 * VBX * n));
+    std::vector<int64_t> len(n);
+    std::vector<Grid> fgs(n);
+    for (int i = 0; i < n; ++i) {
+        len[i] = ops[i]->Nn;
+        fgs[i] = ops[i]->g;
+    }
+    std::vector<int> vfirst;
+    const std::vector<BatchBlk> vmap = vec_blocks(len, vfirst);
+    const std::vector<FixBlk> fmap = fix_blocks(fgs);
+    CK(cudaMalloc(&d_part, sizeof(double) * 2 * vmap.size()));
     std::vector<SolverState> hst(n);
     for (int i = 0; i < n; ++i) {
         fg_op *o = ops[i];
@@ -2348,7 +2389,7 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
         B.x64 = o->xw; B.b64 = o->bw; B.ap64 = o->ap;
         B.r = o->r32; B.z = o->z32; B.p = o->p32; B.ap = o->ap32; B.e = o->e32;
         B.cres = o->cres32; B.cd = o->cd32; B.ct = o->ct32; B.dinv = o->dinv32;
-        B.partials = d_part + (size_t)2 * VBX * i;
+        B.partials = d_part + (size_t)2 * vfirst[i];
         B.st = &d_st[i];
         if (cheb) {
             const ChebCoef cc = cheb_coefs(lmax[i] / (cfg.lmin_ratio > 0 ? cfg.lmin_ratio : 30.0), lmax[i],
@@ -2378,13 +2419,15 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
     FixArgs<float> *d_f32 = nullptr;
     FixArgs<double> *d_f64 = nullptr;
     BatchVec *d_bv = nullptr;
+    BatchBlk *d_vm = nullptr;
+    FixBlk *d_fm = nullptr;
     cudaGraphExec_t gexec = nullptr;
     cudaGraph_t graph = nullptr;
     auto cleanup = [&]() {
         if (gexec) cudaGraphExecDestroy(gexec);
         if (graph) cudaGraphDestroy(graph);
         for (auto &G : groups) if (G.bmap) cudaFree(G.bmap);
-        void *ptrs[] = {d_a32, d_a64, d_t32, d_t64, d_f32, d_f64, d_bv, d_st, d_part};
+        void *ptrs[] = {d_a32, d_a64, d_t32, d_t64, d_f32, d_f64, d_bv, d_st, d_part, d_vm, d_fm};
         for (void *p : ptrs) if (p) cudaFree(p);
         cudaStreamDestroy(bs);
     };
@@ -2396,17 +2439,17 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
     }
     if ((rc = dev_upload(&d_a32, a32)) || (rc = dev_upload(&d_a64, a64)) || (rc = dev_upload(&d_t32, t32)) ||
         (rc = dev_upload(&d_t64, t64)) || (rc = dev_upload(&d_f32, f32)) || (rc = dev_upload(&d_f64, f64)) ||
-        (rc = dev_upload(&d_bv, bv)))
+        (rc = dev_upload(&d_bv, bv)) || (rc = dev_upload(&d_vm, vmap)) || (rc = dev_upload(&d_fm, fmap)))
         return rc;
     CK(cudaMemcpy(d_st, hst.data(), sizeof(SolverState) * n, cudaMemcpyHostToDevice));
     FG_LEGACY_FENCE();
-    const dim3 vgrid(VBX, n), fgrid(64, n);
+    const unsigned vgrid = (unsigned)vmap.size(), fgrid = (unsigned)fmap.size();
     auto apply32 = [&](int slot) -> int {
         for (auto &G : groups) {
             int r2 = launch_batched<float>(bs, G, d_a32, d_t32, 2, slot);
             if (r2) return r2;
         }
-        fixup_batched_kernel<float><<<fgrid, 128, 0, bs>>>(d_f32, 2, slot);
+        if (fgrid) fixup_batched_kernel<float><<<fgrid, 128, 0, bs>>>(d_f32, d_fm, 2, slot);
         CK(cudaGetLastError());
         return FG_OK;
     };
@@ -2415,23 +2458,23 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
             int r2 = launch_batched<double>(bs, G, d_a64, d_t64, 1, 0);
             if (r2) return r2;
         }
-        fixup_batched_kernel<double><<<fgrid, 128, 0, bs>>>(d_f64, 1, 0);
+        if (fgrid) fixup_batched_kernel<double><<<fgrid, 128, 0, bs>>>(d_f64, d_fm, 1, 0);
         CK(cudaGetLastError());
         return FG_OK;
     };
     auto precond = [&](int init) -> int {
         if (cheb) {
-            kb_cheb_first<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv);
+            kb_cheb_first<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm);
             for (int sidx = 0; sidx + 1 < cfg.cheb_degree; ++sidx) {
                 int r2 = apply32(1);
                 if (r2) return r2;
-                kb_cheb_step<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, sidx, sidx + 2 == cfg.cheb_degree ? 1 : 0);
+                kb_cheb_step<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm, sidx, sidx + 2 == cfg.cheb_degree ? 1 : 0);
             }
-            kb_rz<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, init, 0);
+            kb_rz<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm, init, 0);
         } else {
-            kb_rz<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, init, 1);
+            kb_rz<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm, init, 1);
         }
-        kb_pupdate<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, init);
+        kb_pupdate<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm, init);
         CK(cudaGetLastError());
         return FG_OK;
     };
@@ -2443,20 +2486,20 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     CK(cudaEventRecord(e0, bs));
-    kb_zero_e<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv);
+    kb_zero_e<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm);
     if ((rc = apply64())) return rc;
-    kb_rel_residual<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, 1);
+    kb_rel_residual<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm, 1);
     if ((rc = precond(1))) return rc;
     // one chunk of iterations, captured once and replayed
     const int chunk = std::max(1, cfg.check_interval);
     CK(cudaStreamBeginCapture(bs, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < chunk; ++k) {
         if ((rc = apply32(0))) { cudaStreamEndCapture(bs, &graph); return rc; }
-        kb_pap<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv);
-        kb_rel_step<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv);
-        kb_rel_xupdate<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv);
+        kb_pap<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm);
+        kb_rel_step<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm);
+        kb_rel_xupdate<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm);
         if ((rc = apply64())) { cudaStreamEndCapture(bs, &graph); return rc; }
-        kb_rel_residual<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, 0);
+        kb_rel_residual<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm, 0);
         if ((rc = precond(0))) { cudaStreamEndCapture(bs, &graph); return rc; }
     }
     CK(cudaStreamEndCapture(bs, &graph));
@@ -2477,7 +2520,7 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
     for (int i = 0; i < n; ++i)
         CK(cudaMemcpyAsync(&d_st[i].skip_rel, &hst[i].skip_rel, sizeof(int), cudaMemcpyHostToDevice, bs));
     if ((rc = apply64())) return rc;
-    kb_true_residual<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv);
+    kb_true_residual<<<vgrid, VEC_THREADS, 0, bs>>>(d_bv, d_vm);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(hst.data(), d_st, sizeof(SolverState) * n, cudaMemcpyDeviceToHost, bs));
     CK(cudaStreamSynchronize(bs));

@@ -1512,21 +1512,26 @@ __global__ void __launch_bounds__(128) fixup_range_kernel(const Grid g, T *__res
     fixup_row<T>(g, r, y, face);
 }
 
-// Batched fix-up: blockIdx.y = instance; blocks stride over the instance's
-// rows of shared-face DOFs.
+// Batched fix-up: block b works on the rows [row0, row0 + nrows) of instance
+// inst, as the map says.  The map cuts all instances' rows into about equal
+// blocks (fix_blocks): with 64 blocks for every instance (the form before) the
+// one with 3,600 rows set the time of the launch, 135 us against 9 us.
 template <typename T> struct FixArgs {
     Grid g;
     T *y;
     const T *face;
     const int *skip;
 };
+struct FixBlk {
+    int inst, row0, nrows;
+};
 template <typename T>
-__global__ void __launch_bounds__(128) fixup_batched_kernel(const FixArgs<T> *args, int nslots,
+__global__ void __launch_bounds__(128) fixup_batched_kernel(const FixArgs<T> *args, const FixBlk *map, int nslots,
                                                             int slot) {
-    const FixArgs<T> &A = args[blockIdx.y * nslots + slot];
+    const FixBlk m = map[blockIdx.x];
+    const FixArgs<T> &A = args[m.inst * nslots + slot];
     if (A.skip && *A.skip) return;
-    const int rows = fixup_rows(A.g);
-    for (int r = blockIdx.x; r < rows; r += gridDim.x) fixup_row<T>(A.g, r, A.y, A.face);
+    for (int r = m.row0; r < m.row0 + m.nrows; ++r) fixup_row<T>(A.g, r, A.y, A.face);
 }
 
 // ---------------------------------------------------------------------------

@@ -56,20 +56,21 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *sm) {
     __syncthreads();
 }
 
-// Writes this block's partials; returns true in the last block, whose thread 0
-// then holds the grand totals in `tot` (summed in block order).
+// Writes this block's partials; returns true in the last of the sum's nb
+// blocks, whose thread 0 then holds the grand totals in `tot` (summed in block
+// order).  bid: this block's place among them.
 template <int NV>
 __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, SolverState *st,
-                                         double (&tot)[NV]) {
+                                         double (&tot)[NV], int bid, int nb) {
     __shared__ double sm[NV * (VEC_THREADS / 32)];
     __shared__ int last;
     block_sum<NV>(v, sm);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int k = 0; k < NV; ++k) partials[blockIdx.x * NV + k] = v[k];
+        for (int k = 0; k < NV; ++k) partials[bid * NV + k] = v[k];
         __threadfence();
         const unsigned t = atomicAdd(&st->ticket, 1u);
-        last = (t == gridDim.x - 1);
+        last = (t == (unsigned)nb - 1);
     }
     __syncthreads();
     if (!last) return false;
@@ -78,7 +79,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, Solv
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] = 0.0;
     // fixed order: thread i sums blocks i, i+256, ... then a fixed tree
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += VEC_THREADS)
+    for (int b = threadIdx.x; b < nb; b += VEC_THREADS)
 #pragma unroll
         for (int k = 0; k < NV; ++k) acc[k] += __ldcg(&partials[b * NV + k]);
     block_sum<NV>(acc, sm);
@@ -88,6 +89,11 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, Solv
         st->ticket = 0;
     }
     return true;
+}
+
+template <int NV>
+__device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, SolverState *st, double (&tot)[NV]) {
+    return grid_sum<NV>(v, partials, st, tot, (int)blockIdx.x, (int)gridDim.x);
 }
 
 #define FG_VEC_LOOP(i, n) \
@@ -832,17 +838,30 @@ struct BatchVec {
     double c1[BATCH_MAXK], c2[BATCH_MAXK];
 };
 
-__global__ void __launch_bounds__(VEC_THREADS) kb_pap(const BatchVec *bv) {
-    const BatchVec &B = bv[blockIdx.y];
+// One block of a batched vector kernel: the instance it works on, its place
+// among that instance's blocks and their number.  An instance gets blocks in
+// proportion to its length: with the same 64 for every instance (the form
+// before), the largest of 16 uneven ones (3M DOFs) set the time of each launch,
+// 42 us for a sweep that takes 9 us of bandwidth.
+struct BatchBlk {
+    int inst, bid, nb;
+};
+#define FG_BVEC4_LOOP(q, n)                                                                \
+    for (int64_t q = (int64_t)K.bid * VEC_THREADS + threadIdx.x; q < ((n) >> 2);           \
+         q += (int64_t)K.nb * VEC_THREADS)
+
+__global__ void __launch_bounds__(VEC_THREADS) kb_pap(const BatchVec *bv, const BatchBlk *map) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
     if (st->done) return;
     double v[1] = {0.0};
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         const V4<float> pv = ld4(B.p, q), av = ld4(B.ap, q);
         FG_K4 v[0] += (double)pv.a[k] * (double)av.a[k];
     }
     double tot[1];
-    if (grid_sum<1>(v, B.partials, st, tot) && threadIdx.x == 0) {
+    if (grid_sum<1>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0) {
         st->pap = tot[0];
         if (fabs(tot[0]) < 1e-30) {
             st->breakdown = 1;
@@ -854,13 +873,14 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_pap(const BatchVec *bv) {
     }
 }
 
-__global__ void __launch_bounds__(VEC_THREADS) kb_rel_step(const BatchVec *bv) {
-    const BatchVec &B = bv[blockIdx.y];
+__global__ void __launch_bounds__(VEC_THREADS) kb_rel_step(const BatchVec *bv, const BatchBlk *map) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
     if (st->done) return;
     const float alpha = (float)st->alpha;
     double v[1] = {0.0};
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         V4<float> xv = ld4(B.e, q), rv = ld4(B.r, q);
         const V4<float> pv = ld4(B.p, q), av = ld4(B.ap, q);
         FG_K4 {
@@ -872,7 +892,7 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_step(const BatchVec *bv) {
         st4(B.r, q, rv);
     }
     double tot[1];
-    if (grid_sum<1>(v, B.partials, st, tot) && threadIdx.x == 0) {
+    if (grid_sum<1>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0) {
         st->iter += 1;
         st->rr = tot[0];
         const double rn = sqrt(tot[0]);
@@ -883,10 +903,11 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_step(const BatchVec *bv) {
     }
 }
 
-__global__ void __launch_bounds__(VEC_THREADS) kb_rel_xupdate(const BatchVec *bv) {
-    const BatchVec &B = bv[blockIdx.y];
+__global__ void __launch_bounds__(VEC_THREADS) kb_rel_xupdate(const BatchVec *bv, const BatchBlk *map) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     if (!B.st->trigger) return;
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         V4<double> xv = ld4(B.x64, q);
         const V4<float> lv = ld4(B.e, q);
         FG_K4 xv.a[k] += (double)lv.a[k];
@@ -895,12 +916,13 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_xupdate(const BatchVec *bv
     }
 }
 
-__global__ void __launch_bounds__(VEC_THREADS) kb_rel_residual(const BatchVec *bv, int init) {
-    const BatchVec &B = bv[blockIdx.y];
+__global__ void __launch_bounds__(VEC_THREADS) kb_rel_residual(const BatchVec *bv, const BatchBlk *map, int init) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
     if (!init && !st->trigger) return;
     double v[2] = {0.0, 0.0};
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         const V4<double> bb = ld4(B.b64, q), av = ld4(B.ap64, q);
         V4<float> rv;
         FG_K4 {
@@ -912,7 +934,7 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_residual(const BatchVec *b
         st4(B.r, q, rv);
     }
     double tot[2];
-    if (grid_sum<2>(v, B.partials, st, tot) && threadIdx.x == 0) {
+    if (grid_sum<2>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0) {
         if (init) {
             st->bb = tot[1];
             st->bnorm = sqrt(tot[1]);
@@ -939,11 +961,12 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_residual(const BatchVec *b
     }
 }
 
-__global__ void __launch_bounds__(VEC_THREADS) kb_cheb_first(const BatchVec *bv) {
-    const BatchVec &B = bv[blockIdx.y];
+__global__ void __launch_bounds__(VEC_THREADS) kb_cheb_first(const BatchVec *bv, const BatchBlk *map) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     if (B.st->done) return;
     const float it = (float)B.inv_theta;
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         const V4<float> rv = ld4(B.r, q), dv = ld4(B.dinv, q);
         V4<float> sv, dd;
         FG_K4 {
@@ -958,11 +981,12 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_cheb_first(const BatchVec *bv)
 
 // last: the final sweep, whose residual and d are not needed afterwards (two
 // stores fewer; z is the same)
-__global__ void __launch_bounds__(VEC_THREADS) kb_cheb_step(const BatchVec *bv, int s, int last) {
-    const BatchVec &B = bv[blockIdx.y];
+__global__ void __launch_bounds__(VEC_THREADS) kb_cheb_step(const BatchVec *bv, const BatchBlk *map, int s, int last) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     if (B.st->done) return;
     const float a1 = (float)B.c1[s], a2 = (float)B.c2[s];
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         const V4<float> tv = ld4(B.ct, q), dv = ld4(B.dinv, q);
         V4<float> sv = ld4(B.cres, q), dd = ld4(B.cd, q), zv = ld4(B.z, q);
         FG_K4 {
@@ -979,12 +1003,13 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_cheb_step(const BatchVec *bv, 
 }
 
 // jacobi: z = dinv r first; then rz_new = r.z, beta (init: rz only)
-__global__ void __launch_bounds__(VEC_THREADS) kb_rz(const BatchVec *bv, int init, int jacobi) {
-    const BatchVec &B = bv[blockIdx.y];
+__global__ void __launch_bounds__(VEC_THREADS) kb_rz(const BatchVec *bv, const BatchBlk *map, int init, int jacobi) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
     if (st->done) return;
     double v[1] = {0.0};
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         const V4<float> rv = ld4(B.r, q);
         V4<float> zv;
         if (jacobi) {
@@ -997,17 +1022,18 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rz(const BatchVec *bv, int ini
         FG_K4 v[0] += (double)rv.a[k] * (double)zv.a[k];
     }
     double tot[1];
-    if (grid_sum<1>(v, B.partials, st, tot) && threadIdx.x == 0) {
+    if (grid_sum<1>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0) {
         if (!init) st->beta = tot[0] / st->rz;
         st->rz = tot[0];
     }
 }
 
-__global__ void __launch_bounds__(VEC_THREADS) kb_pupdate(const BatchVec *bv, int init) {
-    const BatchVec &B = bv[blockIdx.y];
+__global__ void __launch_bounds__(VEC_THREADS) kb_pupdate(const BatchVec *bv, const BatchBlk *map, int init) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     if (B.st->done) return;
     const float beta = init ? 0.0f : (float)B.st->beta;
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         const V4<float> zv = ld4(B.z, q);
         V4<float> pv = init ? zv : ld4(B.p, q);  // first direction: p is not read
         if (!init) {
@@ -1017,16 +1043,18 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_pupdate(const BatchVec *bv, in
     }
 }
 
-__global__ void __launch_bounds__(VEC_THREADS) kb_zero_e(const BatchVec *bv) {
-    const BatchVec &B = bv[blockIdx.y];
-    FG_VEC4_LOOP(q, B.n) st4(B.e, q, V4<float>{{0.0f, 0.0f, 0.0f, 0.0f}});
+__global__ void __launch_bounds__(VEC_THREADS) kb_zero_e(const BatchVec *bv, const BatchBlk *map) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
+    FG_BVEC4_LOOP(q, B.n) st4(B.e, q, V4<float>{{0.0f, 0.0f, 0.0f, 0.0f}});
 }
 
-__global__ void __launch_bounds__(VEC_THREADS) kb_true_residual(const BatchVec *bv) {
-    const BatchVec &B = bv[blockIdx.y];
+__global__ void __launch_bounds__(VEC_THREADS) kb_true_residual(const BatchVec *bv, const BatchBlk *map) {
+    const BatchBlk K = map[blockIdx.x];
+    const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
     double v[1] = {0.0};
-    FG_VEC4_LOOP(q, B.n) {
+    FG_BVEC4_LOOP(q, B.n) {
         const V4<double> bb = ld4(B.b64, q), av = ld4(B.ap64, q);
         FG_K4 {
             const double s = bb.a[k] - av.a[k];
@@ -1034,7 +1062,7 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_true_residual(const BatchVec *
         }
     }
     double tot[1];
-    if (grid_sum<1>(v, B.partials, st, tot) && threadIdx.x == 0)
+    if (grid_sum<1>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0)
         st->tmp[0] = st->bnorm == 0.0 ? 0.0 : sqrt(tot[0]) / st->bnorm;
 }
 
