@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_pap(int64_t n, const T *__r
     double v[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
         const V4<T> pv = ld4(p, q), av = ld4(ap, q);
-        FG_K4 v[0] += (double)pv.a[k] * (double)av.a[k];
+        FG_K4 v[0] = fma((double)pv.a[k], (double)av.a[k], v[0]);
     }
     double tot[1];
     if (grid_sum<1>(v, partials, st, tot) && threadIdx.x == 0) {
@@ -207,10 +207,10 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_update(int64_t n, T *__rest
         FG_K4 {
             xv.a[k] += alpha * pv.a[k];
             rv.a[k] = rv.a[k] - alpha * av.a[k];
-            v[0] += (double)rv.a[k] * (double)rv.a[k];
+            v[0] = fma((double)rv.a[k], (double)rv.a[k], v[0]);
             if (jacobi) {
                 zv.a[k] = dv.a[k] * rv.a[k];
-                v[1] += (double)rv.a[k] * (double)zv.a[k];
+                v[1] = fma((double)rv.a[k], (double)zv.a[k], v[1]);
             }
         }
         st4(x, q, xv);
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_fused_jacobi(int64_t n, T *
     double v1[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
         const V4<T> pv = ld4(p, q), av = ld4(ap, q);
-        FG_K4 v1[0] += (double)pv.a[k] * (double)av.a[k];
+        FG_K4 v1[0] = fma((double)pv.a[k], (double)av.a[k], v1[0]);
     }
     double pap[1];
     all_blocks_sum<1>(v1, partials, bar, err, ok, pap);
@@ -306,9 +306,9 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_fused_jacobi(int64_t n, T *
         FG_K4 {
             xv.a[k] += alpha * pv.a[k];
             rv.a[k] = rv.a[k] - alpha * av.a[k];
-            v2[0] += (double)rv.a[k] * (double)rv.a[k];
+            v2[0] = fma((double)rv.a[k], (double)rv.a[k], v2[0]);
             zv.a[k] = dv.a[k] * rv.a[k];
-            v2[1] += (double)rv.a[k] * (double)zv.a[k];
+            v2[1] = fma((double)rv.a[k], (double)zv.a[k], v2[1]);
         }
         st4(x, q, xv);
         st4(r, q, rv);
