@@ -225,8 +225,10 @@ static int cfg_wy(int p) { return p == 1 ? KCfg<1>::WY : p == 2 ? KCfg<2>::WY : 
 struct fg_op {
     std::mutex mu;
     int device = 0;
-    Grid g{};
+    Grid g{};              // FP64 full format; the other forms' tiles in gv
+    Grid gv[2][2];         // [FP32][affine]: the same mesh, each form with its own tile shape
     int ess_tags = 0, kind = 0, p = 0;
+    bool tile_set = false;  // item depth chosen by fg_op_set_tile or the autotuner
     int64_t N = 0, Nn = 0;
     double *qd = nullptr, *face = nullptr;
     double *xs = nullptr, *ys = nullptr;
@@ -394,34 +396,45 @@ template <> struct KCfg32<3> { static constexpr int WY = FG_Q3_WY, S = FG_F32_Q3
 #ifndef FG_AFFINE_AS  // affine-format qdata ring depth of the other orders and precisions
 #define FG_AFFINE_AS 2
 #endif
+#ifndef FG_Q3_S8  // Q3 FP64 full-format ring depth of the 8-wide lane shape
+#define FG_Q3_S8 2
+#endif
 template <int P, typename T> constexpr int affine_stages() {
     return std::is_same<T, float>::value ? (P == 2 ? FG_F32_Q2_AS : (P == 3 ? FG_F32_Q3_AS : FG_AFFINE_AS))
                                          : FG_AFFINE_AS;
+}
+template <int P, typename T> struct KC;
+template <int P> struct KC<P, double> : KCfg<P> {};
+template <int P> struct KC<P, float> : KCfg32<P> {};
+// Ring depth of an apply kernel.  Q3 FP64: the 8-wide lane shape exchanges a
+// quarter of the y faces through shared memory, which leaves room for a second
+// stage at the same 4 CTAs per SM; with one stage each of a layer's 16 columns
+// waits out its own copy.
+template <int P, typename T, int FMT, int LX> constexpr int ring_stages() {
+    if (FMT == 1) return affine_stages<P, T>();
+    if (P == 3 && LX == 8 && std::is_same<T, double>::value) return FG_Q3_S8;
+    return KC<P, T>::S;
 }
 // CTAs/SM hint of an apply kernel
 template <int P, typename T, int FMT, int MINB> constexpr int apply_minb() {
     return (FMT == 1 && P == 2 && std::is_same<T, float>::value) ? FG_F32_Q2_AMINB : MINB;
 }
-template <int P, typename T> struct KC;
-template <int P> struct KC<P, double> : KCfg<P> {};
-template <int P> struct KC<P, float> : KCfg32<P> {};
-
 template <typename T> struct TmapType;
 template <> struct TmapType<double> { static constexpr CUtensorMapDataType v = CU_TENSOR_MAP_DATA_TYPE_FLOAT64; };
 template <> struct TmapType<float> { static constexpr CUtensorMapDataType v = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; };
 
-template <int P, int OPK, typename T, int FMT>
+template <int P, int OPK, typename T, int FMT, int LX>
 static int launch_apply_t(fg_op *op, const Grid &g, const T *qd, T *face, const T *x, T *y,
                           int accumulate, const int *skip, unsigned *fixcnt = nullptr, int item0 = 0,
                           int nitems = -1) {
     using C = KC<P, T>;
     static_assert(C::WY == KCfg<P>::WY, "FP32 and FP64 share the item tiling");
-    constexpr int S = FMT == 0 ? C::S : affine_stages<P, T>();  // affine format: one element layer per stage
-    using SM = ApplySmem<P, T, C::WY, S, stage_elems<P, OPK, FMT>() / 32>;
+    constexpr int S = ring_stages<P, T, FMT, LX>();
+    using SM = ApplySmem<P, T, C::WY, S, stage_elems<P, OPK, FMT>() / 32, LX>;
     // per device, set once; handles on several host threads may race here, and
     // setting the same attribute twice is harmless
     static std::atomic<bool> attr_set[64];
-    auto kern = pa_apply_kernel<P, OPK, T, C::WY, S, apply_minb<P, T, FMT, C::MINB>(), FMT>;
+    auto kern = pa_apply_kernel<P, OPK, T, C::WY, S, apply_minb<P, T, FMT, C::MINB>(), FMT, LX>;
     if (!attr_set[op->device].load(std::memory_order_acquire)) {
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::bytes));
         attr_set[op->device].store(true, std::memory_order_release);
@@ -441,6 +454,16 @@ static int launch_apply_t(fg_op *op, const Grid &g, const T *qd, T *face, const 
     return FG_OK;
 }
 
+// grid (tile shape) of the applies in precision T and the handle's format
+template <typename T> static const Grid &grid_of(const fg_op *op) {
+    return op->gv[std::is_same<T, float>::value ? 1 : 0][op->fmt];
+}
+// face slots that hold either format's partials of a precision
+static int64_t face_words(const fg_op *op, int fp32) {
+    const Grid &a = op->gv[fp32][0], &b = op->gv[fp32][1];
+    return std::max((int64_t)a.n_items() * a.face_stride(), (int64_t)b.n_items() * b.face_stride());
+}
+
 template <typename T> static const T *qdata_of(fg_op *op);
 template <> const double *qdata_of<double>(fg_op *op) { return op->fmt ? op->qa64 : op->qd; }
 template <> const float *qdata_of<float>(fg_op *op) { return op->fmt ? op->qa32 : op->qd32; }
@@ -450,17 +473,23 @@ static int launch_apply_p(fg_op *op, const Grid &g, const T *, T *face, const T 
                           int accumulate, const int *skip, unsigned *fixcnt, int item0 = 0, int nitems = -1) {
     const T *qd = qdata_of<T>(op);
     if (!qd) return fail(FG_INVALID_ARGUMENT, "quadrature data for this precision/format not built");
-    if (op->fmt == 0) {
-        switch (op->kind) {
-        case FG_MASS: return launch_apply_t<P, 1, T, 0>(op, g, qd, face, x, y, accumulate, skip, fixcnt, item0, nitems);
-        case FG_DIFF: return launch_apply_t<P, 2, T, 0>(op, g, qd, face, x, y, accumulate, skip, fixcnt, item0, nitems);
-        default: return launch_apply_t<P, 3, T, 0>(op, g, qd, face, x, y, accumulate, skip, fixcnt, item0, nitems);
-        }
-    }
-    switch (op->kind) {
-    case FG_MASS: return launch_apply_t<P, 1, T, 1>(op, g, qd, face, x, y, accumulate, skip, fixcnt, item0, nitems);
-    case FG_DIFF: return launch_apply_t<P, 2, T, 1>(op, g, qd, face, x, y, accumulate, skip, fixcnt, item0, nitems);
-    default: return launch_apply_t<P, 3, T, 1>(op, g, qd, face, x, y, accumulate, skip, fixcnt, item0, nitems);
+    auto run = [&](auto kind, auto fmt) -> int {
+        constexpr int OPK = decltype(kind)::value, FMT = decltype(fmt)::value;
+        if (g.LX == 8)
+            return launch_apply_t<P, OPK, T, FMT, 8>(op, g, qd, face, x, y, accumulate, skip, fixcnt, item0, nitems);
+        return launch_apply_t<P, OPK, T, FMT, 32>(op, g, qd, face, x, y, accumulate, skip, fixcnt, item0, nitems);
+    };
+    using I0 = std::integral_constant<int, 0>;
+    using I1 = std::integral_constant<int, 1>;
+    using I2 = std::integral_constant<int, 2>;
+    using I3 = std::integral_constant<int, 3>;
+    switch (op->kind * 2 + (op->fmt ? 1 : 0)) {
+    case FG_MASS * 2: return run(I1{}, I0{});
+    case FG_MASS * 2 + 1: return run(I1{}, I1{});
+    case FG_DIFF * 2: return run(I2{}, I0{});
+    case FG_DIFF * 2 + 1: return run(I2{}, I1{});
+    case FG_MASS_DIFF * 2: return run(I3{}, I0{});
+    default: return run(I3{}, I1{});
     }
 }
 
@@ -492,7 +521,7 @@ static int apply_native_t(fg_op *op, const T *qd, T *face, const T *x, T *y, int
                           int constrained, const int *skip) {
     if (op->unstr) return hex_apply<T>(op, qd, x, y, accumulate, constrained, skip);
     unsigned *fixcnt = fixcnt_for<T>(op, face);
-    Grid g = op->g;
+    Grid g = grid_of<T>(op);
     g.ess = constrained ? op->ess_tags : 0;
     int rc;
     switch (op->p) {
@@ -512,7 +541,8 @@ static int apply_native(fg_op *op, const double *x, double *y, int accumulate, i
 template <int P, int OPK> static int launch_diag_t(fg_op *op, const Grid &g, double *y) {
     constexpr int WY = KCfg<P>::WY;
     ApplyArgs<double> A{g, op->qd, y, op->face, 0, op->d_err, nullptr};
-    pa_diag_kernel<P, OPK, double, WY><<<g.n_items(), WY * 32, 0, op->stream>>>(A);
+    if (g.LX == 8) pa_diag_kernel<P, OPK, double, WY, 8><<<g.n_items(), WY * 32, 0, op->stream>>>(A);
+    else pa_diag_kernel<P, OPK, double, WY, 32><<<g.n_items(), WY * 32, 0, op->stream>>>(A);
     CK(cudaGetLastError());
     return FG_OK;
 }
@@ -567,6 +597,104 @@ template <int P> static int launch_setup_p(fg_op *op, SetupArgs &S, int64_t *qsi
 // ---------------------------------------------------------------------------
 // C ABI
 // ---------------------------------------------------------------------------
+// z depth of the items
+static void set_depth(Grid &g, int TZ) {
+    g.TZ = TZ;
+    g.ntz = (g.nz + TZ - 1) / TZ;
+}
+
+// Items of NW warps of LX x (32 / LX) elements.
+static void set_lanes(Grid &g, int LX) {
+    g.LX = LX;
+    g.WY = g.NW * (32 / LX);
+    g.ntx = (g.nx + LX - 1) / LX;
+    g.nty = (g.ny + g.WY - 1) / g.WY;
+}
+
+// The tiling by which fg_op_apply_native_noalloc's scratch limit counts:
+// 32-wide items of up to 8 layers, fewer while there are less than 592 items.
+static void set_scratch_tiling(Grid &g) {
+    set_lanes(g, 32);
+    int TZ = 8;
+    while (TZ > 1 && (int64_t)g.ntx * g.nty * ((g.nz + TZ - 1) / TZ) < 148 * 4) TZ /= 2;
+    set_depth(g, TZ);
+}
+
+#define FG_NOALLOC_FACE_DOUBLES (4u << 20)  // 4 Mi doubles = 32 MiB of static face scratch
+
+// Tile shape of one form (precision, format) of the apply: the lane shape, 32
+// elements in x or 8 in x by 4 in y, and the layers TZ per item.
+//
+// A warp of these kernels takes about the same time per layer whether it shares
+// its SM or has it to itself (45 x 41 x 38 Q3 FP32 affine: 7.5 us a layer with one to four
+// CTAs per SM), so the time is the number of rounds of resident CTAs times the
+// layers of one, plus what a CTA spends before its first layer's data arrive
+// (about 0.8 layer).  Rounds count whole up to four (the last one leaves SMs
+// idle), above that half a round is lost on average; a small term counts the
+// warps that work at all, which separates the lane shapes when the rounds do
+// not.  The 8 x 4 shape pays for its shuffles and shorter rows of stores (2 %;
+// 128^3 Q2 FP64 517 against 552 us), except in the Q3 FP64 full format, where it has
+// the deeper ring (64^3: 245 against 275 us).  The rule before this one took 32 lanes
+// in x and halved the depth until there were 592 items, which left a nearly empty
+// last round or lane padding: apply and fix-up on a B200, then -> now: 48^3 Q3 FP32
+// affine 45.6 -> 34.8 us, 33x40x37 38.0 -> 24.8, 48x40x44 Q2 FP64 42.9 -> 34.1,
+// 45x41x38 Q3 FP64 121 -> 97, 100x90x80 Q1 FP64 76.9 -> 57.6, 64^3 Q2 FP32 affine
+// mass + diffusion 32.6 -> 30.6.
+static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size_t face_limit) {
+    // CTAs per SM by registers and shared memory, [fp32][affine][order]
+    static const int resident[2][2][3] = {{{3, 2, 4}, {3, 2, 2}}, {{5, 3, 4}, {5, 5, 4}}};
+    const int R = (fp32 && affine && g.p == 2 && (kind & FG_MASS)) ? 4 : resident[fp32][affine][g.p - 1];
+    const double slots = 148.0 * R;
+    Grid best = g;
+    double best_cost = 1e300;
+    int warps32 = 0;  // warps per layer of the 32-wide shape
+    for (int LX : {32, 8}) {
+        if (lanes && LX != lanes) continue;
+        Grid c = g;
+        set_lanes(c, LX);
+        const int warps = c.ntx * c.nty * c.NW, live = c.ntx * ((c.ny + 32 / LX - 1) / (32 / LX));
+        if (LX == 32) warps32 = warps;
+        // 8-wide items may not outnumber the 32-wide ones by more than a tenth: a warp
+        // without elements still holds its registers, and the face slots grow
+        else if (!lanes && 10 * warps > 11 * warps32) continue;
+        const double shape = LX == 32 ? 1.0 : (g.p == 3 && !fp32 && !affine) ? 0.92 : 1.02;
+        const double work = (double)(LX == 32 ? warps : live) * c.nz / (c.NW * slots);
+        for (int tz = 1; tz <= std::min(g.nz, 16); ++tz) {
+            set_depth(c, tz);
+            if (face_limit && (size_t)c.n_items() * (size_t)c.face_stride() > face_limit) continue;
+            const double w = c.n_items() / slots;
+            const double cost = shape * ((w >= 4.0 ? w + 0.5 : std::ceil(w)) * (tz + 0.8) + 0.25 * work);
+            if (cost < best_cost * (1.0 - 1e-9)) {
+                best_cost = cost;
+                best = c;
+            }
+        }
+    }
+    if (best_cost == 1e300) set_scratch_tiling(best);
+    g = best;
+}
+
+// Tile shapes of the handle's four forms.  FG_LANES_X=8 or 32 fixes the lane shape.
+static void choose_tiles(fg_op *op) {
+    int lanes = 0;
+    if (const char *e = std::getenv("FG_LANES_X")) {
+        const int v = std::atoi(e);
+        if (v == 8 || v == 32) lanes = v;
+    }
+    Grid w = op->g;
+    set_scratch_tiling(w);
+    const size_t old = (size_t)w.n_items() * (size_t)w.face_stride();
+    for (int fp32 = 0; fp32 < 2; ++fp32)
+        for (int affine = 0; affine < 2; ++affine) {
+            Grid &g = op->gv[fp32][affine];
+            g = op->g;
+            // an operator that fits the static scratch by its 32-wide tiling must fit it by the chosen one
+            choose_tile(g, op->kind, fp32, affine, lanes,
+                        !fp32 && !affine && old <= FG_NOALLOC_FACE_DOUBLES ? FG_NOALLOC_FACE_DOUBLES : 0);
+        }
+    op->g = op->gv[0][0];
+}
+
 extern "C" {
 
 FG_API void fg_cfg_default(fg_cfg *c) {
@@ -628,14 +756,8 @@ FG_API int fg_op_create(const fg_mesh *mesh, int order, int nq1d, int kind, doub
     g.nx = mesh->nx; g.ny = mesh->ny; g.nz = mesh->nz; g.p = order;
     g.NI = (int)NI; g.NJ = (int)NJ; g.NK = (int)NK;
     g.NIp = round_up((int)NI, 4);
-    g.WY = cfg_wy(order);
-    g.ntx = (g.nx + 31) / 32;
-    g.nty = (g.ny + g.WY - 1) / g.WY;
-    // layers per item: as many as keep >= 4 items per SM slot on a 148-SM part
-    int TZ = 8;
-    while (TZ > 1 && (int64_t)g.ntx * g.nty * ((g.nz + TZ - 1) / TZ) < 148 * 4) TZ /= 2;
-    g.TZ = TZ;
-    g.ntz = (g.nz + TZ - 1) / TZ;
+    g.NW = cfg_wy(order);
+    choose_tiles(op);
     g.ess = 0;
     op->N = NI * NJ * NK;
     op->Nn = (int64_t)g.NIp * NJ * NK;
@@ -661,8 +783,11 @@ FG_API int fg_op_create(const fg_mesh *mesh, int order, int nq1d, int kind, doub
     if (cudaMalloc(&op->st, sizeof(SolverState)) != cudaSuccess ||
         cudaMemset(op->st, 0, sizeof(SolverState)) != cudaSuccess)
         return bail(fail(FG_CUDA_ERROR, "cudaMalloc failed"));
-    if ((rc = alloc_vec(&op->face, (int64_t)g.n_items() * g.face_stride()))) return bail(rc);
-    op->fixcnt_items = (int64_t)g.ntx * g.nty * g.nz;  // items at one layer each: any tiling fits
+    if ((rc = alloc_vec(&op->face, face_words(op, 0)))) return bail(rc);
+    for (int k = 0; k < 4; ++k) {  // items at one layer each: any depth of any form fits
+        const Grid &q = op->gv[k >> 1][k & 1];
+        op->fixcnt_items = std::max(op->fixcnt_items, (int64_t)q.ntx * q.nty * q.nz);
+    }
     if ((rc = alloc_vec(&op->fixcnt, 2 * op->fixcnt_items))) return bail(rc);
     if ((rc = alloc_vec(&op->xs, op->Nn)) || (rc = alloc_vec(&op->ys, op->Nn))) return bail(rc);
     if ((rc = alloc_vec(&op->partials, VEC_GRID * 4))) return bail(rc);
@@ -854,7 +979,7 @@ static int from_native(fg_op *op, double *dst, const double *src, int mem) {
 // on the way in and y planes on the way out: a y range is packed only after
 // the x planes it overlaps were repacked, and uploads never touch it again.
 static int apply_host_pipelined(fg_op *op, const double *x, double *y, int constrained) {
-    Grid g = op->g;
+    Grid g = grid_of<double>(op);
     g.ess = constrained ? op->ess_tags : 0;
     static const int max_ranges = [] {  // FG_PIPE_RANGES: z ranges of the pipeline (default 16)
         const char *e = std::getenv("FG_PIPE_RANGES");
@@ -943,7 +1068,7 @@ FG_API int fg_op_apply(fg_op *op, const double *x, double *y, int accumulate, in
     std::lock_guard<std::mutex> lk(op->mu);
     CK(cudaSetDevice(op->device));
     int rc;
-    if (mem == FG_HOST && !accumulate && !op->unstr && !op->fused_fixup && op->g.ntz >= 2 && op->pipelined) {
+    if (mem == FG_HOST && !accumulate && !op->unstr && !op->fused_fixup && grid_of<double>(op).ntz >= 2 && op->pipelined) {
         if ((rc = apply_host_pipelined(op, x, y, constrained))) return rc;
         return check_device_error(op);
     }
@@ -981,7 +1106,8 @@ FG_API int fg_op_diagonal(fg_op *op, double *d, int constrained, int mem) {
 template <int P, int OPK, typename T> static void launch_compress(fg_op *op, T *dst) {
     const int64_t total = (int64_t)op->g.nx * op->g.ny * op->g.nz * (P + 1) * (P + 1) * (P + 1);
     const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 32);
-    qdata_compress_kernel<P, OPK, T><<<blocks, 256, 0, op->stream>>>(op->g, op->qd, dst, op->d_err);
+    qdata_compress_kernel<P, OPK, T><<<blocks, 256, 0, op->stream>>>(
+        op->g, op->gv[std::is_same<T, float>::value][1], op->qd, dst, op->d_err);
 }
 template <int P, typename T> static void launch_compress_p(fg_op *op, T *dst) {
     switch (op->kind) {
@@ -993,7 +1119,7 @@ template <int P, typename T> static void launch_compress_p(fg_op *op, T *dst) {
 template <typename T> static int64_t affine_size(fg_op *op) {
     auto sz = [&](auto pk, auto ok) -> int64_t {
         constexpr int P = decltype(pk)::value, OPK = decltype(ok)::value;
-        return qd_size_fmt<P, OPK, 1>(op->g);
+        return qd_size_fmt<P, OPK, 1>(op->gv[std::is_same<T, float>::value][1]);
     };
     using I1 = std::integral_constant<int, 1>;
     using I2 = std::integral_constant<int, 2>;
@@ -1050,16 +1176,43 @@ static int ensure_dinv(fg_op *op) {
     return FG_OK;
 }
 
-// FP32 copy of the quadrature data (same layout) and the FP32 work vectors.
+// Full-format quadrature data of the handle (FP64, tile shape op->g) in
+// precision T and the tile shape gn, in a new buffer; pads are zero.
+template <int P, int OPK, typename T> static int relayout_t(fg_op *op, const Grid &gn, T **dst, int64_t *size) {
+    int rc;
+    *size = qd_size<P, OPK>(gn);
+    if ((rc = alloc_vec(dst, *size))) return rc;
+    const int64_t total = (int64_t)gn.nx * gn.ny * gn.nz * (P + 1) * (P + 1) * (P + 1);
+    const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 32);
+    qdata_relayout_kernel<P, OPK, T><<<blocks, 256, 0, op->stream>>>(op->g, gn, op->qd, *dst);
+    CK(cudaGetLastError());
+    return FG_OK;
+}
+template <typename T> static int relayout(fg_op *op, const Grid &gn, T **dst, int64_t *size) {
+    switch (op->p * 4 + op->kind) {
+    case 1 * 4 + FG_MASS: return relayout_t<1, 1, T>(op, gn, dst, size);
+    case 1 * 4 + FG_DIFF: return relayout_t<1, 2, T>(op, gn, dst, size);
+    case 1 * 4 + FG_MASS_DIFF: return relayout_t<1, 3, T>(op, gn, dst, size);
+    case 2 * 4 + FG_MASS: return relayout_t<2, 1, T>(op, gn, dst, size);
+    case 2 * 4 + FG_DIFF: return relayout_t<2, 2, T>(op, gn, dst, size);
+    case 2 * 4 + FG_MASS_DIFF: return relayout_t<2, 3, T>(op, gn, dst, size);
+    case 3 * 4 + FG_MASS: return relayout_t<3, 1, T>(op, gn, dst, size);
+    case 3 * 4 + FG_DIFF: return relayout_t<3, 2, T>(op, gn, dst, size);
+    default: return relayout_t<3, 3, T>(op, gn, dst, size);
+    }
+}
+
+// FP32 copy of the quadrature data (in its own tile shape) and the FP32 work vectors.
 static int ensure_fp32(fg_op *op) {
     int rc;
-    if (!op->qd32) {
+    if (!op->qd32 && op->unstr) {
         if ((rc = alloc_vec(&op->qd32, op->qsize))) return rc;
         k_to_f32<<<VEC_GRID * 4, VEC_THREADS, 0, op->stream>>>(op->qsize, op->qd, op->qd32);
         CK(cudaGetLastError());
     }
-    if (!op->face32 && (rc = alloc_vec(&op->face32, (int64_t)op->g.n_items() * op->g.face_stride())))
-        return rc;
+    int64_t n32 = 0;
+    if (!op->qd32 && (rc = relayout<float>(op, op->gv[1][0], &op->qd32, &n32))) return rc;
+    if (!op->face32 && (rc = alloc_vec(&op->face32, op->unstr ? 1 : face_words(op, 1)))) return rc;
     if (op->fmt == 1 && !op->qa32 && (rc = build_affine<float>(op, &op->qa32))) return rc;
     float **v[] = {&op->r32, &op->z32, &op->p32, &op->ap32, &op->e32, &op->b32, &op->cres32,
                    &op->cd32, &op->ct32, &op->xs32, &op->ys32};
@@ -1888,11 +2041,11 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
 // ---------------------------------------------------------------------------
 }  // extern "C"
 
-template <int P, typename T, int FMT>
+template <int P, typename T, int FMT, int LX>
 static int encode_xmap_t(const Grid &g, const T *x, CUtensorMap *tmap) {
     using C = KC<P, T>;
-    constexpr int S = FMT == 0 ? C::S : affine_stages<P, T>();
-    using SM = ApplySmem<P, T, C::WY, S, 1>;
+    constexpr int S = ring_stages<P, T, FMT, LX>();
+    using SM = ApplySmem<P, T, C::WY, S, 1, LX>;
     cuuint64_t gdim[3] = {(cuuint64_t)g.NI, (cuuint64_t)g.NJ, (cuuint64_t)g.NK};
     cuuint64_t gstr[2] = {(cuuint64_t)g.NIp * sizeof(T), (cuuint64_t)g.NIp * g.NJ * sizeof(T)};
     cuuint32_t box[3] = {(cuuint32_t)SM::XW, (cuuint32_t)SM::RY, (cuuint32_t)(P + 1)};
@@ -1904,27 +2057,31 @@ static int encode_xmap_t(const Grid &g, const T *x, CUtensorMap *tmap) {
     return FG_OK;
 }
 template <typename T> static int encode_xmap(fg_op *op, const T *x, CUtensorMap *tmap) {
-    switch (op->p) {
-    case 1: return encode_xmap_t<1, T, 0>(op->g, x, tmap);
-    case 2: return encode_xmap_t<2, T, 0>(op->g, x, tmap);
-    default: return encode_xmap_t<3, T, 0>(op->g, x, tmap);
+    const Grid &g = grid_of<T>(op);
+    switch (g.LX + op->p) {
+    case 32 + 1: return encode_xmap_t<1, T, 0, 32>(g, x, tmap);
+    case 32 + 2: return encode_xmap_t<2, T, 0, 32>(g, x, tmap);
+    case 32 + 3: return encode_xmap_t<3, T, 0, 32>(g, x, tmap);
+    case 8 + 1: return encode_xmap_t<1, T, 0, 8>(g, x, tmap);
+    case 8 + 2: return encode_xmap_t<2, T, 0, 8>(g, x, tmap);
+    default: return encode_xmap_t<3, T, 0, 8>(g, x, tmap);
     }
 }
 
-struct BatchGroup {
-    int p, kind, fmt;
+struct BatchGroup {  // instances of one order, kind, format and lane shape
+    int p, kind, fmt, lx;
     std::vector<int> inst;
     int2 *bmap = nullptr;
     int nblocks = 0;
 };
 
-template <int P, int OPK, typename T, int FMT>
+template <int P, int OPK, typename T, int FMT, int LX>
 static int launch_batched_t(cudaStream_t st, const BatchGroup &G, const ApplyArgs<T> *args,
                             const CUtensorMap *tm, int nslots, int slot) {
     using C = KC<P, T>;
-    constexpr int S = FMT == 0 ? C::S : affine_stages<P, T>();
-    using SM = ApplySmem<P, T, C::WY, S, stage_elems<P, OPK, FMT>() / 32>;
-    auto kern = pa_apply_batched_kernel<P, OPK, T, C::WY, S, apply_minb<P, T, FMT, C::MINB>(), FMT>;
+    constexpr int S = ring_stages<P, T, FMT, LX>();
+    using SM = ApplySmem<P, T, C::WY, S, stage_elems<P, OPK, FMT>() / 32, LX>;
+    auto kern = pa_apply_batched_kernel<P, OPK, T, C::WY, S, apply_minb<P, T, FMT, C::MINB>(), FMT, LX>;
     static std::atomic<bool> attr_set[64];
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -1943,7 +2100,9 @@ template <typename T>
 static int launch_batched(cudaStream_t st, const BatchGroup &G, const ApplyArgs<T> *args,
                           const CUtensorMap *tm, int nslots, int slot) {
 #define FG_BL(P_, K_, F_) \
-    if (G.p == P_ && G.kind == K_ && G.fmt == F_) return launch_batched_t<P_, K_, T, F_>(st, G, args, tm, nslots, slot);
+    if (G.p == P_ && G.kind == K_ && G.fmt == F_)                                     \
+        return G.lx == 8 ? launch_batched_t<P_, K_, T, F_, 8>(st, G, args, tm, nslots, slot) \
+                         : launch_batched_t<P_, K_, T, F_, 32>(st, G, args, tm, nslots, slot);
     FG_BL(1, 1, 0) FG_BL(1, 2, 0) FG_BL(1, 3, 0) FG_BL(2, 1, 0) FG_BL(2, 2, 0) FG_BL(2, 3, 0)
     FG_BL(3, 1, 0) FG_BL(3, 2, 0) FG_BL(3, 3, 0)
     FG_BL(1, 1, 1) FG_BL(1, 2, 1) FG_BL(1, 3, 1) FG_BL(2, 1, 1) FG_BL(2, 2, 1) FG_BL(2, 3, 1)
@@ -1959,47 +2118,26 @@ template <typename T> static int dev_upload(T **dst, const std::vector<T> &v) {
     return FG_OK;
 }
 
-// ---- tile shape: items of 32 x WY x TZ elements -----------------------------
-template <int P, int OPK> static int relayout_t(fg_op *op, const Grid &gn, double *dst) {
-    const int64_t total = (int64_t)op->g.nx * op->g.ny * op->g.nz * (P + 1) * (P + 1) * (P + 1);
-    const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 32);
-    qdata_relayout_kernel<P, OPK><<<blocks, 256, 0, op->stream>>>(op->g, gn, op->qd, dst);
-    CK(cudaGetLastError());
-    return FG_OK;
-}
-template <int P> static int relayout_p(fg_op *op, const Grid &gn, double **dst, int64_t *size) {
-    switch (op->kind) {
-    case FG_MASS: *size = qd_size<P, 1>(gn); break;
-    case FG_DIFF: *size = qd_size<P, 2>(gn); break;
-    default: *size = qd_size<P, 3>(gn); break;
-    }
-    int rc;
-    if ((rc = alloc_vec(dst, *size))) return rc;
-    switch (op->kind) {
-    case FG_MASS: return relayout_t<P, 1>(op, gn, *dst);
-    case FG_DIFF: return relayout_t<P, 2>(op, gn, *dst);
-    default: return relayout_t<P, 3>(op, gn, *dst);
-    }
-}
-
-// Move the operator to items of TZ = tz layers (caller holds op->mu): the
-// full quadrature data is re-laid out on the device, the face slots are
-// re-sized, and the FP32 / affine copies are dropped and rebuilt from the new
-// layout on next use (the affine FP64 copy at once if it is in use).
+// ---- tile depth -------------------------------------------------------------
+// Move every form of the operator to items of TZ = tz layers (caller holds
+// op->mu): the full quadrature data is re-laid out on the device, the face slots
+// are re-sized, and the FP32 / affine copies are dropped and rebuilt on next use
+// (the affine FP64 copy at once if it is in use).
 static int set_tile_locked(fg_op *op, int tz) {
-    if (tz == op->g.TZ) return FG_OK;
-    Grid gn = op->g;
-    gn.TZ = tz;
-    gn.ntz = (gn.nz + tz - 1) / tz;
+    bool same = true;
+    Grid gv[2][2];
+    for (int k = 0; k < 4; ++k) {
+        gv[k >> 1][k & 1] = op->gv[k >> 1][k & 1];
+        same = same && gv[k >> 1][k & 1].TZ == tz;
+        set_depth(gv[k >> 1][k & 1], tz);
+    }
+    if (same) return FG_OK;
     double *nq = nullptr, *nface = nullptr;
     int64_t nsize = 0;
-    int rc;
-    switch (op->p) {
-    case 1: rc = relayout_p<1>(op, gn, &nq, &nsize); break;
-    case 2: rc = relayout_p<2>(op, gn, &nq, &nsize); break;
-    default: rc = relayout_p<3>(op, gn, &nq, &nsize); break;
-    }
-    if (!rc) rc = alloc_vec(&nface, (int64_t)gn.n_items() * gn.face_stride());
+    int rc = relayout<double>(op, gv[0][0], &nq, &nsize);
+    if (!rc)
+        rc = alloc_vec(&nface, std::max((int64_t)gv[0][0].n_items() * gv[0][0].face_stride(),
+                                        (int64_t)gv[0][1].n_items() * gv[0][1].face_stride()));
     if (!rc && cudaStreamSynchronize(op->stream) != cudaSuccess)
         rc = fail(FG_CUDA_ERROR, "quadrature-data re-layout failed: %s", cudaGetErrorString(cudaGetLastError()));
     if (rc) {
@@ -2016,23 +2154,26 @@ static int set_tile_locked(fg_op *op, int tz) {
     op->qd = nq;
     op->face = nface;
     op->qsize = nsize;
-    op->g = gn;
+    for (int k = 0; k < 4; ++k) op->gv[k >> 1][k & 1] = gv[k >> 1][k & 1];
+    op->g = gv[0][0];
+    op->tile_set = true;
     if (op->fmt == 1 && (rc = build_affine<double>(op, &op->qa64))) return rc;
     return FG_OK;
 }
 
 // batched launches over a set of instances: block map with the instances
 // holding the most items first (fewer idle SMs at the end of a launch)
+template <typename T>
 static std::vector<int2> largest_first_bmap(fg_op *const *ops, const std::vector<int> &inst,
                                             const std::vector<int> &slot_of) {
     std::vector<int> order(inst.size());
     for (size_t k = 0; k < inst.size(); ++k) order[k] = (int)k;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-        return ops[inst[a]]->g.n_items() > ops[inst[b]]->g.n_items();
+        return grid_of<T>(ops[inst[a]]).n_items() > grid_of<T>(ops[inst[b]]).n_items();
     });
     std::vector<int2> m;
     for (int k : order)
-        for (int it = 0; it < ops[inst[k]]->g.n_items(); ++it) m.push_back(make_int2(slot_of[k], it));
+        for (int it = 0; it < grid_of<T>(ops[inst[k]]).n_items(); ++it) m.push_back(make_int2(slot_of[k], it));
     return m;
 }
 
@@ -2081,7 +2222,7 @@ static int time_batched_apply(fg_op *const *ops, const std::vector<int> &inst, c
     for (int j = 0; j < k; ++j) {
         fg_op *o = ops[inst[j]];
         if ((rc = ensure_fp32(o))) return rc;
-        Grid g = o->g;
+        Grid g = grid_of<float>(o);
         g.ess = o->ess_tags;
         a[j] = ApplyArgs<float>{g, qdata_of<float>(o), o->ap32, o->face32, 0, o->d_err, nullptr};
         if ((rc = encode_xmap<float>(o, o->p32, &t[j]))) return rc;
@@ -2090,9 +2231,20 @@ static int time_batched_apply(fg_op *const *ops, const std::vector<int> &inst, c
         CK(cudaStreamSynchronize(o->stream));
     }
     fg_op *o0 = ops[inst[0]];
-    BatchGroup G{o0->p, o0->kind, o0->fmt, {}};
-    const std::vector<int2> m = largest_first_bmap(ops, inst, slot);
-    G.nblocks = (int)m.size();
+    std::vector<BatchGroup> groups;  // one per lane shape in the class
+    std::vector<std::vector<int2>> gmap;
+    for (int lx : {32, 8}) {
+        std::vector<int> in, sl;
+        for (int j = 0; j < k; ++j)
+            if (grid_of<float>(ops[inst[j]]).LX == lx) {
+                in.push_back(inst[j]);
+                sl.push_back(slot[j]);
+            }
+        if (in.empty()) continue;
+        gmap.push_back(largest_first_bmap<float>(ops, in, sl));
+        groups.push_back(BatchGroup{o0->p, o0->kind, o0->fmt, lx, {}});
+        groups.back().nblocks = (int)gmap.back().size();
+    }
     ApplyArgs<float> *d_a = nullptr;
     CUtensorMap *d_t = nullptr;
     FixArgs<float> *d_f = nullptr;
@@ -2102,20 +2254,24 @@ static int time_batched_apply(fg_op *const *ops, const std::vector<int> &inst, c
     FixBlk *d_fm = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     auto cleanup = [&]() {
-        void *ptrs[] = {G.bmap, d_a, d_t, d_f, d_fm};
+        void *ptrs[] = {d_a, d_t, d_f, d_fm};
         for (void *q : ptrs) if (q) cudaFree(q);
+        for (BatchGroup &G : groups) if (G.bmap) cudaFree(G.bmap);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
     };
     struct Guard { std::function<void()> f; ~Guard() { f(); } } guard{cleanup};
-    if ((rc = dev_upload(&G.bmap, m)) || (rc = dev_upload(&d_a, a)) || (rc = dev_upload(&d_t, t)) ||
-        (rc = dev_upload(&d_f, f)) || (rc = dev_upload(&d_fm, fm)))
+    for (size_t q = 0; q < groups.size(); ++q)
+        if ((rc = dev_upload(&groups[q].bmap, gmap[q]))) return rc;
+    if ((rc = dev_upload(&d_a, a)) || (rc = dev_upload(&d_t, t)) || (rc = dev_upload(&d_f, f)) || (rc = dev_upload(&d_fm, fm)))
         return rc;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     auto once = [&]() -> int {
-        int r2 = launch_batched<float>(bs, G, d_a, d_t, 1, 0);
-        if (r2) return r2;
+        for (const BatchGroup &G : groups) {
+            const int r2 = launch_batched<float>(bs, G, d_a, d_t, 1, 0);
+            if (r2) return r2;
+        }
         if (!fm.empty()) fixup_batched_kernel<float><<<(unsigned)fm.size(), 128, 0, bs>>>(d_f, d_fm, 1, 0);
         CK(cudaGetLastError());
         return FG_OK;
@@ -2149,9 +2305,10 @@ FG_API int fg_op_set_tile(fg_op *op, int tz) {
 FG_API int fg_op_tile(const fg_op *op, int dims[3]) {
     FG_NEED_BOX(op, "fg_op_tile");
     if (!op || !dims) return fail(FG_INVALID_ARGUMENT, "NULL argument");
-    dims[0] = 32;
-    dims[1] = op->g.WY;
-    dims[2] = op->g.TZ;
+    const Grid &g = grid_of<double>(op);
+    dims[0] = g.LX;
+    dims[1] = g.WY;
+    dims[2] = g.TZ;
     return FG_OK;
 }
 
@@ -2358,32 +2515,33 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
     double *d_part = nullptr;
     CK(cudaMalloc(&d_st, sizeof(SolverState) * n));
     std::vector<int64_t> len(n);
-    std::vector<Grid> fgs(n);
+    std::vector<Grid> g32(n), g64(n);
     for (int i = 0; i < n; ++i) {
         len[i] = ops[i]->Nn;
-        fgs[i] = ops[i]->g;
+        g32[i] = grid_of<float>(ops[i]);
+        g64[i] = grid_of<double>(ops[i]);
     }
     std::vector<int> vfirst;
     const std::vector<BatchBlk> vmap = vec_blocks(len, vfirst);
-    const std::vector<FixBlk> fmap = fix_blocks(fgs);
+    const std::vector<FixBlk> fmap = fix_blocks(g32), fmap64 = fix_blocks(g64);
     CK(cudaMalloc(&d_part, sizeof(double) * 2 * vmap.size()));
     std::vector<SolverState> hst(n);
     for (int i = 0; i < n; ++i) {
         fg_op *o = ops[i];
-        Grid g = o->g;
-        g.ess = o->ess_tags;
+        Grid g = grid_of<float>(o), h64 = grid_of<double>(o);
+        g.ess = h64.ess = o->ess_tags;
         const float *q32 = qdata_of<float>(o);
         const double *q64 = qdata_of<double>(o);
         a32[2 * i] = ApplyArgs<float>{g, q32, o->ap32, o->face32, 0, o->d_err, &d_st[i].done};
         a32[2 * i + 1] = ApplyArgs<float>{g, q32, o->ct32, o->face32, 0, o->d_err, &d_st[i].done};
-        a64[i] = ApplyArgs<double>{g, q64, o->ap, o->face, 0, o->d_err, &d_st[i].skip_rel};
+        a64[i] = ApplyArgs<double>{h64, q64, o->ap, o->face, 0, o->d_err, &d_st[i].skip_rel};
         if ((rc = encode_xmap<float>(o, o->p32, &t32[2 * i])) ||
             (rc = encode_xmap<float>(o, o->cd32, &t32[2 * i + 1])) ||
             (rc = encode_xmap<double>(o, o->xw, &t64[i])))
             return rc;
         f32[2 * i] = FixArgs<float>{g, o->ap32, o->face32, &d_st[i].done};
         f32[2 * i + 1] = FixArgs<float>{g, o->ct32, o->face32, &d_st[i].done};
-        f64[i] = FixArgs<double>{g, o->ap, o->face, &d_st[i].skip_rel};
+        f64[i] = FixArgs<double>{h64, o->ap, o->face, &d_st[i].skip_rel};
         BatchVec &B = bv[i];
         B.n = o->Nn;
         B.x64 = o->xw; B.b64 = o->bw; B.ap64 = o->ap;
@@ -2403,15 +2561,19 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
         h.delta = (cfg.inner_rtol > 0 && cfg.inner_rtol < 1) ? cfg.inner_rtol : 0.1;
         h.skip_rel = 0;  // the initial FP64 residual always runs
     }
-    // groups of equal (order, kind, format); block maps
-    std::vector<BatchGroup> groups;
-    for (int i = 0; i < n; ++i) {
+    // groups of equal (order, kind, format, lane shape) per precision; block maps
+    std::vector<BatchGroup> groups32, groups64;
+    auto add = [&](std::vector<BatchGroup> &groups, int i, int lx) {
         fg_op *o = ops[i];
         auto it = std::find_if(groups.begin(), groups.end(), [&](const BatchGroup &G) {
-            return G.p == o->p && G.kind == o->kind && G.fmt == o->fmt;
+            return G.p == o->p && G.kind == o->kind && G.fmt == o->fmt && G.lx == lx;
         });
-        if (it == groups.end()) { groups.push_back(BatchGroup{o->p, o->kind, o->fmt, {}}); it = groups.end() - 1; }
+        if (it == groups.end()) { groups.push_back(BatchGroup{o->p, o->kind, o->fmt, lx, {}}); it = groups.end() - 1; }
         it->inst.push_back(i);
+    };
+    for (int i = 0; i < n; ++i) {
+        add(groups32, i, g32[i].LX);
+        add(groups64, i, g64[i].LX);
     }
     ApplyArgs<float> *d_a32 = nullptr;
     ApplyArgs<double> *d_a64 = nullptr;
@@ -2420,32 +2582,40 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
     FixArgs<double> *d_f64 = nullptr;
     BatchVec *d_bv = nullptr;
     BatchBlk *d_vm = nullptr;
-    FixBlk *d_fm = nullptr;
+    FixBlk *d_fm = nullptr, *d_fm64 = nullptr;
     cudaGraphExec_t gexec = nullptr;
     cudaGraph_t graph = nullptr;
     auto cleanup = [&]() {
         if (gexec) cudaGraphExecDestroy(gexec);
         if (graph) cudaGraphDestroy(graph);
-        for (auto &G : groups) if (G.bmap) cudaFree(G.bmap);
-        void *ptrs[] = {d_a32, d_a64, d_t32, d_t64, d_f32, d_f64, d_bv, d_st, d_part, d_vm, d_fm};
+        for (auto &G : groups32) if (G.bmap) cudaFree(G.bmap);
+        for (auto &G : groups64) if (G.bmap) cudaFree(G.bmap);
+        void *ptrs[] = {d_a32, d_a64, d_t32, d_t64, d_f32, d_f64, d_bv, d_st, d_part, d_vm, d_fm, d_fm64};
         for (void *p : ptrs) if (p) cudaFree(p);
         cudaStreamDestroy(bs);
     };
     struct Guard { std::function<void()> f; ~Guard() { f(); } } guard{cleanup};
-    for (auto &G : groups) {
-        const std::vector<int2> m = largest_first_bmap(ops, G.inst, G.inst);
+    for (auto &G : groups32) {
+        const std::vector<int2> m = largest_first_bmap<float>(ops, G.inst, G.inst);
+        G.nblocks = (int)m.size();
+        if ((rc = dev_upload(&G.bmap, m))) return rc;
+    }
+    for (auto &G : groups64) {
+        const std::vector<int2> m = largest_first_bmap<double>(ops, G.inst, G.inst);
         G.nblocks = (int)m.size();
         if ((rc = dev_upload(&G.bmap, m))) return rc;
     }
     if ((rc = dev_upload(&d_a32, a32)) || (rc = dev_upload(&d_a64, a64)) || (rc = dev_upload(&d_t32, t32)) ||
         (rc = dev_upload(&d_t64, t64)) || (rc = dev_upload(&d_f32, f32)) || (rc = dev_upload(&d_f64, f64)) ||
-        (rc = dev_upload(&d_bv, bv)) || (rc = dev_upload(&d_vm, vmap)) || (rc = dev_upload(&d_fm, fmap)))
+        (rc = dev_upload(&d_bv, bv)) || (rc = dev_upload(&d_vm, vmap)) || (rc = dev_upload(&d_fm, fmap)) ||
+        (rc = dev_upload(&d_fm64, fmap64)))
         return rc;
     CK(cudaMemcpy(d_st, hst.data(), sizeof(SolverState) * n, cudaMemcpyHostToDevice));
     FG_LEGACY_FENCE();
-    const unsigned vgrid = (unsigned)vmap.size(), fgrid = (unsigned)fmap.size();
+    const unsigned vgrid = (unsigned)vmap.size(), fgrid = (unsigned)fmap.size(),
+                   fgrid64 = (unsigned)fmap64.size();
     auto apply32 = [&](int slot) -> int {
-        for (auto &G : groups) {
+        for (auto &G : groups32) {
             int r2 = launch_batched<float>(bs, G, d_a32, d_t32, 2, slot);
             if (r2) return r2;
         }
@@ -2454,11 +2624,11 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
         return FG_OK;
     };
     auto apply64 = [&]() -> int {
-        for (auto &G : groups) {
+        for (auto &G : groups64) {
             int r2 = launch_batched<double>(bs, G, d_a64, d_t64, 1, 0);
             if (r2) return r2;
         }
-        if (fgrid) fixup_batched_kernel<double><<<fgrid, 128, 0, bs>>>(d_f64, d_fm, 1, 0);
+        if (fgrid64) fixup_batched_kernel<double><<<fgrid64, 128, 0, bs>>>(d_f64, d_fm64, 1, 0);
         CK(cudaGetLastError());
         return FG_OK;
     };
@@ -2478,10 +2648,11 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
         CK(cudaGetLastError());
         return FG_OK;
     };
-    for (auto &G : groups)  // kernel attributes are set outside the graph capture
-        if ((rc = launch_batched<float>(bs, G, nullptr, nullptr, 2, 0)) ||
-            (rc = launch_batched<double>(bs, G, nullptr, nullptr, 1, 0)))
-            return rc;
+    // kernel attributes are set outside the graph capture
+    for (auto &G : groups32)
+        if ((rc = launch_batched<float>(bs, G, nullptr, nullptr, 2, 0))) return rc;
+    for (auto &G : groups64)
+        if ((rc = launch_batched<double>(bs, G, nullptr, nullptr, 1, 0))) return rc;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -2756,7 +2927,6 @@ FG_API int fg_vec_pupdate(fg_op *op, const double *z, double *p, const double *n
 // depends on allocator state.  The array lives in every GPU context that
 // loads the library until the process exits.
 // ---------------------------------------------------------------------------
-#define FG_NOALLOC_FACE_DOUBLES (4u << 20)  // 4 Mi doubles = 32 MiB
 static __device__ __align__(256) double g_noalloc_face[FG_NOALLOC_FACE_DOUBLES];
 // device address of g_noalloc_face per device, with the context it was resolved in
 static double *g_noalloc_face_ptr[64];
@@ -2798,12 +2968,13 @@ static int noalloc_scratch(int dev, double **out) {
     return FG_OK;
 }
 
-template <int P, int OPK>
+template <int P, int OPK, int LX>
 static int noalloc_launch_apply_t(fg_op *op, const Grid &g, const double *x, double *y,
                                   int accumulate, double *face) {
     using C = KCfg<P>;
-    using SM = ApplySmem<P, double, C::WY, C::S, stage_elems<P, OPK, 0>() / 32>;
-    auto kern = pa_apply_kernel<P, OPK, double, C::WY, C::S, C::MINB>;
+    constexpr int S = ring_stages<P, double, 0, LX>();
+    using SM = ApplySmem<P, double, C::WY, S, stage_elems<P, OPK, 0>() / 32, LX>;
+    auto kern = pa_apply_kernel<P, OPK, double, C::WY, S, C::MINB, 0, LX>;
     // per device, set once (as launch_apply_t does); racing setters are harmless
     static std::atomic<bool> attr_set[64];
     if (op->device < 0 || op->device >= 64) return fail(FG_CUDA_ERROR, "device id %d out of range", op->device);
@@ -2832,9 +3003,15 @@ template <int P>
 static int noalloc_launch_apply_p(fg_op *op, const Grid &g, const double *x, double *y,
                                   int accumulate, double *face) {
     switch (op->kind) {
-    case FG_MASS: return noalloc_launch_apply_t<P, 1>(op, g, x, y, accumulate, face);
-    case FG_DIFF: return noalloc_launch_apply_t<P, 2>(op, g, x, y, accumulate, face);
-    default: return noalloc_launch_apply_t<P, 3>(op, g, x, y, accumulate, face);
+    case FG_MASS:
+        return g.LX == 8 ? noalloc_launch_apply_t<P, 1, 8>(op, g, x, y, accumulate, face)
+                         : noalloc_launch_apply_t<P, 1, 32>(op, g, x, y, accumulate, face);
+    case FG_DIFF:
+        return g.LX == 8 ? noalloc_launch_apply_t<P, 2, 8>(op, g, x, y, accumulate, face)
+                         : noalloc_launch_apply_t<P, 2, 32>(op, g, x, y, accumulate, face);
+    default:
+        return g.LX == 8 ? noalloc_launch_apply_t<P, 3, 8>(op, g, x, y, accumulate, face)
+                         : noalloc_launch_apply_t<P, 3, 32>(op, g, x, y, accumulate, face);
     }
 }
 
@@ -2847,7 +3024,13 @@ extern "C" FG_API int fg_op_apply_native_noalloc(fg_op *op, const double *x, dou
     CK(cudaSetDevice(op->device));
     Grid g = op->g;
     g.ess = constrained ? op->ess_tags : 0;
-    const size_t need = (size_t)g.n_items() * (size_t)g.face_stride();
+    // the limit counts the face scratch of 32-wide tiles, whichever shape the
+    // operator uses (choose_tile keeps the chosen one inside it)
+    Grid w = g;
+    set_scratch_tiling(w);
+    if (op->tile_set) set_depth(w, g.TZ);
+    const size_t need = std::max((size_t)g.n_items() * (size_t)g.face_stride(),
+                                 (size_t)w.n_items() * (size_t)w.face_stride());
     if (need > FG_NOALLOC_FACE_DOUBLES)
         return fail(FG_INVALID_ARGUMENT,
                     "fg_op_apply_native_noalloc: this operator needs %zu doubles of face scratch, "

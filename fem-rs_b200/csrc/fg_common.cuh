@@ -59,7 +59,9 @@ __host__ __device__ constexpr int round_up(int a, int b) { return (a + b - 1) / 
 struct Grid {
     int nx, ny, nz, p;
     int NI, NJ, NK, NIp;   // DOF grid and padded row pitch
-    int WY, TZ;            // tile: 32 elements in x (one warp), WY rows in y, TZ layers in z
+    int LX;                // elements in x of a warp (32 or 8); its 32 / LX element rows in y
+    int NW;                // warps per tile
+    int WY, TZ;            // tile: LX elements in x, WY = NW * 32 / LX rows in y, TZ layers in z
     int ntx, nty, ntz;     // tiles per direction
     int ess;               // essential-face bits (tag t -> bit t-1: z0,z1,y0,y1,x0,x1)
     __host__ __device__ int64_t dof(int I, int J, int K) const {
@@ -71,10 +73,18 @@ struct Grid {
                ((ess & 16) && I == 0) || ((ess & 32) && I == NI - 1);
     }
     __host__ __device__ int n_items() const { return ntx * nty * ntz; }
+    // place of element (ex, ey, ez): item, warp of the item, layer, lane
+    __host__ __device__ void place(int ex, int ey, int ez, int &item, int &warp, int &lz, int &lane) const {
+        const int row = ey % WY, LY = 32 / LX;
+        item = ((ez / TZ) * nty + ey / WY) * ntx + ex / LX;
+        warp = row / LY;
+        lz = ez % TZ;
+        lane = (row % LY) * LX + ex % LX;
+    }
     // per-item face-slot sizes (x-hi, y-hi, z-hi planes of the item box)
     __host__ __device__ int fx() const { return (TZ * p + 1) * (WY * p + 1); }
-    __host__ __device__ int fy() const { return (TZ * p + 1) * (32 * p + 1); }
-    __host__ __device__ int fz() const { return (WY * p + 1) * (32 * p + 1); }
+    __host__ __device__ int fy() const { return (TZ * p + 1) * (LX * p + 1); }
+    __host__ __device__ int fz() const { return (WY * p + 1) * (LX * p + 1); }
     __host__ __device__ int face_stride() const { return fx() + fy() + fz(); }
 };
 

@@ -13,12 +13,12 @@
 //   B^T  the transposed contractions,
 //   E^T  a deterministic scatter with no floating-point atomics.
 //
-// Work decomposition.  A CTA owns an "item": a tile of 32 elements in x
-// (one warp, one element per lane) by WY element rows in y (one warp per row),
-// and sweeps TZ element layers in z.  Each thread keeps its element's
-// contractions in registers.  Contributions of neighbouring elements to the
-// DOFs they share are summed in a fixed order: across x by a warp shuffle,
-// across y through shared memory between the row warps, across z by carrying
+// Work decomposition.  A CTA owns an "item": WY warps of 32 elements (one per
+// lane), 32 in x or 8 in x by 4 in y (LX), stacked in y, and sweeps TZ element
+// layers in z.  Each thread keeps its element's contractions in registers.
+// Contributions of neighbouring elements to the DOFs they share are summed in
+// a fixed order: across x by a warp shuffle, across y by a shuffle inside a
+// warp and through shared memory between the warps, across z by carrying
 // the top DOF plane of a layer in shared memory into the next layer.  DOFs on
 // the three upper faces of an item that belong to a neighbouring item are
 // written to a per-item face buffer; fixup_kernel then adds them to the owner
@@ -65,13 +65,13 @@ template <int P, int OPK>
 __host__ __device__ inline int64_t qd_index(const Grid &g, int item, int w, int lz, int col,
                                             int qz, int comp, int lane) {
     constexpr int Q = P + 1, NC = NComp<OPK>::v;
-    return (((((int64_t)item * g.WY + w) * g.TZ + lz) * (Q * Q) + col) * Q + qz) * (NC * 32) +
+    return (((((int64_t)item * g.NW + w) * g.TZ + lz) * (Q * Q) + col) * Q + qz) * (NC * 32) +
            comp * 32 + lane;
 }
 template <int P, int OPK>
 __host__ __device__ inline int64_t qd_size(const Grid &g) {
     constexpr int Q = P + 1, NC = NComp<OPK>::v;
-    return (int64_t)g.n_items() * g.WY * g.TZ * Q * Q * Q * NC * 32;
+    return (int64_t)g.n_items() * g.NW * g.TZ * Q * Q * Q * NC * 32;
 }
 
 template <typename T> struct ApplyArgs {
@@ -113,25 +113,26 @@ template <int P, int OPK, int FMT>
 __host__ __device__ inline int64_t qd_size_fmt(const Grid &g) {
     // stages per layer: Q^2 columns (FMT 0) or 1 (FMT 1)
     constexpr int U = FMT == 0 ? (P + 1) * (P + 1) : 1;
-    return (int64_t)g.n_items() * g.WY * g.TZ * U * stage_elems<P, OPK, FMT>();
+    return (int64_t)g.n_items() * g.NW * g.TZ * U * stage_elems<P, OPK, FMT>();
 }
 
 // Shared-memory plan of the apply kernel (bytes).  NC here is the stage size
 // in units of 32-lane vectors.
-template <int P, typename T, int WY, int S, int NC> struct ApplySmem {
+// WY: warps per item; LX: elements in x of a warp (32 / LX element rows).
+template <int P, typename T, int WY, int S, int NC, int LX> struct ApplySmem {
     static constexpr int D = P + 1, Q = P + 1;
     // x tile buffers: two (the next layer's tile loads during this layer's
     // math) except for Q3 in FP64, where one buffer lets 3 CTAs share an SM
     static constexpr int NXB = (P == 3 && sizeof(T) == 8) ? FG_Q3_NXB : 2;
-    static constexpr int XW = round_up(32 * P + 1, 16 / (int)sizeof(T));
-    static constexpr int RY = WY * P + 1;
+    static constexpr int XW = round_up(LX * P + 1, 16 / (int)sizeof(T));
+    static constexpr int RY = WY * (32 / LX) * P + 1;
     static constexpr int XTILE = (P + 1) * RY * XW;               // elements
     static constexpr int XB = round_up(XTILE * (int)sizeof(T), 128);
     static constexpr int STAGE = NC * 32;                         // elements
     static constexpr int QB = STAGE * (int)sizeof(T);
     static constexpr int off_q = NXB * XB;
     static constexpr int off_y = off_q + WY * S * QB;
-    static constexpr int off_c = off_y + WY * D * D * 32 * (int)sizeof(T);
+    static constexpr int off_c = off_y + WY * D * D * LX * (int)sizeof(T);
     static constexpr int off_b = round_up(off_c + D * D * WY * 32 * (int)sizeof(T), 8);
     static constexpr int bytes = off_b + (2 + WY * S) * 8;
 };
@@ -143,36 +144,50 @@ template <int P, typename T, int WY, int S, int NC> struct ApplySmem {
 // neighbour item).  `essval(c,b,a)` returns the value written on essential
 // DOFs (x for the constrained apply, 1 for the diagonal).
 // ---------------------------------------------------------------------------
-template <int P, typename T, int WY, class EssVal>
+template <int P, typename T, int WY, int LX, class EssVal>
 __device__ __forceinline__ void merge_and_store(T (&out)[P + 1][P + 1][P + 1], const Grid &g,
                                                 T *ybuf, T *carry, int lz, int nl, int tz,
                                                 int warp, int lane, int item, bool valid,
-                                                int lane_last, int w_last, bool fx0, bool fx1,
+                                                int lx_last, int row_last, bool fx0, bool fx1,
                                                 bool fy0, bool fy1, bool fz0, bool fz1, T *y,
                                                 T *face, int accumulate, EssVal essval) {
     constexpr int D = P + 1;
     constexpr int NT = WY * 32;
-    // x: lane l receives the a=P face of lane l-1 into its a=0 face
+    constexpr int LY = 32 / LX;  // element rows of a warp: lane = ly * LX + lx
+    const int lx = lane % LX, ly = lane / LX, row = warp * LY + ly;
+    // x: element lx receives the a=P face of element lx-1 into its a=0 face
 #pragma unroll
     for (int c = 0; c < D; ++c)
 #pragma unroll
         for (int b = 0; b < D; ++b) {
             T v = __shfl_up_sync(0xffffffffu, out[c][b][P], 1);
-            if (lane > 0) out[c][b][0] += v;
+            if (lx > 0) out[c][b][0] += v;
         }
-    // y: row warp w receives the b=P row of warp w-1 into its b=0 row
-    T *yb = ybuf + warp * (D * D * 32);
-#pragma unroll
-    for (int c = 0; c < D; ++c)
-#pragma unroll
-        for (int a = 0; a < D; ++a) yb[(c * D + a) * 32 + lane] = out[c][P][a];
-    __syncthreads();
-    if (warp > 0) {
-        const T *yp = ybuf + (warp - 1) * (D * D * 32);
+    // y: an element row receives the b=P row of the row below into its b=0 row:
+    // inside the warp by a shuffle, from the warp below through shared memory
+    T *yb = ybuf + warp * (D * D * LX);
+    if (LY == 1 || ly == LY - 1) {
 #pragma unroll
         for (int c = 0; c < D; ++c)
 #pragma unroll
-            for (int a = 0; a < D; ++a) out[c][0][a] += yp[(c * D + a) * 32 + lane];
+            for (int a = 0; a < D; ++a) yb[(c * D + a) * LX + lx] = out[c][P][a];
+    }
+    if constexpr (LY > 1) {
+#pragma unroll
+        for (int c = 0; c < D; ++c)
+#pragma unroll
+            for (int a = 0; a < D; ++a) {
+                const T v = __shfl_up_sync(0xffffffffu, out[c][P][a], LX);
+                if (ly > 0) out[c][0][a] += v;
+            }
+    }
+    __syncthreads();
+    if (warp > 0 && (LY == 1 || ly == 0)) {
+        const T *yp = ybuf + (warp - 1) * (D * D * LX);
+#pragma unroll
+        for (int c = 0; c < D; ++c)
+#pragma unroll
+            for (int a = 0; a < D; ++a) out[c][0][a] += yp[(c * D + a) * LX + lx];
     }
     // z: layer lz receives the c=P plane of layer lz-1 into its c=0 plane
     const int tid = warp * 32 + lane;
@@ -190,9 +205,9 @@ __device__ __forceinline__ void merge_and_store(T (&out)[P + 1][P + 1][P + 1], c
     }
     if (!valid) return;
     const int tx = item % g.ntx, ty = (item / g.ntx) % g.nty;
-    const int I0 = tx * 32 * P, J0 = ty * WY * P, K0 = tz * g.TZ * P;
-    const int ex = tx * 32 + lane, ey = ty * WY + warp, ez = tz * g.TZ + lz;
-    const int SX = 32 * P + 1, SY = WY * P + 1;
+    const int I0 = tx * LX * P, J0 = ty * (WY * LY) * P, K0 = tz * g.TZ * P;
+    const int ex = tx * LX + lx, ey = ty * (WY * LY) + row, ez = tz * g.TZ + lz;
+    const int SX = LX * P + 1, SY = WY * LY * P + 1;
     T *fxp = face + (int64_t)item * g.face_stride();
     T *fyp = fxp + g.fx();
     T *fzp = fyp + g.fy();
@@ -204,13 +219,13 @@ __device__ __forceinline__ void merge_and_store(T (&out)[P + 1][P + 1][P + 1], c
         const bool zhi = (c == P) && (ez != g.nz - 1);
 #pragma unroll
         for (int b = 0; b < D; ++b) {
-            if (b == P && warp != w_last) continue;
-            const int J = J0 + P * warp + b;
+            if (b == P && row != row_last) continue;
+            const int J = J0 + P * row + b;
             const bool yhi = (b == P) && (ey != g.ny - 1);
 #pragma unroll
             for (int a = 0; a < D; ++a) {
-                if (a == P && lane != lane_last) continue;
-                const int I = I0 + P * lane + a;
+                if (a == P && lx != lx_last) continue;
+                const int I = I0 + P * lx + a;
                 const bool xhi = (a == P) && (ex != g.nx - 1);
                 T v = out[c][b][a];
                 if (xhi) {
@@ -234,7 +249,7 @@ __device__ __forceinline__ void merge_and_store(T (&out)[P + 1][P + 1][P + 1], c
 // ---------------------------------------------------------------------------
 // The apply kernel.
 // ---------------------------------------------------------------------------
-template <int P, int OPK, typename T, int WY, int S, int FMT>
+template <int P, int OPK, typename T, int WY, int S, int FMT, int LX>
 __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const ApplyArgs<T> &A,
                                               const int item) {
     constexpr int D = P + 1, Q = P + 1, NC = NComp<OPK>::v;
@@ -242,7 +257,7 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
     constexpr int COLS = Q * Q;
     constexpr int UPL = FMT == 0 ? COLS : 1;  // stream units per layer
     constexpr int NCE = AffineComp<OPK>::NCE, NCQ = AffineComp<OPK>::NCQ;
-    using SM = ApplySmem<P, T, WY, S, stage_elems<P, OPK, FMT>() / 32>;
+    using SM = ApplySmem<P, T, WY, S, stage_elems<P, OPK, FMT>() / 32, LX>;
     constexpr int STAGE = SM::STAGE, XW = SM::XW, RY = SM::RY;
     using TB = Tab<T>;
 
@@ -261,12 +276,16 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tx = item % g.ntx, ty = (item / g.ntx) % g.nty, tz = item / (g.ntx * g.nty);
     const int nl = min(g.TZ, g.nz - tz * g.TZ);
-    const int ex = tx * 32 + lane, ey = ty * WY + warp;
+    constexpr int LY = 32 / LX, ROWS = WY * LY;
+    const int lx = lane % LX, row = warp * LY + lane / LX;  // element of the item's cross-section
+    const int ex = tx * LX + lx, ey = ty * ROWS + row;
     const bool valid = ex < g.nx && ey < g.ny;
-    const int lane_last = min(31, g.nx - 1 - tx * 32);
-    const int w_last = min(WY - 1, g.ny - 1 - ty * WY);
-    const int I0 = tx * 32 * P, J0 = ty * WY * P, K0 = tz * g.TZ * P;
-    const int total_cols = nl * UPL;
+    const int lx_last = min(LX - 1, g.nx - 1 - tx * LX);
+    const int row_last = min(ROWS - 1, g.ny - 1 - ty * ROWS);
+    const int I0 = tx * LX * P, J0 = ty * ROWS * P, K0 = tz * g.TZ * P;
+    // a warp of several rows that holds no element streams and computes nothing
+    const bool wlive = LX == 32 || ty * ROWS + warp * LY < g.ny;
+    const int total_cols = wlive ? nl * UPL : 0;
     const T *qdw = A.qd + (int64_t)(item * WY + warp) * g.TZ * UPL * STAGE;
     T *qsw = qs + warp * S * STAGE;
     uint64_t *qbw = qbar + warp * S;
@@ -320,6 +339,7 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
                                                   xb * SM::XB);
 
         T out[D][D][D];
+        if (wlive) {
         if constexpr (HK && ((std::is_same<T, float>::value &&
                                ((P == 1 && FG_Q1_COLLOC) || (P == 2 && FG_F32_Q2_COLLOC) ||
                                 (P == 3 && FMT == 1 && FG_F32_Q3_COLLOC))) ||
@@ -346,7 +366,7 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
                 float2 up[NPC][D][D];
                 float us[D][D];
                 auto ld = [&](int c, int b, int a) -> float {
-                    const float v = xt[(c * RY + warp * P + b) * XW + lane * P + a];
+                    const float v = xt[(c * RY + row * P + b) * XW + lx * P + a];
                     const bool e = (a == 0 && fx0) || (a == P && fx1) || (b == 0 && fy0) || (b == P && fy1) ||
                                    (c == 0 && fz0) || (c == P && fz1);
                     return e ? 0.f : v;
@@ -422,7 +442,7 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
                     for (int b = 0; b < D; ++b)
 #pragma unroll
                         for (int a = 0; a < D; ++a) {
-                            const T v = xt[(c * RY + warp * P + b) * XW + lane * P + a];
+                            const T v = xt[(c * RY + row * P + b) * XW + lx * P + a];
                             const bool e = (a == 0 && fx0) || (a == P && fx1) || (b == 0 && fy0) ||
                                            (b == P && fy1) || (c == 0 && fz0) || (c == P && fz1);
                             u[c][b][a] = e ? T(0) : v;
@@ -663,7 +683,7 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
                 for (int b = 0; b < D; ++b)
 #pragma unroll
                     for (int a = 0; a < D; ++a) {
-                        const float v = xt[(c * RY + warp * P + b) * XW + lane * P + a];
+                        const float v = xt[(c * RY + row * P + b) * XW + lx * P + a];
                         const bool e = (a == 0 && fx0) || (a == P && fx1) || (b == 0 && fy0) ||
                                        (b == P && fy1) || (c == 0 && fz0) || (c == P && fz1);
                         u[c][b][a] = e ? 0.f : v;
@@ -819,7 +839,7 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
                 for (int b = 0; b < D; ++b)
     #pragma unroll
                     for (int a = 0; a < D; ++a) {
-                        const T v = xt[(c * RY + warp * P + b) * XW + lane * P + a];
+                        const T v = xt[(c * RY + row * P + b) * XW + lx * P + a];
                         const bool e = (a == 0 && fx0) || (a == P && fx1) || (b == 0 && fy0) ||
                                        (b == P && fy1) || (c == 0 && fz0) || (c == P && fz1);
                         u[c][b][a] = e ? T(0) : v;
@@ -1006,7 +1026,7 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
                     for (int a = 0; a < D; ++a) out[c][b][a] = T(0);
             // (a per-element branch around the mask measured slower than the
             // predicated form: it splits the unrolled code in two)
-            const T *xe = xt + (warp * P) * XW + lane * P;
+            const T *xe = xt + (row * P) * XW + lx * P;
             auto uval = [&](int c, int b, int a) -> T {
                 const T v = xe[(c * RY + b) * XW + a];
                 const bool e = (a == 0 && fx0) || (a == P && fx1) || (b == 0 && fy0) || (b == P && fy1) ||
@@ -1181,11 +1201,19 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
                 }
             }
         }
+        } else {
+#pragma unroll
+            for (int c = 0; c < D; ++c)
+#pragma unroll
+                for (int b = 0; b < D; ++b)
+#pragma unroll
+                    for (int a = 0; a < D; ++a) out[c][b][a] = T(0);
+        }
         // ---- E^T: merge + store --------------------------------------------
-        merge_and_store<P, T, WY>(
-            out, g, ybuf, carry, lz, nl, tz, warp, lane, item, valid, lane_last, w_last, fx0, fx1,
+        merge_and_store<P, T, WY, LX>(
+            out, g, ybuf, carry, lz, nl, tz, warp, lane, item, valid, lx_last, row_last, fx0, fx1,
             fy0, fy1, fz0, fz1, A.y, A.face, A.accumulate,
-            [&](int c, int b, int a) { return xt[(c * RY + warp * P + b) * XW + lane * P + a]; });
+            [&](int c, int b, int a) { return xt[(c * RY + row * P + b) * XW + lx * P + a]; });
         __syncthreads();
     }
     // After a timeout, drain the copies this thread issued and has not seen
@@ -1199,10 +1227,10 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
 }
 
 // Single operator: one CTA per item; the x tile map is a kernel parameter.
-template <int P, int OPK, typename T, int WY, int S, int MINB, int FMT = 0>
+template <int P, int OPK, typename T, int WY, int S, int MINB, int FMT, int LX>
 __global__ void __launch_bounds__(WY * 32, MINB)
     pa_apply_kernel(const __grid_constant__ CUtensorMap xmap, const ApplyArgs<T> A) {
-    pa_apply_body<P, OPK, T, WY, S, FMT>(&xmap, A, A.item0 + blockIdx.x);
+    pa_apply_body<P, OPK, T, WY, S, FMT, LX>(&xmap, A, A.item0 + blockIdx.x);
 }
 
 // Batched operators (many independent instances of the same order, kind and
@@ -1215,11 +1243,11 @@ template <typename T> struct BatchApply {
     const int2 *bmap;            // [block] -> (instance, item)
     int nslots, slot;
 };
-template <int P, int OPK, typename T, int WY, int S, int MINB, int FMT = 0>
+template <int P, int OPK, typename T, int WY, int S, int MINB, int FMT, int LX>
 __global__ void __launch_bounds__(WY * 32, MINB) pa_apply_batched_kernel(const BatchApply<T> B) {
     const int2 m = B.bmap[blockIdx.x];
     const int k = m.x * B.nslots + B.slot;
-    pa_apply_body<P, OPK, T, WY, S, FMT>(&B.tmaps[k], B.args[k], m.y);
+    pa_apply_body<P, OPK, T, WY, S, FMT, LX>(&B.tmaps[k], B.args[k], m.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -1227,22 +1255,23 @@ __global__ void __launch_bounds__(WY * 32, MINB) pa_apply_batched_kernel(const B
 // element diagonal sum_q g_i^T D_q g_i (+ m_q phi_i^2) is formed directly from
 // the quadrature data in global memory (a setup-time kernel).
 // ---------------------------------------------------------------------------
-template <int P, int OPK, typename T, int WY>
+template <int P, int OPK, typename T, int WY, int LX>
 __global__ void __launch_bounds__(WY * 32) pa_diag_kernel(const ApplyArgs<T> A) {
     constexpr int D = P + 1, Q = P + 1, NC = NComp<OPK>::v;
     constexpr bool HM = (OPK & 1) != 0, HK = (OPK & 2) != 0;
     using TB = Tab<T>;
     const Grid g = A.g;
-    __shared__ T ybuf[WY * D * D * 32];
+    __shared__ T ybuf[WY * D * D * LX];
     __shared__ T carry[D * D * WY * 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.x;
     const int tx = item % g.ntx, ty = (item / g.ntx) % g.nty, tz = item / (g.ntx * g.nty);
     const int nl = min(g.TZ, g.nz - tz * g.TZ);
-    const int ex = tx * 32 + lane, ey = ty * WY + warp;
+    constexpr int LY = 32 / LX, ROWS = WY * LY;
+    const int ex = tx * LX + lane % LX, ey = ty * ROWS + warp * LY + lane / LX;
     const bool valid = ex < g.nx && ey < g.ny;
-    const int lane_last = min(31, g.nx - 1 - tx * 32);
-    const int w_last = min(WY - 1, g.ny - 1 - ty * WY);
+    const int lx_last = min(LX - 1, g.nx - 1 - tx * LX);
+    const int row_last = min(ROWS - 1, g.ny - 1 - ty * ROWS);
     const int ess = g.ess;
     const bool fx0 = (ess & 16) && ex == 0, fx1 = (ess & 32) && ex == g.nx - 1;
     const bool fy0 = (ess & 4) && ey == 0, fy1 = (ess & 8) && ey == g.ny - 1;
@@ -1286,8 +1315,8 @@ __global__ void __launch_bounds__(WY * 32) pa_diag_kernel(const ApplyArgs<T> A) 
                                 out[c][b][a] += s;
                             }
                 }
-        merge_and_store<P, T, WY>(out, g, ybuf, carry, lz, nl, tz, warp, lane, item, valid,
-                                  lane_last, w_last, fx0, fx1, fy0, fy1, fz0, fz1, A.y, A.face, 0,
+        merge_and_store<P, T, WY, LX>(out, g, ybuf, carry, lz, nl, tz, warp, lane, item, valid,
+                                  lx_last, row_last, fx0, fx1, fy0, fy1, fz0, fz1, A.y, A.face, 0,
                                   [](int, int, int) { return T(1); });
         __syncthreads();
     }
@@ -1313,7 +1342,7 @@ template <bool CG, typename T> __device__ __forceinline__ T ld_face(const T *p) 
 template <typename T, bool CG = false>
 __device__ __forceinline__ T fixup_acc(const Grid &g, int I, int J, int K, int tx, int ty, int tz,
                                        int sx, int sy, int sz, T own, const T *__restrict__ face) {
-    const int SXe = 32 * g.p, SYe = g.WY * g.p, SZe = g.TZ * g.p;
+    const int SXe = g.LX * g.p, SYe = g.WY * g.p, SZe = g.TZ * g.p;
     const int fs = g.face_stride(), fxs = g.fx(), fys = g.fy();
     T sum = own;
     for (int dz = 0; dz <= sz; ++dz)
@@ -1344,14 +1373,14 @@ __host__ __device__ inline int fixup_rows(const Grid &g) {
 // One row of the fix-up, by the whole block.  Everything fixed along the row
 // (its plane, the owner item across the plane, the essential faces it lies on)
 // is worked out once; per DOF only the position along the row is classified,
-// by a division by the compile-time 32 P.  A DOF (I, J, K) with sx = (0 < I < NI-1
-// and I % 32P == 0), sy, sz alike, owned by item (min(I / 32P, ntx-1), ...), gets
+// by a division by the compile-time LX P.  A DOF (I, J, K) with sx = (0 < I < NI-1
+// and I % LX P == 0), sy, sz alike, owned by item (min(I / LX P, ntx-1), ...), gets
 // the sum of fixup_acc.  y planes skip DOFs on x planes, z planes skip DOFs on x or
 // y planes; essential DOFs keep the owner's value.
-template <typename T, int P>
+template <typename T, int P, int LX>
 __device__ __forceinline__ void fixup_row_t(const Grid &g, int r, T *__restrict__ y,
                                             const T *__restrict__ face) {
-    constexpr int SXe = 32 * P;
+    constexpr int SXe = LX * P;
     const int SYe = g.WY * P, SZe = g.TZ * P;
     const int rx = (g.ntx - 1) * g.NK, ry = (g.nty - 1) * g.NK;
     const int ess = g.ess;
@@ -1397,10 +1426,13 @@ __device__ __forceinline__ void fixup_row_t(const Grid &g, int r, T *__restrict_
 template <typename T>
 __device__ __forceinline__ void fixup_row(const Grid &g, int r, T *__restrict__ y,
                                           const T *__restrict__ face) {
-    switch (g.p) {
-    case 1: fixup_row_t<T, 1>(g, r, y, face); break;
-    case 2: fixup_row_t<T, 2>(g, r, y, face); break;
-    default: fixup_row_t<T, 3>(g, r, y, face); break;
+    switch (g.LX + g.p) {
+    case 32 + 1: fixup_row_t<T, 1, 32>(g, r, y, face); break;
+    case 32 + 2: fixup_row_t<T, 2, 32>(g, r, y, face); break;
+    case 32 + 3: fixup_row_t<T, 3, 32>(g, r, y, face); break;
+    case 8 + 1: fixup_row_t<T, 1, 8>(g, r, y, face); break;
+    case 8 + 2: fixup_row_t<T, 2, 8>(g, r, y, face); break;
+    default: fixup_row_t<T, 3, 8>(g, r, y, face); break;
     }
 }
 
@@ -1410,7 +1442,7 @@ __device__ __forceinline__ void fixup_row(const Grid &g, int r, T *__restrict__ 
 template <typename T, int P>
 __device__ __forceinline__ void fixup_owner(const Grid &g, T *y, const T *face, int ox, int oy,
                                             int oz) {
-    constexpr int SXe = 32 * P;
+    const int SXe = g.LX * P;
     const int SYe = g.WY * P, SZe = g.TZ * P;
     const int I0 = ox * SXe, J0 = oy * SYe, K0 = oz * SZe;
     const int I1 = ox == g.ntx - 1 ? g.NI - 1 : I0 + SXe - 1;
@@ -1550,13 +1582,13 @@ struct SetupArgs {
     int *err;
 };
 
-// Re-layout of full-format quadrature data for another z extent of the items
-// (TZ): the data of element e, point (col, qz), component c moves from its
-// place under grid go to its place under grid gn (same mesh, same WY).  One
+// Re-layout of full-format quadrature data for another tile shape (and
+// precision): the data of element e, point (col, qz), component c moves from
+// its place under grid go to its place under grid gn (same mesh).  One
 // thread per (element, point); pads of the new layout stay as initialised.
-template <int P, int OPK>
+template <int P, int OPK, typename T>
 __global__ void qdata_relayout_kernel(const Grid go, const Grid gn, const double *__restrict__ src,
-                                      double *__restrict__ dst) {
+                                      T *__restrict__ dst) {
     constexpr int Q = P + 1, NC = NComp<OPK>::v;
     const int64_t total = (int64_t)go.nx * go.ny * go.nz * Q * Q * Q;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -1564,24 +1596,24 @@ __global__ void qdata_relayout_kernel(const Grid go, const Grid gn, const double
         const int64_t e = t / (Q * Q * Q);
         const int col = cq / Q, qz = cq % Q;
         const int ex = (int)(e % go.nx), ey = (int)((e / go.nx) % go.ny), ez = (int)(e / ((int64_t)go.nx * go.ny));
-        const int tx = ex / 32, lane = ex % 32, ty = ey / go.WY, wy = ey % go.WY;
-        const int io = ((ez / go.TZ) * go.nty + ty) * go.ntx + tx, lo = ez % go.TZ;
-        const int in = ((ez / gn.TZ) * gn.nty + ty) * gn.ntx + tx, ln = ez % gn.TZ;
-        const double *s = src + qd_index<P, OPK>(go, io, wy, lo, col, qz, 0, lane);
-        double *d = dst + qd_index<P, OPK>(gn, in, wy, ln, col, qz, 0, lane);
+        int io, lo, wo, ao, in, ln, wn, an;
+        go.place(ex, ey, ez, io, wo, lo, ao);
+        gn.place(ex, ey, ez, in, wn, ln, an);
+        const double *s = src + qd_index<P, OPK>(go, io, wo, lo, col, qz, 0, ao);
+        T *d = dst + qd_index<P, OPK>(gn, in, wn, ln, col, qz, 0, an);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) d[c * 32] = s[c * 32];
+        for (int c = 0; c < NC; ++c) d[c * 32] = (T)s[c * 32];
     }
 }
 
 // Affine-compressed quadrature data (FMT 1) derived from the full FP64 data:
 // on an element with constant J every D_q is w_q kappa_q times the same
 // symmetric matrix |detJ| J^-1 J^-T, so G_e = D_{q0} and s_q = tr(D_q)/tr(D_{q0})
-// reproduce D_q = s_q G_e.  Each thread (element, quadrature point) checks
+// reproduce D_q = s_q G_e.  g: tile shape of the full data, ga: of the result.  Each thread (element, quadrature point) checks
 // that identity to 1e-10 relative and raises FG_DERR_BOUNDS otherwise (the
 // mesh is not affine: the format is refused).  The mass scalar is copied.
 template <int P, int OPK, typename T>
-__global__ void qdata_compress_kernel(const Grid g, const double *__restrict__ qfull,
+__global__ void qdata_compress_kernel(const Grid g, const Grid ga, const double *__restrict__ qfull,
                                       T *__restrict__ qaff, int *err) {
     constexpr int Q = P + 1, NC = NComp<OPK>::v;
     constexpr bool HM = (OPK & 1) != 0, HK = (OPK & 2) != 0;
@@ -1595,13 +1627,14 @@ __global__ void qdata_compress_kernel(const Grid g, const double *__restrict__ q
         const int64_t e = t / (Q * Q * Q);
         const int qx = q % Q, qy = (q / Q) % Q, qz = q / (Q * Q);
         const int ex = (int)(e % g.nx), ey = (int)((e / g.nx) % g.ny), ez = (int)(e / ((int64_t)g.nx * g.ny));
-        const int tx = ex / 32, lane = ex % 32, ty = ey / g.WY, wy = ey % g.WY, tz = ez / g.TZ,
-                  lz = ez % g.TZ;
-        const int item = (tz * g.nty + ty) * g.ntx + tx;
+        int item, wy, lz, lane;
+        g.place(ex, ey, ez, item, wy, lz, lane);
         const int col = qy * Q + qx;
         const double *src = qfull + qd_index<P, OPK>(g, item, wy, lz, col, qz, 0, lane);
         const double *src0 = qfull + qd_index<P, OPK>(g, item, wy, lz, 0, 0, 0, lane);
-        T *base = qaff + ((((int64_t)item * g.WY + wy) * g.TZ + lz) * STG) + lane;
+        int ia, wa, la, na;
+        ga.place(ex, ey, ez, ia, wa, la, na);
+        T *base = qaff + ((((int64_t)ia * ga.NW + wa) * ga.TZ + la) * STG) + na;
         T *qq = base + (NCE + (col * Q + qz) * NCQ) * 32;
         if (HK) {
             const double tr = src[0] + src[96] + src[160];
@@ -1699,9 +1732,8 @@ __global__ void qdata_setup_kernel(const SetupArgs S, T *__restrict__ qd) {
         const double rho = S.rho_q ? S.rho_q[e * (Q * Q * Q) + q] : S.rho_c;
         double D[6], m;
         if (!hex_point_qdata(xv, xi, w, kap, S.c_k, rho, S.c_m, D, m) && S.err) atomicOr(S.err, FG_DERR_BOUNDS);
-        const int tx = ex / 32, lane = ex % 32, ty = ey / g.WY, wy = ey % g.WY, tz = ez / g.TZ,
-                  lz = ez % g.TZ;
-        const int item = (tz * g.nty + ty) * g.ntx + tx;
+        int item, wy, lz, lane;
+        g.place(ex, ey, ez, item, wy, lz, lane);
         T *dst = qd + qd_index<P, OPK>(g, item, wy, lz, qy * Q + qx, qz, 0, lane);
         if (HK)
             for (int k = 0; k < 6; ++k) dst[k * 32] = (T)D[k];

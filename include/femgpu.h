@@ -363,11 +363,14 @@ FG_API int fg_op_collect_residuals(fg_op *op, const double *b, const fg_cfg *cfg
 FG_API int fg_unet_train_energy(fg_unet *net, fg_op *op, const double *res, int B, float lr, float *loss);
 
 /* ---- tile shape and the batched autotuner ------------------------------------ */
-/* An apply work item (one CTA's unit) is a box of 32 x WY x TZ elements; WY is
- * fixed per order, TZ (layers per item) is chosen at creation (8, halved until
- * there are >= 592 items) and can be changed: fg_op_set_tile re-lays out the
- * quadrature data on the device.  fg_op_tile returns {32, WY, TZ}.  No
- * reference counterpart (tuning of this library's kernels). */
+/* An apply work item (one CTA's unit) is a box of LX x WY x TZ elements: a warp
+ * holds 32 elements, 32 in x (LX = 32) or 8 in x by 4 in y (LX = 8), an item has
+ * 4 warps (order 3: 2).  LX and TZ (layers per item) are chosen at creation for
+ * each precision and quadrature-data format from the mesh's extents; TZ can be
+ * changed: fg_op_set_tile re-lays out the quadrature data on the device and
+ * applies to all forms.  fg_op_tile returns {LX, WY, TZ} of the FP64 apply in the
+ * handle's format.  Environment, read by fg_op_create: FG_LANES_X=8 or 32 fixes
+ * LX.  No reference counterpart (tuning of this library's kernels). */
 FG_API int fg_op_set_tile(fg_op *op, int tz);
 FG_API int fg_op_tile(const fg_op *op, int dims[3]);
 
