@@ -63,6 +63,7 @@ static int fail(int status, const char *fmt, ...) {
             return fail(FG_UNSUPPORTED, "%s needs a structured hex box (fg_op_create)", what); \
     } while (0)
 
+#include "chunk_host.cuh"
 #include "unet_host.cuh"
 #include "tet_host.cuh"
 
@@ -272,18 +273,11 @@ struct fg_op {
     struct NnTimes { int ir, fmt, degree; double plain_ms, learned_ms; };
     std::vector<NnTimes> nn_times;
     int fmt = 0;
-    // unstructured Hex8 mesh (fg_op_create_hex): element maps in the chunk
-    // order, the chunk scatter's lists, essential-DOF mask; vectors are plain
-    // (no pads)
+    // unstructured Hex8 mesh (fg_op_create_hex): element maps and slot lists in the
+    // chunk order; vectors are plain (no pads)
     bool unstr = false;
-    int64_t u_E = 0, u_chunks = 0, u_nshared = 0;
-    int u_max_nu = 0;
-    int32_t *u_dofs = nullptr;
-    uint8_t *u_ess = nullptr;
-    uint64_t *u_emsk = nullptr;  // [E] essential local DOFs of each element (bit k)
-    int32_t *u_cu_off = nullptr, *u_cu_dof = nullptr, *u_cu_pid = nullptr, *u_cu_soff = nullptr;
-    int32_t *u_sh_dof = nullptr, *u_sh_off = nullptr;
-    uint16_t *u_cu_slots = nullptr;
+    int64_t u_E = 0, u_chunks = 0;
+    ChunkBufs u_lists;
     double *u_part = nullptr;  // partials of the shared DOFs (FP64 or FP32 applies)
     double *qa64 = nullptr;
     float *qa32 = nullptr;
@@ -309,14 +303,8 @@ static void free_op(fg_op *op) {
     double *bufs[] = {op->qd, op->face, op->xs, op->ys, op->dinv, op->ones, op->r, op->z, op->pv, op->ap,
                       op->xw, op->bw, op->cres, op->cd, op->ct, op->partials, op->stage};
     if (op->fixcnt) cudaFree(op->fixcnt);
-    if (op->u_dofs) cudaFree(op->u_dofs);
-    if (op->u_ess) cudaFree(op->u_ess);
-    {
-        void *u[] = {op->u_emsk, op->u_cu_off, op->u_cu_dof, op->u_cu_pid, op->u_cu_soff, op->u_sh_dof, op->u_sh_off,
-                     op->u_cu_slots, op->u_part};
-        for (void *q : u)
-            if (q) cudaFree(q);
-    }
+    op->u_lists.release();
+    if (op->u_part) cudaFree(op->u_part);
     for (int k = 0; k < CHEB_MAXD; ++k) {
         if (op->cdk[k]) cudaFree(op->cdk[k]);
         if (op->cdk32[k]) cudaFree(op->cdk32[k]);
@@ -3770,46 +3758,22 @@ FG_API int fg_tet_create(int order, int64_t n_nodes, const double *coords, int64
         if (v >= 32 && v <= 1024 && v * nl <= 65536) t->CE = v;
     }
     if (const char *ev = std::getenv("FG_TET_WIDE")) t->wide = std::atoi(ev) != 0;
+    std::vector<uint8_t> he;
+    if (ess) {
+        he.resize(n_dofs);
+        CK(cudaMemcpy(he.data(), ess, n_dofs, cudaMemcpyDefault));
+    }
     ChunkPlan plan;
     std::vector<int32_t> perm;
-    tet_plan_chunks(h, hc, n_elem, n_dofs, nl, t->CE, perm, plan);
+    tet_plan_chunks(h, hc, n_elem, n_dofs, nl, t->CE, ess ? he.data() : nullptr, perm, plan);
     t->n_chunks = (int)plan.n_chunks;
-    t->max_nu = plan.max_nu;
-    if (tet_chunk_smem(nl, t->CE, t->max_nu) > 227 * 1024)
+    if (tet_chunk_smem(nl, t->CE, plan.max_nu) > 227 * 1024)
         return fail(FG_UNSUPPORTED, "tet chunk of %d elements needs too much shared memory", t->CE);
-    t->n_shared = (int64_t)plan.sh_dof.size();
-    t->n_part = plan.n_part;
-    if ((rc = tet_upload(&t->dofs, soa.data(), soa.size())) ||
-        (rc = tet_upload(&t->cu_slots, plan.cu_slots.data(), plan.cu_slots.size())) ||
-        (rc = tet_upload(&t->cu_off, plan.cu_off.data(), plan.cu_off.size())) ||
-        (rc = tet_upload(&t->cu_dof, plan.cu_dof.data(), plan.cu_dof.size())) ||
-        (rc = tet_upload(&t->cu_pid, plan.cu_pid.data(), plan.cu_pid.size())) ||
-        (rc = tet_upload(&t->cu_soff, plan.cu_soff.data(), plan.cu_soff.size())) ||
-        (rc = tet_upload(&t->sh_dof, plan.sh_dof.data(), plan.sh_dof.size())) ||
-        (rc = tet_upload(&t->sh_off, plan.sh_off.data(), plan.sh_off.size())) ||
+    t->has_ess = ess != nullptr;
+    if ((rc = tet_upload(&t->dofs, soa.data(), soa.size())) || (rc = t->lists.upload(plan)) ||
         (rc = tet_upload(&t->coords, coords, (size_t)n_nodes * 3)))
         return rc;
-    CK(cudaMalloc(&t->part, sizeof(double) * std::max<int64_t>(t->n_part, 1)));
-    {   // element map and essential local DOFs in the chunk order
-        std::vector<int32_t> ed(h.size());
-        std::vector<uint8_t> he;
-        if (ess) {
-            he.resize(n_dofs);
-            CK(cudaMemcpy(he.data(), ess, n_dofs, cudaMemcpyDefault));
-        }
-        std::vector<uint32_t> em(ess ? n_elem : 0, 0u);
-        for (int64_t n = 0; n < n_elem; ++n) {
-            const int64_t e = perm[n];
-            for (int i = 0; i < nl; ++i) {
-                const int32_t d = h[e * nl + i];
-                ed[(int64_t)i * n_elem + n] = d;
-                if (ess && he[d]) em[n] |= 1u << i;
-            }
-        }
-        if ((rc = tet_upload(&t->edof, ed.data(), ed.size()))) return rc;
-        if (ess && (rc = tet_upload(&t->emsk, em.data(), em.size()))) return rc;
-    }
-    if (ess && (rc = tet_upload(&t->ess, ess, (size_t)n_dofs))) return rc;
+    CK(cudaMalloc(&t->part, sizeof(double) * std::max<int64_t>(plan.n_part, 1)));
     // rule tables
     std::vector<double> pts, w;
     t->nq = tet_rule_host(quad_order, pts, w);
@@ -3894,7 +3858,7 @@ FG_API int fg_tet_quadrature_points(fg_tet *t, double *xyz, int mem) {
 FG_API int fg_tet_apply(fg_tet *t, const double *x, double *y, int accumulate, int constrained, int mem) {
     if (!t || !x || !y) return fail(FG_INVALID_ARGUMENT, "NULL argument");
     if (mem != FG_HOST && mem != FG_DEVICE) return fail(FG_INVALID_ARGUMENT, "bad mem %d", mem);
-    if (constrained && !t->ess) return fail(FG_INVALID_ARGUMENT, "constrained apply needs the essential mask");
+    if (constrained && !t->has_ess) return fail(FG_INVALID_ARGUMENT, "constrained apply needs the essential mask");
     std::lock_guard<std::mutex> lk(t->mu);
     CK(cudaSetDevice(t->device));
     const double *xd = x;
@@ -3917,7 +3881,7 @@ FG_API int fg_tet_apply(fg_tet *t, const double *x, double *y, int accumulate, i
 
 FG_API int fg_tet_apply_native(fg_tet *t, const double *x, double *y, int accumulate, int constrained) {
     if (!t || !x || !y) return fail(FG_INVALID_ARGUMENT, "NULL argument");
-    if (constrained && !t->ess) return fail(FG_INVALID_ARGUMENT, "constrained apply needs the essential mask");
+    if (constrained && !t->has_ess) return fail(FG_INVALID_ARGUMENT, "constrained apply needs the essential mask");
     std::lock_guard<std::mutex> lk(t->mu);
     CK(cudaSetDevice(t->device));
     return tet_launch_apply(t, x, y, accumulate, constrained, 0);
@@ -3945,7 +3909,7 @@ FG_API int fg_tet_check(fg_tet *t) {
 FG_API int fg_tet_diagonal(fg_tet *t, double *d, int constrained, int mem) {
     if (!t || !d) return fail(FG_INVALID_ARGUMENT, "NULL argument");
     if (mem != FG_HOST && mem != FG_DEVICE) return fail(FG_INVALID_ARGUMENT, "bad mem %d", mem);
-    if (constrained && !t->ess) return fail(FG_INVALID_ARGUMENT, "constrained diagonal needs the essential mask");
+    if (constrained && !t->has_ess) return fail(FG_INVALID_ARGUMENT, "constrained diagonal needs the essential mask");
     std::lock_guard<std::mutex> lk(t->mu);
     CK(cudaSetDevice(t->device));
     double *dd = d;

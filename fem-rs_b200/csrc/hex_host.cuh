@@ -5,7 +5,7 @@
 // fg_op whose applies and diagonal go through hex_kernels.cuh, so fg_op_apply,
 // fg_op_diagonal and fg_pcg serve both mesh kinds.
 #pragma once
-#include "chunk_plan.h"
+#include "chunk_host.cuh"
 #include "hex_kernels.cuh"
 
 // Warps per CTA (a chunk is WARPS * 32 elements), stages of the per-warp
@@ -23,10 +23,7 @@ static HexApply<T> hex_args(fg_op *op, const T *qd, const T *x, T *y, int accumu
     HexApply<T> A{};
     A.E = op->u_E;
     A.N = op->N;
-    A.dofs = op->u_dofs;
     A.qd = qd;
-    A.ess = op->u_ess;
-    A.emsk = op->u_emsk;
     A.x = x;
     A.y = y;
     A.accumulate = accumulate;
@@ -34,16 +31,7 @@ static HexApply<T> hex_args(fg_op *op, const T *qd, const T *x, T *y, int accumu
     A.skip = skip;
     A.err = op->d_err;
     A.wait_ns = op->wait_ns;
-    A.L.cu_off = op->u_cu_off;
-    A.L.cu_dof = op->u_cu_dof;
-    A.L.cu_pid = op->u_cu_pid;
-    A.L.cu_soff = op->u_cu_soff;
-    A.L.cu_slots = op->u_cu_slots;
-    A.L.part = op->u_part;
-    A.L.sh_dof = op->u_sh_dof;
-    A.L.sh_off = op->u_sh_off;
-    A.L.n_shared = op->u_nshared;
-    A.L.max_nu = op->u_max_nu;
+    A.L = op->u_lists.device(op->u_part);
     return A;
 }
 
@@ -65,7 +53,7 @@ static int hex_apply_t(fg_op *op, const HexApply<T> &A) {
     using SM = HexSmem<P, OPK, T, WARPS, S>;
     auto kern = hex_apply_kernel<P, OPK, T, WARPS, S, HexCfg<P>::MINB>;
     static std::atomic<int> lim[64];
-    const int bytes = SM::bytes(op->u_max_nu);
+    const int bytes = SM::bytes(op->u_lists.max_nu);
     int rc;
     if ((rc = hex_smem_limit(kern, op->device, bytes, lim))) return rc;
     kern<<<(unsigned)op->u_chunks, BS, bytes, op->stream>>>(A);
@@ -74,9 +62,9 @@ static int hex_apply_t(fg_op *op, const HexApply<T> &A) {
 }
 
 template <typename T> static int hex_shared(fg_op *op, const HexApply<T> &A, int diag) {
-    if (!op->u_nshared) return FG_OK;
-    const int db = (int)std::min<int64_t>((op->u_nshared + 255) / 256, 148 * 16);
-    chunk_shared_kernel<T><<<db, 256, 0, op->stream>>>(A.L, A.ess, A.x, A.y, A.accumulate, A.constrained, diag,
+    if (!op->u_lists.n_shared) return FG_OK;
+    const int db = (int)std::min<int64_t>((op->u_lists.n_shared + 255) / 256, 148 * 16);
+    chunk_shared_kernel<T><<<db, 256, 0, op->stream>>>(A.L, A.x, A.y, A.accumulate, A.constrained, diag,
                                                        A.skip);
     CK(cudaGetLastError());
     return FG_OK;
@@ -105,7 +93,7 @@ template <int P, int OPK> static int hex_diag_t(fg_op *op, const HexApply<double
     constexpr int BS = HexCfg<P>::WARPS * 32, NL = (P + 1) * (P + 1) * (P + 1);
     auto kern = hex_diag_kernel<P, OPK, BS>;
     static std::atomic<int> lim[64];
-    const int bytes = (int)(sizeof(double) * NL * BS + chunk_list_smem(NL, BS, op->u_max_nu));
+    const int bytes = (int)sizeof(double) * NL * BS + chunk_list_smem(NL, BS, op->u_lists.max_nu);
     int rc;
     if ((rc = hex_smem_limit(kern, op->device, bytes, lim))) return rc;
     kern<<<(unsigned)op->u_chunks, BS, bytes, op->stream>>>(A);
@@ -199,17 +187,11 @@ extern "C" FG_API int fg_op_create_hex(int order, int64_t n_nodes, const double 
         morton_order(cen, E, perm);
     }
     const int64_t Ep = (E + 31) / 32 * 32;
-    std::vector<int32_t> eid((size_t)Ep, -1), smap((size_t)Ep * nl, -1), sdofs((size_t)Ep * nl, -1);
+    std::vector<int32_t> eid((size_t)Ep, -1), smap((size_t)Ep * nl, -1);
     for (int64_t s = 0; s < E; ++s) {
         eid[(size_t)s] = perm[(size_t)s];
-        for (int k = 0; k < nl; ++k) {
-            const int32_t d = lexmap[(size_t)perm[(size_t)s] * nl + k];
-            smap[(size_t)s * nl + k] = d;
-            sdofs[(size_t)k * Ep + s] = d;
-        }
+        for (int k = 0; k < nl; ++k) smap[(size_t)s * nl + k] = lexmap[(size_t)perm[(size_t)s] * nl + k];
     }
-    ChunkPlan plan;
-    plan_chunk_lists(smap, Ep, N, nl, CE, plan);
     std::vector<uint8_t> mask((size_t)N, 0);
     if (n_ess > 0) {
         std::vector<uint32_t> h_ess((size_t)n_ess);
@@ -219,6 +201,8 @@ extern "C" FG_API int fg_op_create_hex(int order, int64_t n_nodes, const double 
             mask[d] = 1;
         }
     }
+    ChunkPlan plan;
+    plan_chunk_lists(smap, Ep, N, nl, CE, mask.data(), plan);
 
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -231,8 +215,6 @@ extern "C" FG_API int fg_op_create_hex(int order, int64_t n_nodes, const double 
     op->unstr = true;
     op->u_E = Ep;
     op->u_chunks = plan.n_chunks;
-    op->u_nshared = (int64_t)plan.sh_dof.size();
-    op->u_max_nu = plan.max_nu;
     op->N = N;
     // native vectors: one row of the N plain values padded with zeros to a
     // multiple of 4 (the solver's vector kernels work in 4-wide groups); no tiles
@@ -263,29 +245,9 @@ extern "C" FG_API int fg_op_create_hex(int order, int64_t n_nodes, const double 
         return bail(rc);
     cudaEventCreate(&op->ev0);
     cudaEventCreate(&op->ev1);
-    if (cudaMalloc(&op->u_dofs, sizeof(int32_t) * sdofs.size()) ||
-        cudaMemcpy(op->u_dofs, sdofs.data(), sizeof(int32_t) * sdofs.size(), cudaMemcpyHostToDevice) ||
-        cudaMalloc(&op->u_ess, (size_t)N) || cudaMemcpy(op->u_ess, mask.data(), (size_t)N, cudaMemcpyHostToDevice))
-        return bail(fail(FG_CUDA_ERROR, "upload of the element maps failed"));
-    {
-        auto up = [](auto **dst, const auto &v) {
-            using V = typename std::remove_reference<decltype(v)>::type::value_type;
-            const size_t n = std::max<size_t>(v.size(), 1);
-            if (cudaMalloc(dst, sizeof(V) * n) != cudaSuccess) return false;
-            return v.empty() || cudaMemcpy(*dst, v.data(), sizeof(V) * v.size(), cudaMemcpyHostToDevice) == cudaSuccess;
-        };
-        std::vector<uint64_t> em((size_t)Ep, 0ull);
-        for (int64_t s = 0; s < Ep; ++s)
-            for (int k = 0; k < nl; ++k) {
-                const int32_t d = smap[(size_t)s * nl + k];
-                if (d >= 0 && mask[(size_t)d]) em[(size_t)s] |= 1ull << k;
-            }
-        if (!up(&op->u_emsk, em) || !up(&op->u_cu_off, plan.cu_off) || !up(&op->u_cu_dof, plan.cu_dof) || !up(&op->u_cu_pid, plan.cu_pid) ||
-            !up(&op->u_cu_soff, plan.cu_soff) || !up(&op->u_cu_slots, plan.cu_slots) ||
-            !up(&op->u_sh_dof, plan.sh_dof) || !up(&op->u_sh_off, plan.sh_off) ||
-            cudaMalloc(&op->u_part, sizeof(double) * std::max<int64_t>(plan.n_part, 1)) != cudaSuccess)
-            return bail(fail(FG_CUDA_ERROR, "upload of the chunk lists failed"));
-    }
+    if (cudaMalloc(&op->u_part, sizeof(double) * std::max<int64_t>(plan.n_part, 1)) != cudaSuccess ||
+        (rc = op->u_lists.upload(plan)))
+        return bail(rc ? rc : fail(FG_CUDA_ERROR, "upload of the chunk lists failed"));
 
     // quadrature data
     const int NC = kind == FG_MASS ? 1 : (kind == FG_DIFF ? 6 : 7);

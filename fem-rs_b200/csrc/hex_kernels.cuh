@@ -8,9 +8,10 @@
 // into chunks of CE = WARPS * 32 elements, one CTA each (the last chunk padded
 // to whole 32-element warp groups: padding elements have map entries -1 and
 // zero quadrature data).
-//   dofs [nl][E]         int32 element-to-DOF map, local DOF (c,b,a) at
-//                        k = (c*D + b)*D + a (tensor order on the reference cube);
-//                        element-major, so a warp reads each entry in one load
+//   lmap [nl][E]         position of the element's local DOF in its chunk's DOF
+//                        list (16 bits), local DOF (c,b,a) at k = (c*D + b)*D + a
+//                        (tensor order on the reference cube); element-major, so a
+//                        warp reads each entry in one 64-byte load
 //   qd                   quadrature data in each warp's consumption order:
 //                        [group][col = qy*Q + qx][qz][comp][lane], comp the 6
 //                        symmetric w|detJ| kappa J^-1 J^-T and/or w|detJ| rho.
@@ -18,16 +19,18 @@
 //                        streamed into a per-warp ring of shared-memory stages by
 //                        1-D bulk copies on mbarriers (bounded waits, drained on
 //                        timeout)
-//   ess  [N]             essential-DOF mask (constrained applies)
-//   emsk [E]             per element, bit k set: local DOF k is essential (the
-//                        gather masks with it instead of reading ess per DOF)
 //
-// Scatter without float atomics and without an element-result array in HBM
-// (chunk_plan.h, chunk_scatter.cuh): a CTA puts its element results in shared
-// memory and sums each DOF of its chunk's list over the DOF's element slots in
-// a fixed order; a DOF owned by the chunk is stored, a DOF shared with other
-// chunks gets a partial that chunk_shared_kernel adds in chunk order.  The
-// sums are the same from run to run.
+// Gather and scatter (chunk_plan.h, chunk_scatter.cuh): a CTA reads the DOFs of
+// its chunk once into shared memory (while the first quadrature columns arrive),
+// its elements take their values from there; the element results go to shared
+// memory and each DOF of the list is summed over its element slots in a fixed
+// order, stored (owned by the chunk) or left as a partial that
+// chunk_shared_kernel adds in chunk order.  No float atomics, no element-result
+// array in HBM; the sums are the same from run to run.
+//
+// What bounds it: the latency of one chunk's phases (gather, columns, sums) with
+// three CTAs per SM.  64^3 Q2 FP64, apply and shared DOFs: 159 us with a
+// 32-bit map and per-element x loads, 143 us as above.
 //
 // Element math: slab sum factorisation (one qy slab of QH quadrature columns
 // at a time: y then x contraction of the element values, per column z, D, z^T,
@@ -42,10 +45,7 @@ namespace fg {
 
 template <typename T> struct HexApply {
     int64_t E, N;          // elements (padded to whole 32-element groups), DOFs
-    const int32_t *dofs;   // [nl][E]
     const T *qd;           // per-group streams (layout above)
-    const uint8_t *ess;    // [N] or null
-    const uint64_t *emsk;  // [E] essential local DOFs (bit k), or null
     const T *x;            // null: diagonal
     T *y;
     int accumulate, constrained;
@@ -61,19 +61,19 @@ template <int P, int OPK> __host__ __device__ inline int64_t hex_qd_index(int64_
     return (((e >> 5) * (Q * Q) + col) * Q + qz) * (NC * 32) + comp * 32 + (e & 31);
 }
 
-// Shared memory (bytes): a region holding first the per-warp quadrature-data
-// rings and, after the element phase, the chunk's lists; the element values
-// (then results), one column per thread; the ring barriers.
+// Shared memory (bytes): the per-warp quadrature-data rings; the element values
+// (then results), one column per thread; a region holding first the chunk's x
+// values and, once the elements have taken them, the chunk's slot lists; the
+// ring barriers.
 template <int P, int OPK, typename T, int WARPS, int S> struct HexSmem {
     static constexpr int Q = P + 1, NL = (P + 1) * (P + 1) * (P + 1), BS = WARPS * 32;
     static constexpr int STAGE = Q * NComp<OPK>::v * 32;  // elements of one column stage
-    static constexpr int RING = WARPS * S * STAGE * (int)sizeof(T);
-    static __host__ __device__ int region(int max_nu) {
-        const int l = (int)chunk_list_smem(NL, BS, max_nu);
-        return round_up(RING > l ? RING : l, 128);
+    static constexpr int off_x = WARPS * S * STAGE * (int)sizeof(T);
+    static constexpr int off_l = off_x + NL * BS * (int)sizeof(T);
+    static __host__ __device__ int off_b(int max_nu) {
+        const int l = chunk_list_smem(NL, BS, max_nu), u = max_nu * (int)sizeof(T);
+        return off_l + round_up(l > u ? l : u, 16);
     }
-    static __host__ __device__ int off_x(int max_nu) { return region(max_nu); }
-    static __host__ __device__ int off_b(int max_nu) { return round_up(off_x(max_nu) + NL * BS * (int)sizeof(T), 8); }
     static __host__ __device__ int bytes(int max_nu) { return off_b(max_nu) + WARPS * S * 8; }
 };
 
@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
     if (A.skip && *A.skip) return;
     const int MU = A.L.max_nu;
     T *ring = reinterpret_cast<T *>(hex_smem);
-    T *xs = reinterpret_cast<T *>(hex_smem + SM::off_x(MU));
+    T *xs = reinterpret_cast<T *>(hex_smem + SM::off_x);
+    T *xu = reinterpret_cast<T *>(hex_smem + SM::off_l);
     uint64_t *bars = reinterpret_cast<uint64_t *>(hex_smem + SM::off_b(MU));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
     const int64_t E = A.E;
@@ -109,26 +110,31 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
     const T *qdw = A.qd + group * COLS * STAGE;
     int q_issued = 0, q_waited = 0;
     bool ok = true;
+    if (wvalid && lane == 0) {
+        for (int j = 0; j < S && j < COLS; ++j) {
+            mbar_arrive_expect_tx(&qbw[j], QBYTES);
+            bulk_g2s(qsw + j * STAGE, qdw + (int64_t)j * STAGE, QBYTES, &qbw[j]);
+            q_issued = j + 1;
+        }
+    }
+    // gather (E): the chunk's DOFs once, zero on the essential ones; padding
+    // elements take position 0 (their quadrature data are zero and no slot names them)
+    uint32_t lm[(NL + 1) / 2];
     if (wvalid) {
-        if (lane == 0) {
-            for (int j = 0; j < S && j < COLS; ++j) {
-                mbar_arrive_expect_tx(&qbw[j], QBYTES);
-                bulk_g2s(qsw + j * STAGE, qdw + (int64_t)j * STAGE, QBYTES, &qbw[j]);
-                q_issued = j + 1;
-            }
-        }
-        // gather (E) with the essential columns masked; padding elements hold -1
-        const bool evalid = __ldg(A.dofs + e) >= 0;
-        const uint64_t m = (A.constrained && A.emsk) ? __ldg(A.emsk + e) : 0ull;
 #pragma unroll
-        for (int k = 0; k < NL; ++k) {
-            T v = T(0);
-            if (evalid) {
-                const T xv = __ldg(A.x + __ldg(A.dofs + (int64_t)k * E + e));
-                v = ((m >> k) & 1ull) ? T(0) : xv;
-            }
-            xs[k * BS + tid] = v;
-        }
+        for (int k = 0; k < NL; k += 2)
+            lm[k / 2] = (uint32_t)__ldg(A.L.lmap + (int64_t)k * E + e) |
+                        (k + 1 < NL ? (uint32_t)__ldg(A.L.lmap + (int64_t)(k + 1) * E + e) << 16 : 0u);
+    }
+    chunk_load_x<T, BS>(A.L, blockIdx.x, A.x, xu, A.constrained);
+    __syncthreads();
+    if (wvalid) {
+#pragma unroll
+        for (int k = 0; k < NL; ++k) xs[k * BS + tid] = xu[(lm[k / 2] >> (16 * (k & 1))) & 0xffffu];
+    }
+    __syncthreads();  // the chunk's x values are free: the slot lists take their place
+    const ChunkStage cst = chunk_stage_lists<BS>(A.L, blockIdx.x, hex_smem + SM::off_l);
+    if (wvalid) {
         auto uval = [&](int c, int b, int a) -> T { return xs[((c * D + b) * D + a) * BS + tid]; };
         T out[D][D][D];
 #pragma unroll
@@ -272,14 +278,11 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
         // after a timeout: wait out the copies still in flight
         if (!ok && lane == 0) drain_stages(qbw, S, q_waited, q_issued);
     }  // wvalid
-    // E^T: the chunk's DOF sums.  The lists are staged where the rings were; a
-    // CTA in which a wait timed out (error word set) stores nothing, so that no
-    // copy that is still late can land in the staged lists.
+    // E^T: the chunk's DOF sums.  A CTA in which a wait timed out (error word set)
+    // stores nothing.
+    chunk_wait();
     if (__syncthreads_or(!ok)) return;
-    ChunkStage st = chunk_stage_at(A.L, hex_smem);
-    chunk_stage_lists<BS>(A.L, blockIdx.x, st);
-    __syncthreads();
-    chunk_sums<T, BS>(A.L, st, xs, A.ess, A.x, A.y, A.accumulate, A.constrained, 0);
+    chunk_sums<T, BS>(A.L, cst, xs, A.x, A.y, A.accumulate, A.constrained, 0);
 }
 
 // Jacobi diagonal: element diagonal sum_q g_i^T D_q g_i (+ m_q phi_i^2), one
@@ -302,7 +305,7 @@ __global__ void __launch_bounds__(BS) hex_diag_kernel(const HexApply<double> A) 
         for (int b = 0; b < D; ++b)
 #pragma unroll
             for (int a = 0; a < D; ++a) out[c][b][a] = 0.0;
-    if (e < E && __ldg(A.dofs + e) >= 0) {
+    if (e < E) {  // padding elements have zero quadrature data and no slot
         for (int qy = 0; qy < Q; ++qy)
             for (int qx = 0; qx < Q; ++qx)
                 for (int qz = 0; qz < Q; ++qz) {
@@ -338,10 +341,10 @@ __global__ void __launch_bounds__(BS) hex_diag_kernel(const HexApply<double> A) 
         for (int b = 0; b < D; ++b)
 #pragma unroll
             for (int a = 0; a < D; ++a) ys[((c * D + b) * D + a) * BS + tid] = out[c][b][a];
-    ChunkStage st = chunk_stage_at(A.L, hex_smem + sizeof(double) * NL * BS);
-    chunk_stage_lists<BS>(A.L, blockIdx.x, st);
+    const ChunkStage st = chunk_stage_lists<BS>(A.L, blockIdx.x, hex_smem + sizeof(double) * NL * BS);
+    chunk_wait();
     __syncthreads();
-    chunk_sums<double, BS>(A.L, st, ys, A.ess, nullptr, A.y, 0, A.constrained, 1);
+    chunk_sums<double, BS>(A.L, st, ys, nullptr, A.y, 0, A.constrained, 1);
 }
 
 // Quadrature-data setup of the unstructured mesh: one thread per (element,

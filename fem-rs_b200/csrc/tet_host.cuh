@@ -7,7 +7,7 @@
 #include <mutex>
 #include <vector>
 
-#include "chunk_plan.h"
+#include "chunk_host.cuh"
 #include "tet_kernels.cuh"
 
 struct fg_tet {
@@ -19,16 +19,11 @@ struct fg_tet {
     double *qp = nullptr, *phi = nullptr, *grad = nullptr;  // rule tables (device)
     std::vector<double> h_phi, h_grad;                       // rule tables (host, kernel parameters)
     int nq = 0;
-    // chunked scatter
-    int CE = 0, max_nu = 0, n_chunks = 0, wide = 0;  // wide: 512-thread CTAs for the P2 moment form
-    int64_t n_shared = 0, n_part = 0;
-    int32_t *edof = nullptr;   // [nl][E] chunk order
-    uint32_t *emsk = nullptr;  // [E] chunk order
-    uint16_t *cu_slots = nullptr;
-    int32_t *cu_off = nullptr, *cu_dof = nullptr, *cu_pid = nullptr, *cu_soff = nullptr;
-    int32_t *sh_dof = nullptr, *sh_off = nullptr;
+    // chunked gather and scatter
+    int CE = 0, n_chunks = 0, wide = 0;  // wide: 512-thread CTAs for the P2 moment form
+    ChunkBufs lists;
     double *part = nullptr;
-    uint8_t *ess = nullptr;
+    bool has_ess = false;
     double *xh = nullptr, *yh = nullptr;  // device copies for host-memory calls
     int *d_err = nullptr;
     cudaStream_t stream = nullptr;
@@ -185,7 +180,6 @@ static TetArgs tet_args(const fg_tet *t) {
     A.G = t->G;
     A.sk = t->sk;
     A.sm = t->sm;
-    A.ess = t->ess;
     A.R = TetRule{t->nq, t->phi, t->grad};
     return A;
 }
@@ -199,19 +193,7 @@ static TetChunk tet_chunk_args(const fg_tet *t) {
     C.Sm = t->Sm;
     C.sk = t->sk;
     C.sm = t->sm;
-    C.edof = t->edof;
-    C.emsk = t->emsk;
-    C.ess = t->ess;
-    C.L.cu_off = t->cu_off;
-    C.L.cu_dof = t->cu_dof;
-    C.L.cu_pid = t->cu_pid;
-    C.L.cu_soff = t->cu_soff;
-    C.L.cu_slots = t->cu_slots;
-    C.L.part = t->part;
-    C.L.sh_dof = t->sh_dof;
-    C.L.sh_off = t->sh_off;
-    C.L.n_shared = t->n_shared;
-    C.L.max_nu = t->max_nu;
+    C.L = t->lists.device(t->part);
     return C;
 }
 
@@ -219,9 +201,8 @@ static void tet_free(fg_tet *t) {
     if (!t) return;
     cudaSetDevice(t->device);
     if (t->stream) cudaStreamSynchronize(t->stream);
-    void *ptrs[] = {t->dofs, t->G, t->sk, t->sm, t->Sm, t->coords, t->qp, t->phi, t->grad, t->edof, t->emsk, t->cu_slots,
-                    t->cu_off, t->cu_dof, t->cu_pid, t->cu_soff, t->sh_dof, t->sh_off, t->part, t->ess, t->xh,
-                    t->yh, t->d_err};
+    void *ptrs[] = {t->dofs, t->G, t->sk, t->sm, t->Sm, t->coords, t->qp, t->phi, t->grad, t->part, t->xh, t->yh, t->d_err};
+    t->lists.release();
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (t->stream && t->own_stream) cudaStreamDestroy(t->stream);
@@ -239,7 +220,7 @@ template <typename T> static int tet_upload(T **dst, const T *src, size_t n) {
 // first four local DOFs) and the chunk DOF lists.  h = element map [E][nl] in
 // the caller's order; perm[n] = the caller's element at position n.
 static void tet_plan_chunks(const std::vector<int32_t> &h, const std::vector<double> &coords, int64_t E,
-                            int64_t N, int nl, int CE, std::vector<int32_t> &perm, ChunkPlan &P) {
+                            int64_t N, int nl, int CE, const uint8_t *ess, std::vector<int32_t> &perm, ChunkPlan &P) {
     std::vector<double> cen((size_t)E * 3);
     for (int64_t e = 0; e < E; ++e)
         for (int a = 0; a < 3; ++a) {
@@ -251,7 +232,7 @@ static void tet_plan_chunks(const std::vector<int32_t> &h, const std::vector<dou
     std::vector<int32_t> smap((size_t)E * nl);
     for (int64_t n = 0; n < E; ++n)
         for (int i = 0; i < nl; ++i) smap[(size_t)n * nl + i] = h[(size_t)perm[n] * nl + i];
-    plan_chunk_lists(smap, E, N, nl, CE, P);
+    plan_chunk_lists(smap, E, N, nl, CE, ess, P);
 }
 
 template <int NL, int MQ, bool MOM, int BT>
@@ -264,7 +245,7 @@ static int tet_launch_t(fg_tet *t, const TetChunk &C, const double *x, double *y
                 R.phi[q][i] = t->h_phi[(size_t)q * NL + i];
                 for (int c = 0; c < 3; ++c) R.grad[q][i][c] = t->h_grad[((size_t)q * NL + i) * 3 + c];
             }
-    const size_t smem = tet_chunk_smem(NL, t->CE, t->max_nu);
+    const size_t smem = tet_chunk_smem(NL, t->CE, t->lists.max_nu);
     if (smem > 48 * 1024)
         CK(cudaFuncSetAttribute(tet_chunk_kernel<NL, MQ, MOM, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)smem));
@@ -292,9 +273,9 @@ static int tet_launch_apply(fg_tet *t, const double *x, double *y, int accumulat
         else rc = tet_launch_t<20, TET_MAXQ, false, 256>(t, C, x, y, accumulate, constrained, diag);
     }
     if (rc) return rc;
-    if (t->n_shared) {
-        const int db = (int)std::min<int64_t>((t->n_shared + 255) / 256, 148 * 16);
-        chunk_shared_kernel<double><<<db, 256, 0, t->stream>>>(C.L, t->ess, diag ? nullptr : x, y, accumulate,
+    if (t->lists.n_shared) {
+        const int db = (int)std::min<int64_t>((t->lists.n_shared + 255) / 256, 148 * 16);
+        chunk_shared_kernel<double><<<db, 256, 0, t->stream>>>(C.L, diag ? nullptr : x, y, accumulate,
                                                                constrained, diag, nullptr);
     }
     CK(cudaGetLastError());

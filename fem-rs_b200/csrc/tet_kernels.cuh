@@ -23,8 +23,7 @@
 //   Sm   [10][E]   diffusion moments (S00, s1, S2 as xx xy xz yy yz zz); P1: [6][E] S00 G
 //   sk   [nq][E]   w_q kappa_q c_k          (diffusion, point form)
 //   sm   [nq][E]   w_q |det J| rho_q c_m    (mass)
-//   edof [nl][E]   int32 element-to-DOF map
-//   emsk [E]       uint32 bit i set: local DOF i is essential
+//   lmap [nl][E]   16-bit position of the local DOF in its chunk's DOF list
 //
 // Scatter without float atomics and without an element-result array in HBM:
 // the elements, sorted along a Morton curve of their centroids, form chunks
@@ -55,7 +54,6 @@ struct TetArgs {
     const int32_t *dofs;       // [nl][E] caller's element order
     const double *G;           // [6][E]
     const double *sk, *sm;     // [nq][E]
-    const uint8_t *ess;        // [N] or null
     TetRule R;
 };
 
@@ -65,9 +63,6 @@ struct TetChunk {
     int CE;                      // elements per chunk
     const double *G, *Sm;        // [6][E], [10][E] (P1: [6][E] S00 G)
     const double *sk, *sm;       // [nq][E]
-    const int32_t *edof;         // [nl][E]
-    const uint32_t *emsk;        // [E] essential local DOFs (bit i), null if no essential list
-    const uint8_t *ess;          // [N] or null
     ChunkLists L;
 };
 
@@ -259,20 +254,19 @@ __device__ __forceinline__ void tet_elem_moments(const double (&md)[TetMom<NL>::
     }
 }
 
-// Shared-memory plan of a chunk (bytes): element results, then the chunk's
-// lists.
+// Shared-memory plan of a chunk (bytes): element results, the chunk's slot
+// lists, its values of x.
 __host__ __device__ inline size_t tet_chunk_smem(int NL, int CE, int max_nu) {
-    return sizeof(double) * (size_t)NL * CE + chunk_list_smem(NL, CE, max_nu);
+    return sizeof(double) * ((size_t)NL * CE + max_nu) + chunk_list_smem(NL, CE, max_nu);
 }
 
-// One CTA (BT threads) per chunk.  First the chunk's DOF list (ids, partial
-// ids, slot offsets relative to the chunk) and local slots are staged in
-// shared memory and the element results are computed into shared memory, the
-// element gathering its x values through the element map: no wait separates
-// the two, so all their loads are in flight together.  After the barrier each
-// DOF's slots are summed from shared memory.  MOM: diffusion-only apply by the
-// moment form.  On essential DOFs of a constrained call the identity row:
-// y_d (+)= x_d (apply) or 1 (diagonal).
+// One CTA (BT threads) per chunk.  The copies of the chunk's slot lists are
+// started and its values of x read once into shared memory; then the element
+// results are computed into shared memory, each element taking its values by
+// its 16-bit positions.  After a barrier each DOF's slots are summed.  MOM:
+// diffusion-only apply by the moment form.  On essential DOFs of a constrained call
+// the identity row: y_d (+)= x_d (apply) or 1 (diagonal).  40^3 x 6 P2 tetrahedra:
+// 41.0 us with x gathered per element through a 32-bit map, 37.0 us this way.
 template <int NL, int MQ, bool MOM, int BT>
 __global__ void __launch_bounds__(BT, MOM ? (BT == 512 ? 2 : 3) : 1) tet_chunk_kernel(const TetChunk C, int kind, int nq,
                                                                   const __grid_constant__ TetTab<NL, MQ> R,
@@ -282,33 +276,29 @@ __global__ void __launch_bounds__(BT, MOM ? (BT == 512 ? 2 : 3) : 1) tet_chunk_k
     extern __shared__ __align__(16) unsigned char tsm_raw[];
     const int CE = C.CE;
     double *ys = reinterpret_cast<double *>(tsm_raw);  // [NL][CE] element results
-    ChunkStage S = chunk_stage_at(C.L, tsm_raw + sizeof(double) * NL * CE);
-    const int c = blockIdx.x;
-    const int64_t e0 = (int64_t)c * CE;
+    const ChunkStage S = chunk_stage_lists<BT>(C.L, blockIdx.x, tsm_raw + sizeof(double) * NL * CE);
+    double *xu = reinterpret_cast<double *>(tsm_raw + sizeof(double) * NL * CE + chunk_list_smem(NL, CE, C.L.max_nu));
+    const int64_t e0 = (int64_t)blockIdx.x * CE;
     const int ne = (int)(C.E - e0 < CE ? C.E - e0 : CE);
-    chunk_stage_lists<BT>(C.L, c, S);
-    const bool mask = constrained && C.emsk;
+    if (!diag) {
+        chunk_load_x<double, BT>(C.L, blockIdx.x, x, xu, constrained);
+        __syncthreads();
+    }
     for (int el = threadIdx.x; el < ne; el += BT) {
         const int64_t e = e0 + el;
         double xe[NL], ye[NL];
         double md[MOM ? TetMom<NL>::n : 1];
-        if constexpr (MOM) tet_load_moments<NL>(C, e, md);  // issued before the dependent x gathers
-        const uint32_t m = mask ? __ldg(C.emsk + e) : 0u;
+        if constexpr (MOM) tet_load_moments<NL>(C, e, md);
 #pragma unroll
-        for (int i = 0; i < NL; ++i) {
-            xe[i] = 0.0;
-            if (!diag) {
-                const double v = __ldg(x + __ldg(C.edof + (int64_t)i * C.E + e));
-                xe[i] = ((m >> i) & 1u) ? 0.0 : v;
-            }
-        }
+        for (int i = 0; i < NL; ++i) xe[i] = diag ? 0.0 : xu[__ldg(C.L.lmap + (int64_t)i * C.E + e)];
         if constexpr (MOM) tet_elem_moments<NL>(md, xe, ye);
         else tet_elem_points<NL, MQ>(C, kind, nq, R, e, xe, ye, diag);
 #pragma unroll
         for (int i = 0; i < NL; ++i) ys[i * CE + el] = ye[i];
     }
+    chunk_wait();
     __syncthreads();
-    chunk_sums<double, BT>(C.L, S, ys, C.ess, x, y, accumulate, constrained, diag);
+    chunk_sums<double, BT>(C.L, S, ys, x, y, accumulate, constrained, diag);
 }
 
 // Reorder the per-element data into the chunk order and form the diffusion
