@@ -620,14 +620,18 @@ static void set_scratch_tiling(Grid &g) {
 // (about 0.8 layer).  Rounds count whole up to four (the last one leaves SMs
 // idle), above that half a round is lost on average; a small term counts the
 // warps that work at all, which separates the lane shapes when the rounds do
-// not.  The 8 x 4 shape pays for its shuffles and shorter rows of stores (2 %;
-// 128^3 Q2 FP64 517 against 552 us), except in the Q3 FP64 full format, where it has
+// not.  32 lanes in x come first and a later candidate must win by a tenth of a
+// layer: the 8 x 4 shape pays for its shuffles and shorter rows of stores (128^3 Q2
+// FP64 517 against 552 us; a few microseconds where one round holds everything),
+// except in the Q3 FP64 full format (0.9 of the cost), where it has
 // the deeper ring (64^3: 245 against 275 us).  The rule before this one took 32 lanes
 // in x and halved the depth until there were 592 items, which left a nearly empty
 // last round or lane padding: apply and fix-up on a B200, then -> now: 48^3 Q3 FP32
 // affine 45.6 -> 34.8 us, 33x40x37 38.0 -> 24.8, 48x40x44 Q2 FP64 42.9 -> 34.1,
 // 45x41x38 Q3 FP64 121 -> 97, 100x90x80 Q1 FP64 76.9 -> 57.6, 64^3 Q2 FP32 affine
-// mass + diffusion 32.6 -> 30.6.
+// mass + diffusion 32.6 -> 30.6.  Over 767 random meshes of 6 to 192 elements a
+// side, all orders, kinds and forms: 2.4 % above the best of 18 shapes on average
+// (the old rule 13 %), 9 % below the old rule's time, at worst 20 % above it.
 static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size_t face_limit) {
     // CTAs per SM by registers and shared memory, [fp32][affine][order]
     static const int resident[2][2][3] = {{{3, 2, 4}, {3, 2, 2}}, {{5, 3, 4}, {5, 5, 4}}};
@@ -645,14 +649,14 @@ static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size
         // 8-wide items may not outnumber the 32-wide ones by more than a tenth: a warp
         // without elements still holds its registers, and the face slots grow
         else if (!lanes && 10 * warps > 11 * warps32) continue;
-        const double shape = LX == 32 ? 1.0 : (g.p == 3 && !fp32 && !affine) ? 0.92 : 1.02;
+        const double shape = LX == 8 && g.p == 3 && !fp32 && !affine ? 0.9 : 1.0;
         const double work = (double)(LX == 32 ? warps : live) * c.nz / (c.NW * slots);
         for (int tz = 1; tz <= std::min(g.nz, 16); ++tz) {
             set_depth(c, tz);
             if (face_limit && (size_t)c.n_items() * (size_t)c.face_stride() > face_limit) continue;
             const double w = c.n_items() / slots;
             const double cost = shape * ((w >= 4.0 ? w + 0.5 : std::ceil(w)) * (tz + 0.8) + 0.25 * work);
-            if (cost < best_cost * (1.0 - 1e-9)) {
+            if (cost < best_cost - 0.1) {
                 best_cost = cost;
                 best = c;
             }
