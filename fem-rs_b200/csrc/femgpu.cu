@@ -1239,12 +1239,12 @@ static int estimate_lmax(fg_op *op, int iters, double *out) {
     int rc;
     const int64_t n = op->Nn;
     k_hash_vector<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(op->g, op->cd, op->partials, op->st);
-    k_scale_by_rho<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->cd, op->cd, op->st);
+    k_scale_by_rho<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->cd, op->cd, op->st);
     CK(cudaGetLastError());
     for (int it = 0; it < iters; ++it) {
         if ((rc = apply_native(op, op->cd, op->ct, 0, 1, nullptr))) return rc;
-        k_dinv_norm<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->ct, op->dinv, op->partials, op->st);
-        k_scale_by_rho<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->ct, op->cd, op->st);
+        k_dinv_norm<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->ct, op->dinv, op->partials, op->st);
+        k_scale_by_rho<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->ct, op->cd, op->st);
         CK(cudaGetLastError());
     }
     SolverState h;
@@ -1302,7 +1302,7 @@ static int cheb_apply(fg_op *op, const PcgBufs<T> &B, const ChebCoef &cc, const 
                 int rc = alloc_vec(&dk[k - 1], n);
                 if (rc) return rc;
             }
-        k_cheb_first_d<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, r, B.dinv, B.cres, B.cd,
+        k_cheb_first_d<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, r, B.dinv, B.cres, B.cd,
                                                                     cc.inv_theta, sst);
         CK(cudaGetLastError());
         const T *dprev = B.cd;
@@ -1310,7 +1310,7 @@ static int cheb_apply(fg_op *op, const PcgBufs<T> &B, const ChebCoef &cc, const 
             int rc = apply_native_t<T>(op, B.qd, B.face, dprev, B.ct, 0, 1, skip);
             if (rc) return rc;
             if (k < s) {
-                k_cheb_mid<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.ct, B.dinv, B.cres, dprev,
+                k_cheb_mid<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.ct, B.dinv, B.cres, dprev,
                                                                         dk[k - 1], cc.c1[k - 1],
                                                                         cc.c2[k - 1], sst);
                 dprev = dk[k - 1];
@@ -1318,7 +1318,7 @@ static int cheb_apply(fg_op *op, const PcgBufs<T> &B, const ChebCoef &cc, const 
                 ChebSum<T> earlier{};
                 earlier.n = s - 1;  // d_0 .. d_{s-2}
                 for (int j = 0; j < s - 1; ++j) earlier.d[j] = j == 0 ? B.cd : dk[j - 1];
-                k_cheb_last<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.ct, B.dinv, B.cres, dprev,
+                k_cheb_last<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.ct, B.dinv, B.cres, dprev,
                                                                          earlier, z, cc.c1[k - 1],
                                                                          cc.c2[k - 1], sst);
             }
@@ -1326,13 +1326,13 @@ static int cheb_apply(fg_op *op, const PcgBufs<T> &B, const ChebCoef &cc, const 
         }
         return FG_OK;
     }
-    k_cheb_first<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, r, B.dinv, B.cres, B.cd, z,
+    k_cheb_first<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, r, B.dinv, B.cres, B.cd, z,
                                                               cc.inv_theta, sst);
     CK(cudaGetLastError());
     for (size_t s = 0; s < cc.c1.size(); ++s) {
         int rc = apply_native_t<T>(op, B.qd, B.face, B.cd, B.ct, 0, 1, skip);
         if (rc) return rc;
-        k_cheb_step<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.ct, B.dinv, B.cres, B.cd, z,
+        k_cheb_step<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.ct, B.dinv, B.cres, B.cd, z,
                                                                  cc.c1[s], cc.c2[s], sst);
         CK(cudaGetLastError());
     }
@@ -1428,7 +1428,7 @@ template <typename T> static int launch_pcg_fused(fg_op *op, const PcgBufs<T> &B
         FG_LEGACY_FENCE();
     }
     cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(VEC_GRID);
+    lc.gridDim = dim3(vec_grid(op->Nn));
     lc.blockDim = dim3(VEC_THREADS);
     lc.stream = op->stream;
     cudaLaunchAttribute at[1];
@@ -1457,13 +1457,13 @@ static int pcg_run(fg_op *op, const PcgBufs<T> &B, bool jacobi_like, const ChebC
         if ((rc = apply_native_t<T>(op, B.qd, B.face, B.x, B.ap, 0, 1, nullptr))) return rc;
         ++*applies;
     }
-    k_pcg_init<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.b, B.ap, B.dinv, B.r, B.z, B.p,
+    k_pcg_init<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.b, B.ap, B.dinv, B.r, B.z, B.p,
                                                             jacobi_like ? 1 : 0, op->partials, B.st);
     CK(cudaGetLastError());
     if (cheb) {
         if ((rc = cheb_apply<T>(op, B, *cc, B.r, B.z, skip))) return rc;
-        k_pcg_rz<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.r, B.z, op->partials, B.st, 1);
-        k_pcg_pupdate<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.z, B.p, B.st, 1);
+        k_pcg_rz<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.r, B.z, op->partials, B.st, 1);
+        k_pcg_pupdate<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.z, B.p, B.st, 1);
         CK(cudaGetLastError());
     }
     int launched = 0;
@@ -1476,14 +1476,14 @@ static int pcg_run(fg_op *op, const PcgBufs<T> &B, bool jacobi_like, const ChebC
             if ((r2 = launch_pcg_fused<T>(op, B, &used))) return r2;
             if (used) return FG_OK;
         }
-        k_pcg_pap<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.p, B.ap, op->partials, B.st);
-        k_pcg_update<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(
+        k_pcg_pap<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.p, B.ap, op->partials, B.st);
+        k_pcg_update<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(
             n, B.x, B.r, B.p, B.ap, B.dinv, B.z, cheb ? 0 : 1, op->partials, B.st);
         if (cheb) {
             if ((r2 = cheb_apply<T>(op, B, *cc, B.r, B.z, skip))) return r2;
-            k_pcg_rz<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.r, B.z, op->partials, B.st, 0);
+            k_pcg_rz<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.r, B.z, op->partials, B.st, 0);
         }
-        k_pcg_pupdate<T><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.z, B.p, B.st, 0);
+        k_pcg_pupdate<T><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.z, B.p, B.st, 0);
         CK(cudaGetLastError());
         return FG_OK;
     };
@@ -1678,7 +1678,7 @@ static int fcg_nn_run(fg_op *op, const PcgBufs<double> &B, const ChebCoef &cc, i
     *fell_back = 0;
     if ((rc = apply_native_t<double>(op, B.qd, B.face, B.x, B.ap, 0, 1, nullptr))) return rc;
     ++*applies;
-    k_pcg_init<double><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.b, B.ap, B.dinv, B.r, B.z, B.p,
+    k_pcg_init<double><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.b, B.ap, B.dinv, B.r, B.z, B.p,
                                                                  0, op->partials, B.st);
     auto direction = [&](int init) -> int {
         const float *f1 = nullptr;
@@ -1686,8 +1686,8 @@ static int fcg_nn_run(fg_op *op, const PcgBufs<double> &B, const ChebCoef &cc, i
         if (nn_on && (r2 = nn_begin<double>(op, B.r, &f1))) return r2;
         if ((r2 = cheb_apply<double>(op, B, cc, B.r, B.z, skip))) return r2;
         if (nn_on && (r2 = nn_end<double>(op, f1, B.z))) return r2;
-        k_fcg_zap<double><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.z, B.ap, op->partials, B.st, init);
-        k_fcg_pupdate_pr<double><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.z, B.p, B.r, op->partials,
+        k_fcg_zap<double><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.z, B.ap, op->partials, B.st, init);
+        k_fcg_pupdate_pr<double><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.z, B.p, B.r, op->partials,
                                                                             B.st, init);
         CK(cudaGetLastError());
         return FG_OK;
@@ -1698,8 +1698,8 @@ static int fcg_nn_run(fg_op *op, const PcgBufs<double> &B, const ChebCoef &cc, i
     auto iteration = [&]() -> int {
         int r2;
         if ((r2 = apply_native_t<double>(op, B.qd, B.face, B.p, B.ap, 0, 1, skip))) return r2;
-        k_pcg_pap<double><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.p, B.ap, op->partials, B.st);
-        k_pcg_update<double><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, B.x, B.r, B.p, B.ap, B.dinv,
+        k_pcg_pap<double><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.p, B.ap, op->partials, B.st);
+        k_pcg_update<double><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, B.x, B.r, B.p, B.ap, B.dinv,
                                                                        B.z, 0, op->partials, B.st);
         return direction(0);
     };
@@ -1930,7 +1930,7 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
         // r = b - A x (FP64), r_lo = r
         if ((rc = apply_native(op, op->xw, op->ap, 0, 1, nullptr))) return rc;
         ++applies;
-        k_rel_residual<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->bw, op->ap, op->r32,
+        k_rel_residual<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->bw, op->ap, op->r32,
                                                                  op->partials, op->st, 1);
         // z = M r_lo ; p = z ; rz
         bool nn_on = learned && use_nn;
@@ -1941,9 +1941,9 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
                 if (nn_on && (rc2 = nn_begin<float>(op, op->r32, &f1))) return rc2;
                 if ((rc2 = cheb_apply<float>(op, B, cc, op->r32, op->z32, done))) return rc2;
                 if (nn_on && (rc2 = nn_end<float>(op, f1, op->z32))) return rc2;
-                k_fcg_zap<float><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->z32, op->ap32, op->partials,
+                k_fcg_zap<float><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->z32, op->ap32, op->partials,
                                                                            op->st, init);
-                k_fcg_pupdate_pr<float><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->z32, op->p32, op->r32,
+                k_fcg_pupdate_pr<float><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->z32, op->p32, op->r32,
                                                                                    op->partials, op->st, init);
                 CK(cudaGetLastError());
                 return FG_OK;
@@ -1951,13 +1951,13 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
             if (cheb) {
                 int rc2 = cheb_apply<float>(op, B, cc, op->r32, op->z32, done);
                 if (rc2) return rc2;
-                k_pcg_rz<float><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->r32, op->z32,
+                k_pcg_rz<float><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->r32, op->z32,
                                                                           op->partials, op->st, init);
             } else {
-                k_jacobi_rz<float><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->r32, dinv32, op->z32,
+                k_jacobi_rz<float><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->r32, dinv32, op->z32,
                                                                              op->partials, op->st, init);
             }
-            k_pcg_pupdate<float><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->z32, op->p32, op->st, init);
+            k_pcg_pupdate<float><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->z32, op->p32, op->st, init);
             CK(cudaGetLastError());
             return FG_OK;
         };
@@ -1967,13 +1967,13 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
         auto iteration = [&]() -> int {
             int r2;
             if ((r2 = apply_native_t<float>(op, op->qd32, op->face32, op->p32, op->ap32, 0, 1, done))) return r2;
-            k_pcg_pap<float><<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->p32, op->ap32, op->partials, op->st);
-            k_rel_step<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->e32, op->r32, op->p32, op->ap32,
+            k_pcg_pap<float><<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->p32, op->ap32, op->partials, op->st);
+            k_rel_step<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->e32, op->r32, op->p32, op->ap32,
                                                                  op->partials, op->st);
             // reliable update (kernels return at once unless triggered)
-            k_rel_xupdate<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->xw, op->e32, op->st);
+            k_rel_xupdate<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->xw, op->e32, op->st);
             if ((r2 = apply_native(op, op->xw, op->ap, 0, 1, skip_rel))) return r2;
-            k_rel_residual<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->bw, op->ap, op->r32, op->partials,
+            k_rel_residual<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->bw, op->ap, op->r32, op->partials,
                                                                      op->st, 0);
             return precond(0);
         };
@@ -1998,7 +1998,7 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
     CK(cudaEventRecord(op->ev1, op->stream));
     // true residual in FP64
     if ((rc = apply_native(op, op->xw, op->ap, 0, 1, nullptr))) return rc;
-    k_true_residual<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->bw, op->ap, op->partials, op->st);
+    k_true_residual<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->bw, op->ap, op->partials, op->st);
     CK(cudaGetLastError());
     SolverState h2;
     if ((rc = read_state(op, &h2))) return rc;
@@ -2766,15 +2766,15 @@ FG_API int fg_sdirk2(fg_op *stiff, fg_op *stage, double *u, double dt, int n_ste
     double *scal = nullptr;  // ||b|| kept in a device scalar between the two calls
     auto normalise = [&](bool before) -> int {
         if (before) {
-            k_norm_tmp<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->bw, stage->partials, stage->st);
-            k_scale_tmp<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->bw, stage->st, 1);
-            k_scale_tmp<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->xw, stage->st, 1);
+            k_norm_tmp<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->bw, stage->partials, stage->st);
+            k_scale_tmp<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->bw, stage->st, 1);
+            k_scale_tmp<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->xw, stage->st, 1);
             CK(cudaMemcpyAsync(scal, &stage->st->tmp[2], sizeof(double), cudaMemcpyDeviceToDevice,
                                stage->stream));
         } else {
             CK(cudaMemcpyAsync(&stage->st->tmp[2], scal, sizeof(double), cudaMemcpyDeviceToDevice,
                                stage->stream));
-            k_scale_tmp<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->xw, stage->st, 0);
+            k_scale_tmp<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->xw, stage->st, 0);
         }
         CK(cudaGetLastError());
         return FG_OK;
@@ -2785,7 +2785,7 @@ FG_API int fg_sdirk2(fg_op *stiff, fg_op *stage, double *u, double dt, int n_ste
         int r2 = apply_native(stiff, ucur, stage->sd_w, 0, 1, nullptr);
         if (r2) return r2;
         ++applies;
-        k_lincomb2<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->bw, -1.0, stage->sd_w, 0.0,
+        k_lincomb2<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->bw, -1.0, stage->sd_w, 0.0,
                                                                  stage->sd_w);
         CK(cudaGetLastError());
         fg_result r{};
@@ -2805,11 +2805,11 @@ FG_API int fg_sdirk2(fg_op *stiff, fg_op *stage, double *u, double dt, int n_ste
         CK(cudaMemcpyAsync(stage->sd_k1, stage->xw, sizeof(double) * n, cudaMemcpyDeviceToDevice,
                            stage->stream));
         // u2 = u + dt (1-g) k1 (held in the solver's r buffer until the stiff apply reads it)
-        k_lincomb2<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->r, 1.0, stage->sd_u,
+        k_lincomb2<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->r, 1.0, stage->sd_u,
                                                                  dt * (1.0 - g), stage->sd_k1);
         if ((rc = apply_native(stiff, stage->r, stage->sd_w, 0, 1, nullptr))) return rc;
         ++applies;
-        k_lincomb2<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->bw, -1.0, stage->sd_w, 0.0,
+        k_lincomb2<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->bw, -1.0, stage->sd_w, 0.0,
                                                                  stage->sd_w);
         {
             fg_result r{};
@@ -2824,9 +2824,9 @@ FG_API int fg_sdirk2(fg_op *stiff, fg_op *stage, double *u, double dt, int n_ste
             max_it = std::max(max_it, (int)r.iterations);
         }
         // u += dt (1-g) k1 + dt g k2
-        k_lincomb2<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->sd_w, dt * (1.0 - g),
+        k_lincomb2<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->sd_w, dt * (1.0 - g),
                                                                  stage->sd_k1, dt * g, stage->xw);
-        k_lincomb2<<<VEC_GRID, VEC_THREADS, 0, stage->stream>>>(n, stage->sd_u, 1.0, stage->sd_u, 1.0,
+        k_lincomb2<<<vec_grid(n), VEC_THREADS, 0, stage->stream>>>(n, stage->sd_u, 1.0, stage->sd_u, 1.0,
                                                                  stage->sd_w);
         CK(cudaGetLastError());
     }
@@ -3395,7 +3395,7 @@ FG_API int fg_op_collect_pairs(fg_op *op, const double *b, const fg_cfg *cfg_in,
     grid_launch(nv, blocks);
     for (size_t j = 0; j < stash.size(); ++j) {
         if ((rc = apply_native(op, stash[j], op->ap, 0, 1, nullptr))) return rc;
-        k_lincomb2<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->r, 1.0, op->bw, -1.0, op->ap);
+        k_lincomb2<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->r, 1.0, op->bw, -1.0, op->ap);
         if ((rc = nn_restrict<double>(op, op->r, op->nn_rc))) return rc;
         rms_kernel<<<1, 1024, 0, op->stream>>>(op->nn_rc, nv, op->nn_scale);
         pack_input_f32_kernel<<<blocks, 256, 0, op->stream>>>(op->nn_rc, op->nn_lk, nv, op->nn_scale,
@@ -3503,7 +3503,7 @@ FG_API int fg_unet_train_energy(fg_unet *u, fg_op *op, const double *d_res, int 
                                                            op->nn_oc);
         if ((rc = nn_prolong<double>(op, op->nn_oc, op->pv, tb + 4 * b, mult, 0))) return rc;
         if ((rc = apply_native(op, op->pv, op->ap, 0, 1, nullptr))) return rc;
-        k_energy_terms<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(n, op->pv, op->ap, r, op->partials, op->st);
+        k_energy_terms<<<vec_grid(n), VEC_THREADS, 0, op->stream>>>(n, op->pv, op->ap, r, op->partials, op->st);
         CK(cudaMemcpyAsync(tb + 4 * b + 1, &op->st->tmp[0], 2 * sizeof(double), cudaMemcpyDeviceToDevice,
                            op->stream));
         if ((rc = nn_restrict<double>(op, op->ap, op->nn_rc))) return rc;

@@ -14,7 +14,16 @@
 namespace fg {
 
 constexpr int VEC_THREADS = 256;
-constexpr int VEC_GRID = 592;  // fixed: the reduction order must not depend on the device
+constexpr int VEC_GRID = 592;  // at most; fixed: the reduction order must not depend on the device
+
+// Blocks of a 4-wide vector kernel over n values: one group of four per thread
+// up to VEC_GRID blocks.  The blocks left out would only add zeros to a sum (the
+// same bits); on a 24^3 Q1 vector (18 blocks instead of 592) they cost more than
+// the work: their launch, their tickets and their arrivals at the grid barriers.
+inline unsigned vec_grid(int64_t n) {
+    const int64_t b = (n / 4 + VEC_THREADS - 1) / VEC_THREADS;
+    return (unsigned)(b < 1 ? 1 : b < VEC_GRID ? b : VEC_GRID);
+}
 
 struct SolverState {
     double rz, pap, alpha, beta, rr, bb, bnorm, res;
