@@ -109,6 +109,8 @@ __device__ __forceinline__ void chunk_sums(const ChunkLists &L, const ChunkStage
 template <typename T>
 __global__ void chunk_shared_kernel(const ChunkLists L, const T *__restrict__ x, T *__restrict__ y, int accumulate,
                                     int constrained, int diag, const int *skip) {
+    pdl_trigger();
+    pdl_wait();
     if (skip && *skip) return;
     const T *part = reinterpret_cast<const T *>(L.part);
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < L.n_shared;

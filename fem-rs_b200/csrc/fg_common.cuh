@@ -89,8 +89,16 @@ struct Grid {
 };
 
 // ---------------------------------------------------------------------------
-// PTX helpers: mbarrier, bulk async copies (TMA), timers.
+// PTX helpers: dependent launches, mbarrier, bulk async copies (TMA), timers.
 // ---------------------------------------------------------------------------
+// Dependent launches: a kernel launched with launch_dep may start while its
+// predecessor in the stream is still running, once every CTA of the predecessor
+// has passed pdl_trigger (or exited).  It may touch nothing that an earlier
+// kernel writes or reads before pdl_wait, which returns when the predecessor has
+// completed -- and, as every kernel so launched waits, all before it.  Both are
+// no-ops in a kernel launched the ordinary way.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }

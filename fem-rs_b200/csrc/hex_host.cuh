@@ -56,17 +56,15 @@ static int hex_apply_t(fg_op *op, const HexApply<T> &A) {
     const int bytes = SM::bytes(op->u_lists.max_nu);
     int rc;
     if ((rc = hex_smem_limit(kern, op->device, bytes, lim))) return rc;
-    kern<<<(unsigned)op->u_chunks, BS, bytes, op->stream>>>(A);
-    CK(cudaGetLastError());
+    CK(launch_dep(kern, dim3((unsigned)op->u_chunks), BS, bytes, op->stream, A));
     return FG_OK;
 }
 
 template <typename T> static int hex_shared(fg_op *op, const HexApply<T> &A, int diag) {
     if (!op->u_lists.n_shared) return FG_OK;
     const int db = (int)std::min<int64_t>((op->u_lists.n_shared + 255) / 256, 148 * 16);
-    chunk_shared_kernel<T><<<db, 256, 0, op->stream>>>(A.L, A.x, A.y, A.accumulate, A.constrained, diag,
-                                                       A.skip);
-    CK(cudaGetLastError());
+    CK(launch_dep(chunk_shared_kernel<T>, dim3(db), 256, 0, op->stream, A.L, A.x, A.y, A.accumulate, A.constrained, diag,
+                  A.skip));
     return FG_OK;
 }
 

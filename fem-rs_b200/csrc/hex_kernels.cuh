@@ -88,7 +88,6 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
     constexpr uint32_t QBYTES = (uint32_t)(STAGE * sizeof(T));
     using TB = Tab<T>;
     extern __shared__ __align__(128) unsigned char hex_smem[];
-    if (A.skip && *A.skip) return;
     const int MU = A.L.max_nu;
     T *ring = reinterpret_cast<T *>(hex_smem);
     T *xs = reinterpret_cast<T *>(hex_smem + SM::off_x);
@@ -110,13 +109,16 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
     const T *qdw = A.qd + group * COLS * STAGE;
     int q_issued = 0, q_waited = 0;
     bool ok = true;
-    if (wvalid && lane == 0) {
-        for (int j = 0; j < S && j < COLS; ++j) {
-            mbar_arrive_expect_tx(&qbw[j], QBYTES);
-            bulk_g2s(qsw + j * STAGE, qdw + (int64_t)j * STAGE, QBYTES, &qbw[j]);
-            q_issued = j + 1;
-        }
-    }
+    auto issue_first = [&]() {
+        if (wvalid && lane == 0)
+            for (int j = 0; j < S && j < COLS; ++j) {
+                mbar_arrive_expect_tx(&qbw[j], QBYTES);
+                bulk_g2s(qsw + j * STAGE, qdw + (int64_t)j * STAGE, QBYTES, &qbw[j]);
+                q_issued = j + 1;
+            }
+    };
+    pdl_trigger();
+    if (!A.skip) issue_first();  // quadrature data and maps do not depend on earlier kernels
     // gather (E): the chunk's DOFs once, zero on the essential ones; padding
     // elements take position 0 (their quadrature data are zero and no slot names them)
     uint32_t lm[(NL + 1) / 2];
@@ -125,6 +127,11 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
         for (int k = 0; k < NL; k += 2)
             lm[k / 2] = (uint32_t)__ldg(A.L.lmap + (int64_t)k * E + e) |
                         (k + 1 < NL ? (uint32_t)__ldg(A.L.lmap + (int64_t)(k + 1) * E + e) << 16 : 0u);
+    }
+    pdl_wait();
+    if (A.skip) {
+        if (*A.skip) return;
+        issue_first();
     }
     chunk_load_x<T, BS>(A.L, blockIdx.x, A.x, xu, A.constrained);
     __syncthreads();

@@ -249,8 +249,8 @@ static int tet_launch_t(fg_tet *t, const TetChunk &C, const double *x, double *y
     if (smem > 48 * 1024)
         CK(cudaFuncSetAttribute(tet_chunk_kernel<NL, MQ, MOM, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)smem));
-    tet_chunk_kernel<NL, MQ, MOM, BT><<<t->n_chunks, BT, smem, t->stream>>>(C, t->kind, t->nq, R, x, y, accumulate,
-                                                                            constrained, diag);
+    CK(launch_dep(tet_chunk_kernel<NL, MQ, MOM, BT>, dim3(t->n_chunks), BT, smem, t->stream, C, t->kind, t->nq, R, x, y,
+                  accumulate, constrained, diag));
     return FG_OK;
 }
 
@@ -275,8 +275,8 @@ static int tet_launch_apply(fg_tet *t, const double *x, double *y, int accumulat
     if (rc) return rc;
     if (t->lists.n_shared) {
         const int db = (int)std::min<int64_t>((t->lists.n_shared + 255) / 256, 148 * 16);
-        chunk_shared_kernel<double><<<db, 256, 0, t->stream>>>(C.L, diag ? nullptr : x, y, accumulate,
-                                                               constrained, diag, nullptr);
+        CK(launch_dep(chunk_shared_kernel<double>, dim3(db), 256, 0, t->stream, C.L, diag ? nullptr : x, y, accumulate,
+                      constrained, diag, (const int *)nullptr));
     }
     CK(cudaGetLastError());
     return FG_OK;

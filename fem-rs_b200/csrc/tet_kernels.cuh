@@ -280,6 +280,8 @@ __global__ void __launch_bounds__(BT, MOM ? (BT == 512 ? 2 : 3) : 1) tet_chunk_k
     double *xu = reinterpret_cast<double *>(tsm_raw + sizeof(double) * NL * CE + chunk_list_smem(NL, CE, C.L.max_nu));
     const int64_t e0 = (int64_t)blockIdx.x * CE;
     const int ne = (int)(C.E - e0 < CE ? C.E - e0 : CE);
+    pdl_trigger();
+    pdl_wait();  // the slot lists do not depend on earlier kernels
     if (!diag) {
         chunk_load_x<double, BT>(C.L, blockIdx.x, x, xu, constrained);
         __syncthreads();

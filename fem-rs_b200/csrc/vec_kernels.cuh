@@ -130,6 +130,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_init(int64_t n, const T *__
                                                           T *__restrict__ r, T *__restrict__ z,
                                                           T *__restrict__ p, int jacobi,
                                                           double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     double v[2] = {0.0, 0.0};
     FG_VEC4_LOOP(q, n) {
         const V4<T> bv = ld4(b, q), av = ld4(ap, q);
@@ -178,6 +180,8 @@ template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_pcg_pap(int64_t n, const T *__restrict__ p,
                                                          const T *__restrict__ ap,
                                                          double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (st->done) return;
     double v[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
@@ -205,6 +209,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_update(int64_t n, T *__rest
                                                             const T *__restrict__ dinv,
                                                             T *__restrict__ z, int jacobi,
                                                             double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (st->done) return;
     const T alpha = (T)st->alpha;
     double v[2] = {0.0, 0.0};
@@ -287,6 +293,7 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_fused_jacobi(int64_t n, T *
                                                                   const T *__restrict__ dinv, T *__restrict__ z,
                                                                   double *partials, SolverState *st, unsigned *bar,
                                                                   int *err) {
+    pdl_trigger();
     if (st->done) return;
     const double rz0 = st->rz, bnorm = st->bnorm, rtol = st->rtol, atol = st->atol, stop_abs = st->stop_abs;
     const int iter0 = st->iter, max_iter = st->max_iter, cgop = st->cgop;
@@ -361,6 +368,8 @@ template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_pcg_rz(int64_t n, const T *__restrict__ r,
                                                         const T *__restrict__ z,
                                                         double *partials, SolverState *st, int init) {
+    pdl_trigger();
+    pdl_wait();
     if (st->done) return;
     double v[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
@@ -379,6 +388,8 @@ template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_pcg_pupdate(int64_t n, const T *__restrict__ z,
                                                              T *__restrict__ p,
                                                              const SolverState *st, int init) {
+    pdl_trigger();
+    pdl_wait();
     if (st->done) return;
     const T beta = init ? T(0) : (T)st->beta;
     FG_VEC4_LOOP(q, n) {
@@ -401,6 +412,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_first(int64_t n, const T *
                                                             T *__restrict__ d,
                                                             T *__restrict__ z, double inv_theta,
                                                             const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (st && st->done) return;
     const T it = (T)inv_theta;
     FG_VEC4_LOOP(q, n) {
@@ -424,6 +437,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_step(int64_t n, const T *_
                                                            T *__restrict__ d,
                                                            T *__restrict__ z, double c1,
                                                            double c2, const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (st && st->done) return;
     const T a1 = (T)c1, a2 = (T)c2;
     FG_VEC4_LOOP(q, n) {
@@ -457,6 +472,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_first_d(int64_t n, const T
                                                               const T *__restrict__ dinv,
                                                               T *__restrict__ res, T *__restrict__ d,
                                                               double inv_theta, const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (st && st->done) return;
     const T it = (T)inv_theta;
     FG_VEC4_LOOP(q, n) {
@@ -479,6 +496,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_mid(int64_t n, const T *__
                                                           const T *__restrict__ dprev,
                                                           T *__restrict__ dnext, double c1, double c2,
                                                           const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (st && st->done) return;
     const T a1 = (T)c1, a2 = (T)c2;
     FG_VEC4_LOOP(q, n) {
@@ -501,6 +520,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_last(int64_t n, const T *_
                                                            const T *__restrict__ dprev,
                                                            const ChebSum<T> earlier, T *__restrict__ z,
                                                            double c1, double c2, const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (st && st->done) return;
     const T a1 = (T)c1, a2 = (T)c2;
     FG_VEC4_LOOP(q, n) {
@@ -524,6 +545,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_last(int64_t n, const T *_
 __global__ void __launch_bounds__(VEC_THREADS) k_true_residual(int64_t n, const double *__restrict__ b,
                                                                const double *__restrict__ ap,
                                                                double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     double v[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
         const V4<double> bv = ld4(b, q), av = ld4(ap, q);
@@ -549,6 +572,8 @@ __device__ __forceinline__ double hash_unit(uint64_t i) {
 
 __global__ void __launch_bounds__(VEC_THREADS) k_hash_vector(const Grid g, double *__restrict__ v,
                                                              double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t n = (int64_t)g.NIp * g.NJ * g.NK;
     double acc[1] = {0.0};
     FG_VEC_LOOP(i, n) {
@@ -567,6 +592,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_hash_vector(const Grid g, doubl
 __global__ void __launch_bounds__(VEC_THREADS) k_scale_by_rho(int64_t n, const double *__restrict__ w,
                                                               double *__restrict__ v,
                                                               const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     const double rho = st->rho;
     if (!(rho > 1e-14)) return;
     const double inv = 1.0 / rho;
@@ -581,6 +608,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_scale_by_rho(int64_t n, const d
 __global__ void __launch_bounds__(VEC_THREADS) k_dinv_norm(int64_t n, double *__restrict__ w,
                                                            const double *__restrict__ dinv,
                                                            double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     double acc[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
         V4<double> wv = ld4(w, q);
@@ -599,6 +628,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_dinv_norm(int64_t n, double *__
 template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_invert_diag(const Grid g, const double *__restrict__ d,
                                                              T *__restrict__ dinv) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t n = (int64_t)g.NIp * g.NJ * g.NK;
     FG_VEC_LOOP(i, n) {
         const int I = (int)(i % g.NIp);
@@ -615,6 +646,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_residual(int64_t n, const do
                                                              const double *__restrict__ ap,
                                                              double *__restrict__ r, double *partials,
                                                              SolverState *st, int init) {
+    pdl_trigger();
+    pdl_wait();
     double v[2] = {0.0, 0.0};
     FG_VEC4_LOOP(q, n) {
         const V4<double> bv = ld4(b, q), av = ld4(ap, q);
@@ -650,6 +683,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_residual(int64_t n, const do
 __global__ void __launch_bounds__(VEC_THREADS) k_ir_to_f32(int64_t n, const double *__restrict__ r,
                                                            float *__restrict__ r32,
                                                            const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     const double s = st->rr > 0.0 ? 1.0 / sqrt(st->rr) : 0.0;
     FG_VEC4_LOOP(q, n) {
         const V4<double> rv = ld4(r, q);
@@ -663,6 +698,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_to_f32(int64_t n, const doub
 __global__ void __launch_bounds__(VEC_THREADS) k_ir_update(int64_t n, double *__restrict__ x,
                                                            const float *__restrict__ e,
                                                            const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     const double s = sqrt(st->rr);
     FG_VEC4_LOOP(q, n) {
         V4<double> xv = ld4(x, q);
@@ -675,6 +712,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_update(int64_t n, double *__
 // FP32 copy of an FP64 vector
 __global__ void __launch_bounds__(VEC_THREADS) k_to_f32(int64_t n, const double *__restrict__ a,
                                                         float *__restrict__ b) {
+    pdl_trigger();
+    pdl_wait();
     FG_VEC_LOOP(i, n) b[i] = (float)a[i];
 }
 
@@ -685,6 +724,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_to_f32(int64_t n, const double 
 template <typename T>
 __global__ void __launch_bounds__(256) k_repitch(const T *__restrict__ src, int64_t sp, T *__restrict__ dst,
                                                  int64_t dp, int w, int64_t rows) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -708,6 +749,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_step(int64_t n, float *__re
                                                           const float *__restrict__ p,
                                                           const float *__restrict__ ap,
                                                           double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (st->done) return;
     const float alpha = (float)st->alpha;
     double v[1] = {0.0};
@@ -738,6 +781,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_step(int64_t n, float *__re
 __global__ void __launch_bounds__(VEC_THREADS) k_rel_xupdate(int64_t n, double *__restrict__ x,
                                                              float *__restrict__ xlo,
                                                              const SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     if (!st->trigger) return;
     FG_VEC4_LOOP(q, n) {
         V4<double> xv = ld4(x, q);
@@ -755,6 +800,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_residual(int64_t n, const d
                                                               float *__restrict__ r,
                                                               double *partials, SolverState *st,
                                                               int init) {
+    pdl_trigger();
+    pdl_wait();
     if (!init && !st->trigger) return;
     double v[2] = {0.0, 0.0};
     FG_VEC4_LOOP(q, n) {
@@ -802,6 +849,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_jacobi_rz(int64_t n, const T *_
                                                            const T *__restrict__ dinv,
                                                            T *__restrict__ z, double *partials,
                                                            SolverState *st, int init) {
+    pdl_trigger();
+    pdl_wait();
     if (st->done) return;
     double v[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
@@ -824,6 +873,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_jacobi_rz(int64_t n, const T *_
 __global__ void __launch_bounds__(VEC_THREADS) k_lincomb2(int64_t n, double *__restrict__ out, double a,
                                                           const double *__restrict__ x, double b,
                                                           const double *__restrict__ y) {
+    pdl_trigger();
+    pdl_wait();
     FG_VEC4_LOOP(q, n) {
         const V4<double> xv = ld4(x, q), yv = ld4(y, q);
         V4<double> o;
@@ -1078,6 +1129,8 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_true_residual(const BatchVec *
 // st->tmp[2] = ||v|| (FP64)
 __global__ void __launch_bounds__(VEC_THREADS) k_norm_tmp(int64_t n, const double *__restrict__ v,
                                                           double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     double a[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
         const V4<double> x = ld4(v, q);
@@ -1090,6 +1143,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_norm_tmp(int64_t n, const doubl
 // v *= 1/tmp[2] (inverse = 1) or v *= tmp[2]; no-op when tmp[2] == 0
 __global__ void __launch_bounds__(VEC_THREADS) k_scale_tmp(int64_t n, double *__restrict__ v,
                                                            const SolverState *st, int inverse) {
+    pdl_trigger();
+    pdl_wait();
     const double s = st->tmp[2];
     if (!(s > 0.0)) return;
     const double f = inverse ? 1.0 / s : s;
@@ -1105,6 +1160,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_scale_tmp(int64_t n, double *__
 __global__ void __launch_bounds__(VEC_THREADS) k_energy_terms(int64_t n, const double *__restrict__ c,
                                                               double *__restrict__ ac, const double *__restrict__ r,
                                                               double *partials, SolverState *st) {
+    pdl_trigger();
+    pdl_wait();
     double a[2] = {0.0, 0.0};
     FG_VEC4_LOOP(q, n) {
         const V4<double> cv = ld4(c, q), rv = ld4(r, q);
@@ -1129,6 +1186,8 @@ template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_fcg_zap(int64_t n, const T *__restrict__ z,
                                                          const T *__restrict__ ap, double *partials,
                                                          SolverState *st, int init) {
+    pdl_trigger();
+    pdl_wait();
     if (st->done) return;
     double v[1] = {0.0};
     if (!init) {
@@ -1151,6 +1210,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_fcg_pupdate_pr(int64_t n, const
                                                                 T *__restrict__ p,
                                                                 const T *__restrict__ r, double *partials,
                                                                 SolverState *st, int init) {
+    pdl_trigger();
+    pdl_wait();
     if (st->done) return;
     const T beta = init ? T(0) : (T)st->beta;
     double v[1] = {0.0};
@@ -1184,6 +1245,8 @@ struct VecPairs {
 template <int NV>
 __global__ void __launch_bounds__(VEC_THREADS) k_sh_dots(int64_t n_own, const VecPairs P, double *partials,
                                                          SolverState *st, double *out) {
+    pdl_trigger();
+    pdl_wait();
     double v[NV];
 #pragma unroll
     for (int j = 0; j < NV; ++j) v[j] = 0.0;
@@ -1209,6 +1272,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_sh_update(int64_t n, int64_t n_
                                                            const double *__restrict__ dinv, double *__restrict__ z,
                                                            const double *s, double *partials, SolverState *st,
                                                            double *out) {
+    pdl_trigger();
+    pdl_wait();
     const double alpha = s[0] / s[1];
     double v[2] = {0.0, 0.0};
     FG_VEC4_LOOP(q, n) {
@@ -1240,6 +1305,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_sh_update(int64_t n, int64_t n_
 __global__ void __launch_bounds__(VEC_THREADS) k_sh_pupdate(int64_t n, const double *__restrict__ z,
                                                             double *__restrict__ p, const double *num,
                                                             const double *den) {
+    pdl_trigger();
+    pdl_wait();
     const double beta = *num / *den;
     FG_VEC4_LOOP(q, n) {
         const V4<double> zv = ld4(z, q);
