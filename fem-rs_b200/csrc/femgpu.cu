@@ -3796,7 +3796,7 @@ FG_API int fg_tet_create(int order, int64_t n_nodes, const double *coords, int64
                 return fail(FG_BOUNDS, "element %lld local DOF %d out of range", (long long)e, i);
             soa[(int64_t)i * n_elem + e] = d;
         }
-    t->CE = order == 3 ? 256 : 512;
+    t->CE = order == 3 ? 128 : 512;
     if (const char *ev = std::getenv("FG_TET_CHUNK")) {
         const int v = std::atoi(ev);
         if (v >= 32 && v <= 1024 && v * nl <= 65536) t->CE = v;
@@ -3824,8 +3824,9 @@ FG_API int fg_tet_create(int order, int64_t n_nodes, const double *coords, int64
     if (t->nq > TET_MAXQ) return fail(FG_UNSUPPORTED, "quadrature order %d too high", quad_order);
     std::vector<double> phi((size_t)t->nq * nl), grad((size_t)t->nq * nl * 3);
     for (int q = 0; q < t->nq; ++q) tet_basis_host(order, &pts[3 * q], &phi[(size_t)q * nl], &grad[(size_t)q * nl * 3]);
-    t->h_phi = phi;
-    t->h_grad = grad;
+    std::vector<double> TF, TB;
+    tet_point_tables(nl, kind, t->nq, phi, grad, TF, TB);
+    if ((rc = tet_upload(&t->TF, TF.data(), TF.size())) || (rc = tet_upload(&t->TB, TB.data(), TB.size()))) return rc;
     double *d_w = nullptr;
     if ((rc = tet_upload(&t->qp, pts.data(), pts.size())) || (rc = tet_upload(&t->phi, phi.data(), phi.size())) ||
         (rc = tet_upload(&t->grad, grad.data(), grad.size())) || (rc = tet_upload(&d_w, w.data(), w.size())))

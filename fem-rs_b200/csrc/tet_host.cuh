@@ -17,7 +17,7 @@ struct fg_tet {
     int32_t *dofs = nullptr;  // [nl][E] caller's element order (setup, quadrature points)
     double *G = nullptr, *sk = nullptr, *sm = nullptr, *Sm = nullptr, *coords = nullptr;  // chunk order
     double *qp = nullptr, *phi = nullptr, *grad = nullptr;  // rule tables (device)
-    std::vector<double> h_phi, h_grad;                       // rule tables (host, kernel parameters)
+    double *TF = nullptr, *TB = nullptr;                     // rule tables of tet_point_kernel
     int nq = 0;
     // chunked gather and scatter
     int CE = 0, n_chunks = 0, wide = 0;  // wide: 512-thread CTAs for the P2 moment form
@@ -201,7 +201,7 @@ static void tet_free(fg_tet *t) {
     if (!t) return;
     cudaSetDevice(t->device);
     if (t->stream) cudaStreamSynchronize(t->stream);
-    void *ptrs[] = {t->dofs, t->G, t->sk, t->sm, t->Sm, t->coords, t->qp, t->phi, t->grad, t->part, t->xh, t->yh, t->d_err};
+    void *ptrs[] = {t->dofs, t->G, t->sk, t->sm, t->Sm, t->coords, t->qp, t->phi, t->grad, t->TF, t->TB, t->part, t->xh, t->yh, t->d_err};
     t->lists.release();
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -235,42 +235,79 @@ static void tet_plan_chunks(const std::vector<int32_t> &h, const std::vector<dou
     plan_chunk_lists(smap, E, N, nl, CE, ess, P);
 }
 
-template <int NL, int MQ, bool MOM, int BT>
-static int tet_launch_t(fg_tet *t, const TetChunk &C, const double *x, double *y, int accumulate, int constrained,
-                        int diag) {
-    TetTab<NL, MQ> R{};
-    if (!MOM)
-        for (int q = 0; q < t->nq; ++q)
-            for (int i = 0; i < NL; ++i) {
-                R.phi[q][i] = t->h_phi[(size_t)q * NL + i];
-                for (int c = 0; c < 3; ++c) R.grad[q][i][c] = t->h_grad[((size_t)q * NL + i) * 3 + c];
-            }
-    const size_t smem = tet_chunk_smem(NL, t->CE, t->lists.max_nu);
-    if (smem > 48 * 1024)
-        CK(cudaFuncSetAttribute(tet_chunk_kernel<NL, MQ, MOM, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
-    CK(launch_dep(tet_chunk_kernel<NL, MQ, MOM, BT>, dim3(t->n_chunks), BT, smem, t->stream, C, t->kind, t->nq, R, x, y,
-                  accumulate, constrained, diag));
+// The rule's tables in the fragment order of tet_point_kernel.
+static void tet_point_tables(int nl, int kind, int nq, const std::vector<double> &phi, const std::vector<double> &grad,
+                             std::vector<double> &TF, std::vector<double> &TB) {
+    const int NC = (kind & 2 ? 3 : 0) + (kind & 1 ? 1 : 0), KS = (nl + 3) / 4, IT = (nl + 7) / 8, QT = (nq + 7) / 8;
+    auto at = [&](int c, int q, int i) {
+        if (q >= nq || i >= nl) return 0.0;
+        return (kind & 2) && c < 3 ? grad[((size_t)q * nl + i) * 3 + c] : phi[(size_t)q * nl + i];
+    };
+    TF.clear();
+    TB.clear();
+    for (int t = 0; t < QT; ++t)
+        for (int c = 0; c < NC; ++c) {
+            for (int ks = 0; ks < KS; ++ks)
+                for (int l = 0; l < 32; ++l) TF.push_back(at(c, 8 * t + l / 4, 4 * ks + l % 4));
+            for (int j = 0; j < 2; ++j)
+                for (int it = 0; it < IT; ++it)
+                    for (int l = 0; l < 32; ++l) TB.push_back(at(c, 8 * t + 2 * (l % 4) + j, 8 * it + l / 4));
+        }
+}
+
+// Dynamic shared memory of a chunk kernel, its limit raised where needed.
+template <typename K> static int tet_smem(fg_tet *t, K kern, int NL, size_t *smem) {
+    *smem = tet_chunk_smem(NL, t->CE, t->lists.max_nu);
+    if (*smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+    return FG_OK;
+}
+template <int NL, int BT>
+static int tet_launch_moment(fg_tet *t, const TetChunk &C, const double *x, double *y, int accumulate, int constrained) {
+    size_t smem;
+    int rc;
+    if ((rc = tet_smem(t, tet_moment_kernel<NL, BT>, NL, &smem))) return rc;
+    CK(launch_dep(tet_moment_kernel<NL, BT>, dim3(t->n_chunks), BT, smem, t->stream, C, x, y, accumulate, constrained));
+    return FG_OK;
+}
+template <int NL, int KIND, int BT>
+static int tet_launch_point(fg_tet *t, const TetChunk &C, const double *x, double *y, int accumulate, int constrained) {
+    size_t smem;
+    int rc;
+    if ((rc = tet_smem(t, tet_point_kernel<NL, KIND, BT>, NL, &smem))) return rc;
+    CK(launch_dep(tet_point_kernel<NL, KIND, BT>, dim3(t->n_chunks), BT, smem, t->stream, C, t->nq, t->TF, t->TB, x, y,
+                  accumulate, constrained));
+    return FG_OK;
+}
+template <int NL> static int tet_launch_diag(fg_tet *t, const TetChunk &C, double *y, int constrained) {
+    size_t smem;
+    int rc;
+    if ((rc = tet_smem(t, tet_diag_kernel<NL, 256>, NL, &smem))) return rc;
+    tet_diag_kernel<NL, 256><<<t->n_chunks, 256, smem, t->stream>>>(C, t->kind, t->nq, TetRule{t->nq, t->phi, t->grad}, y,
+                                                                     constrained);
     return FG_OK;
 }
 
 static int tet_launch_apply(fg_tet *t, const double *x, double *y, int accumulate, int constrained, int diag) {
     const TetChunk C = tet_chunk_args(t);
-    const bool small = t->nq <= 4;
-    const bool mom = !diag && t->kind == 2 && t->p <= 2;
     int rc;
-    if (t->p == 1) {
-        if (mom) rc = tet_launch_t<4, 1, true, 256>(t, C, x, y, accumulate, constrained, diag);
-        else if (small) rc = tet_launch_t<4, 4, false, 256>(t, C, x, y, accumulate, constrained, diag);
-        else rc = tet_launch_t<4, TET_MAXQ, false, 256>(t, C, x, y, accumulate, constrained, diag);
-    } else if (t->p == 2) {
-        if (mom && t->wide) rc = tet_launch_t<10, 1, true, 512>(t, C, x, y, accumulate, constrained, diag);
-        else if (mom) rc = tet_launch_t<10, 1, true, 256>(t, C, x, y, accumulate, constrained, diag);
-        else if (small) rc = tet_launch_t<10, 4, false, 256>(t, C, x, y, accumulate, constrained, diag);
-        else rc = tet_launch_t<10, TET_MAXQ, false, 256>(t, C, x, y, accumulate, constrained, diag);
+    if (diag) {
+        rc = t->p == 1 ? tet_launch_diag<4>(t, C, y, constrained)
+             : t->p == 2 ? tet_launch_diag<10>(t, C, y, constrained) : tet_launch_diag<20>(t, C, y, constrained);
     } else {
-        if (small) rc = tet_launch_t<20, 4, false, 256>(t, C, x, y, accumulate, constrained, diag);
-        else rc = tet_launch_t<20, TET_MAXQ, false, 256>(t, C, x, y, accumulate, constrained, diag);
+        switch (t->p * 4 + t->kind) {
+        case 1 * 4 + 1: rc = tet_launch_point<4, 1, 256>(t, C, x, y, accumulate, constrained); break;
+        case 1 * 4 + 2: rc = tet_launch_moment<4, 256>(t, C, x, y, accumulate, constrained); break;
+        case 1 * 4 + 3: rc = tet_launch_point<4, 3, 256>(t, C, x, y, accumulate, constrained); break;
+        case 2 * 4 + 1: rc = tet_launch_point<10, 1, 256>(t, C, x, y, accumulate, constrained); break;
+        case 2 * 4 + 2:
+            rc = t->wide ? tet_launch_moment<10, 512>(t, C, x, y, accumulate, constrained)
+                         : tet_launch_moment<10, 256>(t, C, x, y, accumulate, constrained);
+            break;
+        case 2 * 4 + 3: rc = tet_launch_point<10, 3, 256>(t, C, x, y, accumulate, constrained); break;
+        case 3 * 4 + 1: rc = tet_launch_point<20, 1, 128>(t, C, x, y, accumulate, constrained); break;
+        case 3 * 4 + 2: rc = tet_launch_point<20, 2, 128>(t, C, x, y, accumulate, constrained); break;
+        default: rc = tet_launch_point<20, 3, 128>(t, C, x, y, accumulate, constrained); break;
+        }
     }
     if (rc) return rc;
     if (t->lists.n_shared) {

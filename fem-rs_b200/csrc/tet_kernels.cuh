@@ -107,19 +107,42 @@ __global__ void tet_setup_kernel(TetArgs A, int nl, const double *__restrict__ c
     }
 }
 
-// Rule tables passed by value as a kernel parameter (constant bank): every
-// thread of a warp reads the same entry at the same time, so the reads are
-// broadcasts.  MQ = capacity in points (4 for tet_rule orders <= 2, 35 above).
-template <int NL, int MQ> struct TetTab {
-    double phi[MQ][NL];
-    double grad[MQ][NL][3];
+// ---- point form on the FP64 tensor cores ------------------------------------
+// The point form is two small GEMMs per element with the rule's tables as the
+// fixed operand: values and reference gradients at the points, V = x T (K = the
+// NL local DOFs), then, after the point scalars and G, y = W T^T (K = the points).
+// mma.m8n8k4 (FP64, fused multiply-adds) takes eight elements as its rows: a lane
+// holds element lane / 4, local DOFs 4 ks + lane % 4 of x as the first operand, and gets
+// the points 8 t + 2 (lane % 4) + {0, 1} of each table in the same accumulator
+// registers, so the point scalars apply without moving data.  The second product
+// takes those registers as they are: k-step j of a block of eight points holds
+// points 8 t + 2 (lane % 4) + j, and the table is stored in that order.
+//
+// What bounds it: the FP64 rate once enough warps are there.  One thread per
+// element (the form before) ran 5,600 multiply-adds a P3 element behind indexed
+// constant loads with 234 registers: 8 warps per SM, the pipe a quarter busy.
+// 48,000 P3 tetrahedra, mass + diffusion, 35 points: 122 -> 46.7 us (chunks of 128
+// elements; 256: 82, 64: 47); 280,000 P1, 15 points: 80.8 -> 44.7.  The error against
+// 64-bit sums in another order is unchanged (1.7e-14).
+//
+// Tables in fragment order (tet_point_tables): TF [t][table][ks][lane] =
+// table(point 8 t + lane / 4, DOF 4 ks + lane % 4) and TB [t][table][j][it][lane] =
+// table(point 8 t + 2 (lane % 4) + j, DOF 8 it + lane / 4), zero beyond the rule and
+// the element; tables: the gradient components (diffusion), then the values (mass).
+template <int NL> struct TetPoint {
+    static constexpr int KS = (NL + 3) / 4, IT = (NL + 7) / 8;
 };
 
-// Element results by the point form: ye = A_e xe (diag = 0) or the diagonal of
-// A_e (diag = 1) for element e of the chunk order.
-template <int NL, int MQ>
-__device__ __forceinline__ void tet_elem_points(const TetChunk &C, int kind, int nq, const TetTab<NL, MQ> &R,
-                                                int64_t e, const double (&xe)[NL], double (&ye)[NL], int diag) {
+__device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// Diagonal of element e of the chunk order (a set-up kernel: one thread per element).
+template <int NL>
+__device__ __forceinline__ void tet_elem_diag(const TetChunk &C, int kind, int nq, const TetRule &R, int64_t e,
+                                              double (&ye)[NL]) {
     const int64_t E = C.E;
 #pragma unroll
     for (int i = 0; i < NL; ++i) ye[i] = 0.0;
@@ -128,42 +151,19 @@ __device__ __forceinline__ void tet_elem_points(const TetChunk &C, int kind, int
 #pragma unroll
         for (int k = 0; k < 6; ++k) g[k] = __ldg(C.G + (int64_t)k * E + e);
     for (int q = 0; q < nq; ++q) {
+        const double *gr = R.grad + (int64_t)q * NL * 3, *ph = R.phi + (int64_t)q * NL;
         if (kind & 2) {
             const double s = __ldg(C.sk + (int64_t)q * E + e);
-            if (!diag) {
-                double gu[3] = {0, 0, 0};
 #pragma unroll
-                for (int j = 0; j < NL; ++j)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) gu[c] += xe[j] * R.grad[q][j][c];
-                const double v0 = s * (g[0] * gu[0] + g[1] * gu[1] + g[2] * gu[2]);
-                const double v1 = s * (g[1] * gu[0] + g[3] * gu[1] + g[4] * gu[2]);
-                const double v2 = s * (g[2] * gu[0] + g[4] * gu[1] + g[5] * gu[2]);
-#pragma unroll
-                for (int i = 0; i < NL; ++i)
-                    ye[i] += R.grad[q][i][0] * v0 + R.grad[q][i][1] * v1 + R.grad[q][i][2] * v2;
-            } else {
-#pragma unroll
-                for (int i = 0; i < NL; ++i) {
-                    const double a = R.grad[q][i][0], b = R.grad[q][i][1], c = R.grad[q][i][2];
-                    ye[i] += s * (g[0] * a * a + g[3] * b * b + g[5] * c * c +
-                                  2.0 * (g[1] * a * b + g[2] * a * c + g[4] * b * c));
-                }
+            for (int i = 0; i < NL; ++i) {
+                const double a = __ldg(gr + 3 * i), b = __ldg(gr + 3 * i + 1), c = __ldg(gr + 3 * i + 2);
+                ye[i] += s * (g[0] * a * a + g[3] * b * b + g[5] * c * c + 2.0 * (g[1] * a * b + g[2] * a * c + g[4] * b * c));
             }
         }
         if (kind & 1) {
             const double m = __ldg(C.sm + (int64_t)q * E + e);
-            if (!diag) {
-                double u = 0.0;
 #pragma unroll
-                for (int j = 0; j < NL; ++j) u += R.phi[q][j] * xe[j];
-                const double t = m * u;
-#pragma unroll
-                for (int i = 0; i < NL; ++i) ye[i] += R.phi[q][i] * t;
-            } else {
-#pragma unroll
-                for (int i = 0; i < NL; ++i) ye[i] += m * R.phi[q][i] * R.phi[q][i];
-            }
+            for (int i = 0; i < NL; ++i) ye[i] += m * __ldg(ph + i) * __ldg(ph + i);
         }
     }
 }
@@ -260,19 +260,17 @@ __host__ __device__ inline size_t tet_chunk_smem(int NL, int CE, int max_nu) {
     return sizeof(double) * ((size_t)NL * CE + max_nu) + chunk_list_smem(NL, CE, max_nu);
 }
 
-// One CTA (BT threads) per chunk.  The copies of the chunk's slot lists are
-// started and its values of x read once into shared memory; then the element
+// One CTA (BT threads) per chunk; diffusion by the moment form (P1, P2).  The
+// copies of the chunk's slot lists are started and its values of x read once into shared memory; then the element
 // results are computed into shared memory, each element taking its values by
 // its 16-bit positions.  After a barrier each DOF's slots are summed.  MOM:
 // diffusion-only apply by the moment form.  On essential DOFs of a constrained call
 // the identity row: y_d (+)= x_d (apply) or 1 (diagonal).  40^3 x 6 P2 tetrahedra:
 // 41.0 us with x gathered per element through a 32-bit map, 37.0 us this way.
-template <int NL, int MQ, bool MOM, int BT>
-__global__ void __launch_bounds__(BT, MOM ? (BT == 512 ? 2 : 3) : 1) tet_chunk_kernel(const TetChunk C, int kind, int nq,
-                                                                  const __grid_constant__ TetTab<NL, MQ> R,
-                                                                  const double *__restrict__ x,
-                                                                  double *__restrict__ y, int accumulate,
-                                                                  int constrained, int diag) {
+template <int NL, int BT>
+__global__ void __launch_bounds__(BT, BT == 512 ? 2 : 3) tet_moment_kernel(const TetChunk C, const double *__restrict__ x,
+                                                                         double *__restrict__ y, int accumulate,
+                                                                         int constrained) {
     extern __shared__ __align__(16) unsigned char tsm_raw[];
     const int CE = C.CE;
     double *ys = reinterpret_cast<double *>(tsm_raw);  // [NL][CE] element results
@@ -282,25 +280,147 @@ __global__ void __launch_bounds__(BT, MOM ? (BT == 512 ? 2 : 3) : 1) tet_chunk_k
     const int ne = (int)(C.E - e0 < CE ? C.E - e0 : CE);
     pdl_trigger();
     pdl_wait();  // the slot lists do not depend on earlier kernels
-    if (!diag) {
-        chunk_load_x<double, BT>(C.L, blockIdx.x, x, xu, constrained);
-        __syncthreads();
-    }
+    chunk_load_x<double, BT>(C.L, blockIdx.x, x, xu, constrained);
+    __syncthreads();
     for (int el = threadIdx.x; el < ne; el += BT) {
         const int64_t e = e0 + el;
-        double xe[NL], ye[NL];
-        double md[MOM ? TetMom<NL>::n : 1];
-        if constexpr (MOM) tet_load_moments<NL>(C, e, md);
+        double xe[NL], ye[NL], md[TetMom<NL>::n];
+        tet_load_moments<NL>(C, e, md);
 #pragma unroll
-        for (int i = 0; i < NL; ++i) xe[i] = diag ? 0.0 : xu[__ldg(C.L.lmap + (int64_t)i * C.E + e)];
-        if constexpr (MOM) tet_elem_moments<NL>(md, xe, ye);
-        else tet_elem_points<NL, MQ>(C, kind, nq, R, e, xe, ye, diag);
+        for (int i = 0; i < NL; ++i) xe[i] = xu[__ldg(C.L.lmap + (int64_t)i * C.E + e)];
+        tet_elem_moments<NL>(md, xe, ye);
 #pragma unroll
         for (int i = 0; i < NL; ++i) ys[i * CE + el] = ye[i];
     }
     chunk_wait();
     __syncthreads();
-    chunk_sums<double, BT>(C.L, S, ys, x, y, accumulate, constrained, diag);
+    chunk_sums<double, BT>(C.L, S, ys, x, y, accumulate, constrained, 0);
+}
+
+// The same chunk scheme by the point form: a warp takes 16 elements (two
+// eight-row tiles that share the table operand) at a time.
+template <int NL, int KIND, int BT>
+__global__ void __launch_bounds__(BT) tet_point_kernel(const TetChunk C, int nq, const double *__restrict__ TF,
+                                                       const double *__restrict__ TB, const double *__restrict__ x,
+                                                       double *__restrict__ y, int accumulate, int constrained) {
+    constexpr bool HM = (KIND & 1) != 0, HK = (KIND & 2) != 0;
+    constexpr int NC = (HK ? 3 : 0) + (HM ? 1 : 0), KS = TetPoint<NL>::KS, IT = TetPoint<NL>::IT;
+    extern __shared__ __align__(16) unsigned char tsm_raw[];
+    const int CE = C.CE;
+    const int64_t E = C.E;
+    double *ys = reinterpret_cast<double *>(tsm_raw);  // [NL][CE] element results
+    const ChunkStage S = chunk_stage_lists<BT>(C.L, blockIdx.x, tsm_raw + sizeof(double) * NL * CE);
+    double *xu = reinterpret_cast<double *>(tsm_raw + sizeof(double) * NL * CE + chunk_list_smem(NL, CE, C.L.max_nu));
+    const int64_t e0 = (int64_t)blockIdx.x * CE;
+    const int ne = (int)(E - e0 < CE ? E - e0 : CE);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r8 = lane >> 2, l4 = lane & 3;
+    const int QT = (nq + 7) / 8;
+    pdl_trigger();
+    pdl_wait();
+    chunk_load_x<double, BT>(C.L, blockIdx.x, x, xu, constrained);
+    __syncthreads();
+    for (int t16 = warp * 16; t16 < ne; t16 += BT / 2) {
+        double xa[2][KS], G[2][6], Y[2][IT][2];
+        bool ok[2];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int el = t16 + 8 * p + r8;
+            ok[p] = el < ne;
+            const int64_t e = e0 + (ok[p] ? el : 0);
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks) {
+                const int i = 4 * ks + l4;
+                xa[p][ks] = ok[p] && i < NL ? xu[__ldg(C.L.lmap + (int64_t)i * E + e)] : 0.0;
+            }
+            if (HK)
+#pragma unroll
+                for (int k = 0; k < 6; ++k) G[p][k] = __ldg(C.G + (int64_t)k * E + e);
+#pragma unroll
+            for (int it = 0; it < IT; ++it) Y[p][it][0] = Y[p][it][1] = 0.0;
+        }
+        for (int t = 0; t < QT; ++t) {
+            double sc[2][2], mc[2][2];  // point scalars of this lane's points
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int q = 8 * t + 2 * l4 + j;
+                    const bool v = ok[p] && q < nq;
+                    const int64_t o = (int64_t)q * E + e0 + t16 + 8 * p + r8;
+                    if (HK) sc[p][j] = v ? __ldg(C.sk + o) : 0.0;
+                    if (HM) mc[p][j] = v ? __ldg(C.sm + o) : 0.0;
+                }
+            double V[2][NC][2];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+#pragma unroll
+                for (int p = 0; p < 2; ++p) V[p][c][0] = V[p][c][1] = 0.0;
+#pragma unroll
+                for (int ks = 0; ks < KS; ++ks) {
+                    const double b = __ldg(TF + (((int64_t)t * NC + c) * KS + ks) * 32 + lane);
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) dmma_884(V[p][c], xa[p][ks], b);
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const bool v = 8 * t + 2 * l4 + j < nq;
+                    if (HK) {
+                        const double gx = V[p][0][j], gy = V[p][1][j], gz = V[p][2][j], s = sc[p][j];
+                        V[p][0][j] = v ? s * (G[p][0] * gx + G[p][1] * gy + G[p][2] * gz) : 0.0;
+                        V[p][1][j] = v ? s * (G[p][1] * gx + G[p][3] * gy + G[p][4] * gz) : 0.0;
+                        V[p][2][j] = v ? s * (G[p][2] * gx + G[p][4] * gy + G[p][5] * gz) : 0.0;
+                    }
+                    if (HM) V[p][NC - 1][j] = v ? mc[p][j] * V[p][NC - 1][j] : 0.0;
+                }
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int it = 0; it < IT; ++it) {
+                        const double b = __ldg(TB + ((((int64_t)t * NC + c) * 2 + j) * IT + it) * 32 + lane);
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) dmma_884(Y[p][it], V[p][c][j], b);
+                    }
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+            if (ok[p])
+#pragma unroll
+                for (int it = 0; it < IT; ++it)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int i = 8 * it + 2 * l4 + j;
+                        if (i < NL) ys[i * CE + t16 + 8 * p + r8] = Y[p][it][j];
+                    }
+    }
+    chunk_wait();
+    __syncthreads();
+    chunk_sums<double, BT>(C.L, S, ys, x, y, accumulate, constrained, 0);
+}
+
+// Jacobi diagonal, one thread per element (1 on essential DOFs of a constrained call).
+template <int NL, int BT>
+__global__ void __launch_bounds__(BT) tet_diag_kernel(const TetChunk C, int kind, int nq, const TetRule R,
+                                                      double *__restrict__ y, int constrained) {
+    extern __shared__ __align__(16) unsigned char tsm_raw[];
+    const int CE = C.CE;
+    double *ys = reinterpret_cast<double *>(tsm_raw);
+    const ChunkStage S = chunk_stage_lists<BT>(C.L, blockIdx.x, tsm_raw + sizeof(double) * NL * CE);
+    const int64_t e0 = (int64_t)blockIdx.x * CE;
+    const int ne = (int)(C.E - e0 < CE ? C.E - e0 : CE);
+    for (int el = threadIdx.x; el < ne; el += BT) {
+        double ye[NL];
+        tet_elem_diag<NL>(C, kind, nq, R, e0 + el, ye);
+#pragma unroll
+        for (int i = 0; i < NL; ++i) ys[i * CE + el] = ye[i];
+    }
+    chunk_wait();
+    __syncthreads();
+    chunk_sums<double, BT>(C.L, S, ys, nullptr, y, 0, constrained, 1);
 }
 
 // Reorder the per-element data into the chunk order and form the diffusion

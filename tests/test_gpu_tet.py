@@ -196,3 +196,24 @@ def test_tet_chunk_plans_on_shuffled_mesh(p, kind, chunk, monkeypatch):
         assert rel(y2, ref + 0.5) <= 1e-12
         assert rel(op.diagonal(constrained), O.tet_diagonal(sp, coef, qo, constrained)) <= 1e-12
     assert np.array_equal(op.matvec(x, True), op.matvec(x, True))
+
+
+@pytest.mark.parametrize("p", [1, 2, 3])
+@pytest.mark.parametrize("kind", [femgpu.MASS, femgpu.DIFF, femgpu.MASS_DIFF])
+@pytest.mark.parametrize("quad_order", [1, 2, 5, 7])
+def test_tet_point_form_at_tile_edges(p, kind, quad_order):
+    """The point form at the edges of its tiles: 1, 4, 15 and 35 points (one to
+    five blocks of eight, all ragged), 6 and 48 elements (a part of one
+    sixteen-element pair of tiles, whole pairs); the bound of the apply tests."""
+    need_gpu()
+    for n in (1, 2):
+        coords, dofs, nd, mask = space(n, p, seed=n)
+        nq = len(O.tet_rule(quad_order)[1])
+        rng = np.random.default_rng(10 * p + kind)
+        kq, rq = np.exp(rng.normal(size=dofs.shape[0] * nq)), np.exp(0.3 * rng.normal(size=dofs.shape[0] * nq))
+        op = femgpu.TetOperator(p, coords, dofs, nd, kind=kind, kappa=kq, rho=rq, c_mass=0.7, c_diff=1.3,
+                                quad_order=quad_order, ess=mask)
+        sp = O.TetSpace(p, coords, dofs, nd, mask)
+        coef = O.Coef(kind, c_m=0.7, c_k=1.3, kappa_q=kq, rho_q=rq)
+        x = rng.standard_normal(nd)
+        assert rel(op.matvec(x, False), O.tet_pa_apply(sp, coef, x, quad_order, False)) <= 1e-12
