@@ -25,6 +25,7 @@ struct ConvLayer {
     int cin = 0, cout = 0, kp = 0, kpt = 0;  // kp: padded K of W, kpt: padded K of the flipped W
     float *w = nullptr, *b = nullptr;         // FP32 master parameters (w: [cout][kp])
     __nv_bfloat16 *wb = nullptr;               // BF16 copy used by the kernels
+    __nv_bfloat16 *wt = nullptr;               // flipped copy for the input gradient (in fg_unet::wflip)
     float *gw = nullptr, *gb = nullptr;       // gradients
     float *mw = nullptr, *vw = nullptr, *mb = nullptr, *vb = nullptr;  // Adam moments
 };
@@ -55,6 +56,7 @@ struct fg_unet {
     fg::UnetBufs buf;
     __nv_bfloat16 *wflip = nullptr;
     size_t wflip_n = 0;
+    float *flat = nullptr;  // all parameters or gradients on their way to or from the host
     int step = 0;
     cudaStream_t stream = nullptr;
     int tc = 0;            // FG_UNET_TC=1: convolutions on tcgen05 where the shapes allow (default mma.sync)
@@ -149,26 +151,26 @@ static int unet_ensure_bufs(fg_unet *u, int B, int Z, int Y, int X) {
 
 template <int NT, int KS>
 static void conv_launch(fg_unet *u, bool tapmajor, int blocks, const TView &in, const Vol &V,
-                        const __nv_bfloat16 *w, int cin, int kp, const float *bias, TView out, int relu) {
+                        const __nv_bfloat16 *w, int cin, int kp, const float *bias, TView out, int relu, const TView &mask) {
     if (tapmajor)
-        conv3_fwd16_kernel<NT, KS><<<blocks, 128, 0, u->stream>>>(in, V, cin, w, kp, bias, out, relu);
+        conv3_fwd16_kernel<NT, KS><<<blocks, 128, 0, u->stream>>>(in, V, cin, w, kp, bias, out, relu, mask);
     else
-        conv3_fwd_kernel<NT, KS><<<blocks, 128, 0, u->stream>>>(in, V, cin, w, kp, bias, out, relu);
+        conv3_fwd_kernel<NT, KS><<<blocks, 128, 0, u->stream>>>(in, V, cin, w, kp, bias, out, relu, mask);
 }
 
 template <int KS>
 static int conv_fwd_ks(fg_unet *u, const TView &in, const Vol &V, const __nv_bfloat16 *w, int cin, int cout,
-                       int kp, const float *bias, TView out, int relu) {
+                       int kp, const float *bias, TView out, int relu, const TView &mask) {
     const int64_t tiles = (V.nvox() + 15) / 16;
     const int blocks = (int)((tiles + (4 / KS) - 1) / (4 / KS));
     const bool tm = cin % 16 == 0 && in.cs % 4 == 0 && in.co % 4 == 0;
     switch (cout / 8) {
-    case 1: conv_launch<1, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu); break;
-    case 2: conv_launch<2, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu); break;
-    case 4: conv_launch<4, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu); break;
-    case 6: conv_launch<6, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu); break;
-    case 8: conv_launch<8, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu); break;
-    case 10: conv_launch<10, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu); break;
+    case 1: conv_launch<1, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu, mask); break;
+    case 2: conv_launch<2, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu, mask); break;
+    case 4: conv_launch<4, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu, mask); break;
+    case 6: conv_launch<6, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu, mask); break;
+    case 8: conv_launch<8, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu, mask); break;
+    case 10: conv_launch<10, KS>(u, tm, blocks, in, V, w, cin, kp, bias, out, relu, mask); break;
     default: return fail(FG_UNSUPPORTED, "conv output channels %d not supported", cout);
     }
     CK(cudaGetLastError());
@@ -206,8 +208,9 @@ static int conv_tc_init() {
 // flight; tcgen05 instead where the network asks for it and the shapes allow
 // (on the B200 the mma.sync kernels measured faster at every volume from 9^3
 // to 2 x 65^3, forward and backward)
+static int relu_bwd(fg_unet *u, TView dy, const TView &y, const Vol &V, int C);
 static int conv_fwd(fg_unet *u, const ConvLayer &l, const TView &in, const Vol &V, const __nv_bfloat16 *w,
-                    int cin, int cout, int kp, const float *bias, TView out, int relu) {
+                    int cin, int cout, int kp, const float *bias, TView out, int relu, const TView &mask = TView{}) {
     (void)l;
     if (conv_tc_ok(u, in, out, cin, cout, kp)) {
         const int cinp = (cin + 15) / 16 * 16;
@@ -218,12 +221,12 @@ static int conv_fwd(fg_unet *u, const ConvLayer &l, const TView &in, const Vol &
         default: conv_tc_launch<64>(u, in, V, w, cin, cinp, kp, cout, bias, out, relu); break;
         }
         CK(cudaGetLastError());
-        return FG_OK;
+        return mask.p ? relu_bwd(u, out, mask, V, cout) : FG_OK;
     }
     const int64_t tiles = (V.nvox() + 15) / 16;
-    if (tiles >= 148 * 32) return conv_fwd_ks<1>(u, in, V, w, cin, cout, kp, bias, out, relu);
-    if (tiles >= 148 * 16) return conv_fwd_ks<2>(u, in, V, w, cin, cout, kp, bias, out, relu);
-    return conv_fwd_ks<4>(u, in, V, w, cin, cout, kp, bias, out, relu);
+    if (tiles >= 148 * 32) return conv_fwd_ks<1>(u, in, V, w, cin, cout, kp, bias, out, relu, mask);
+    if (tiles >= 148 * 16) return conv_fwd_ks<2>(u, in, V, w, cin, cout, kp, bias, out, relu, mask);
+    return conv_fwd_ks<4>(u, in, V, w, cin, cout, kp, bias, out, relu, mask);
 }
 
 static int layer_fwd(fg_unet *u, int li, const TView &in, const Vol &V, TView out, int relu) {
@@ -233,34 +236,34 @@ static int layer_fwd(fg_unet *u, int li, const TView &in, const Vol &V, TView ou
 
 static void grid_launch(int64_t n, int &blocks) { blocks = (int)std::min<int64_t>((n + 255) / 256, 148 * 16); }
 
-static bool vec8(const TView &a, const TView &b, int C) {
+static bool vec8(const TView &a, const TView &b, int C) {  // a mask has the layout of an activation: C0, C1 or C2 channels
     return C % 8 == 0 && a.cs % 8 == 0 && a.co % 8 == 0 && b.cs % 8 == 0 && b.co % 8 == 0;
 }
 
 // channel-wise trilinear prolongation Vc -> Vf (out = scale P in (+ out))
 static void launch_prolong(fg_unet *u, const TView &in, const Vol &Vc, TView out, const Vol &Vf, int C,
-                           float scale, int accumulate) {
+                           float scale, int accumulate, const TView &mask = TView{}) {
     int blocks;
     if (vec8(in, out, C)) {
         grid_launch(Vf.nvox() * (C / 8), blocks);
-        prolong_kernel<8><<<blocks, 256, 0, u->stream>>>(in, Vc, out, Vf, C, scale, accumulate);
+        prolong_kernel<8><<<blocks, 256, 0, u->stream>>>(in, Vc, out, Vf, C, scale, accumulate, mask);
     } else {
         grid_launch(Vf.nvox() * (C / 2), blocks);
-        prolong_kernel<2><<<blocks, 256, 0, u->stream>>>(in, Vc, out, Vf, C, scale, accumulate);
+        prolong_kernel<2><<<blocks, 256, 0, u->stream>>>(in, Vc, out, Vf, C, scale, accumulate, mask);
     }
 }
 
 // channel-wise full-weighting restriction Vf -> Vc (out = scale R in)
 static void launch_restrict(fg_unet *u, const TView &in, const Vol &Vf, TView out, const Vol &Vc, int C,
-                            float scale) {
+                            float scale, const TView &mask = TView{}) {
     int blocks;
     // 8 channels per thread only when that still gives a few threads per SM lane
     if (vec8(in, out, C) && Vc.nvox() * (C / 8) >= 148 * 512) {
         grid_launch(Vc.nvox() * (C / 8), blocks);
-        restrict_kernel<8><<<blocks, 256, 0, u->stream>>>(in, Vf, out, Vc, C, scale);
+        restrict_kernel<8><<<blocks, 256, 0, u->stream>>>(in, Vf, out, Vc, C, scale, mask);
     } else {
         grid_launch(Vc.nvox() * (C / 2), blocks);
-        restrict_kernel<2><<<blocks, 256, 0, u->stream>>>(in, Vf, out, Vc, C, scale);
+        restrict_kernel<2><<<blocks, 256, 0, u->stream>>>(in, Vf, out, Vc, C, scale, mask);
     }
 }
 
@@ -285,17 +288,35 @@ static int unet_forward(fg_unet *u) {
     return FG_OK;
 }
 
-// input gradient of one layer: the convolution of dy with the flipped weights
-static int layer_dgrad(fg_unet *u, int li, const Vol &V, const TView &dy, const TView &din) {
-    ConvLayer &l = u->L[li];
-    const size_t nf = (size_t)l.cin * l.kpt;
-    if (nf > u->wflip_n) {
-        if (u->wflip) cudaFree(u->wflip);
-        CK(cudaMalloc(&u->wflip, nf * sizeof(__nv_bfloat16)));
-        u->wflip_n = nf;
+// flipped weights of all layers but the first, for their input gradients
+static int unet_flip(fg_unet *u) {
+    size_t off[NLAYERS] = {}, n = 0;
+    for (int l = 1; l < NLAYERS; ++l) {
+        off[l] = n;
+        n += ((size_t)u->L[l].cin * u->L[l].kpt + 127) / 128 * 128;
     }
-    flip_weights_kernel<<<64, 256, 0, u->stream>>>(l.wb, l.cout, l.cin, l.kp, u->wflip, l.kpt);
-    return conv_fwd(u, l, dy, V, u->wflip, l.cout, l.cin, l.kpt, nullptr, din, 0);
+    if (n > u->wflip_n) {
+        if (u->wflip) cudaFree(u->wflip);
+        u->wflip = nullptr;
+        u->wflip_n = 0;
+        CK(cudaMalloc(&u->wflip, n * sizeof(__nv_bfloat16)));
+        u->wflip_n = n;
+    }
+    FlipArgs A{};
+    for (int l = 1; l < NLAYERS; ++l) {
+        u->L[l].wt = u->wflip + off[l];
+        A.L[l - 1] = {u->L[l].wb, u->L[l].wt, u->L[l].cout, u->L[l].cin, u->L[l].kp, u->L[l].kpt};
+    }
+    flip_weights_kernel<<<dim3(32, NLAYERS - 1), 256, 0, u->stream>>>(A);
+    CK(cudaGetLastError());
+    return FG_OK;
+}
+
+// input gradient of one layer: the convolution of dy with the flipped weights,
+// zero where the activation `mask` is not positive (ReLU backward; none if null)
+static int layer_dgrad(fg_unet *u, int li, const Vol &V, const TView &dy, const TView &din, const TView &mask) {
+    ConvLayer &l = u->L[li];
+    return conv_fwd(u, l, dy, V, l.wt, l.cout, l.cin, l.kpt, nullptr, din, 0, mask);
 }
 
 // Weight and bias gradients of all layers (one launch and its reduction), after
@@ -384,29 +405,25 @@ static int unet_backward(fg_unet *u) {
         dh0{b.dcat0, C1 + C0, C1}, dg1{b.dg1, C1, 0}, dcat1{b.dcat1, C2 + C1, 0}, dup1{b.dcat1, C2 + C1, 0},
         dh1{b.dcat1, C2 + C1, C2}, dh2{b.dh2, C2, 0}, da2{b.da2, C2, 0}, dx2{b.dx2, C1, 0},
         da1{b.da1, C1, 0}, dx1{b.dx1, C0, 0}, da0{b.da0, C0, 0};
-    if ((rc = layer_dgrad(u, LOUT, b.v0, dout, dg0))) return rc;
-    if ((rc = relu_bwd(u, dg0, g0, b.v0, C0))) return rc;
-    if ((rc = layer_dgrad(u, L0C, b.v0, dg0, dcat0))) return rc;
+    const TView none{};
+    if ((rc = unet_flip(u))) return rc;
+    if ((rc = layer_dgrad(u, LOUT, b.v0, dout, dg0, g0))) return rc;
+    if ((rc = layer_dgrad(u, L0C, b.v0, dg0, dcat0, none))) return rc;
     // P^T = 8 R : gradient of the level-1 output g1 from the prolongated channels
-    launch_restrict(u, dup0, b.v0, dg1, b.v1, C1, 8.f);
-    if ((rc = relu_bwd(u, dg1, g1, b.v1, C1))) return rc;
-    if ((rc = layer_dgrad(u, L1C, b.v1, dg1, dcat1))) return rc;
-    launch_restrict(u, dup1, b.v1, dh2, b.v2, C2, 8.f);
-    if ((rc = relu_bwd(u, dh2, h2, b.v2, C2))) return rc;
-    if ((rc = layer_dgrad(u, L2B, b.v2, dh2, da2))) return rc;
-    if ((rc = relu_bwd(u, da2, a2, b.v2, C2))) return rc;
-    if ((rc = layer_dgrad(u, L2A, b.v2, da2, dx2))) return rc;
+    launch_restrict(u, dup0, b.v0, dg1, b.v1, C1, 8.f, g1);
+    if ((rc = layer_dgrad(u, L1C, b.v1, dg1, dcat1, none))) return rc;
+    launch_restrict(u, dup1, b.v1, dh2, b.v2, C2, 8.f, h2);
+    if ((rc = layer_dgrad(u, L2B, b.v2, dh2, da2, a2))) return rc;
+    if ((rc = layer_dgrad(u, L2A, b.v2, da2, dx2, none))) return rc;
     // R^T = P / 8 : add the down-path gradient to the skip gradient of h1
-    launch_prolong(u, dx2, b.v2, dh1, b.v1, C1, 0.125f, 1);
-    if ((rc = relu_bwd(u, dh1, h1, b.v1, C1))) return rc;
-    if ((rc = layer_dgrad(u, L1B, b.v1, dh1, da1))) return rc;
-    if ((rc = relu_bwd(u, da1, a1, b.v1, C1))) return rc;
-    if ((rc = layer_dgrad(u, L1A, b.v1, da1, dx1))) return rc;
-    launch_prolong(u, dx1, b.v1, dh0, b.v0, C0, 0.125f, 1);
-    if ((rc = relu_bwd(u, dh0, h0, b.v0, C0))) return rc;
-    if ((rc = layer_dgrad(u, L0B, b.v0, dh0, da0))) return rc;
-    if ((rc = relu_bwd(u, da0, a0, b.v0, C0))) return rc;
-    const WgItem items[] = {{LOUT, g0, dout, b.v0}, {L0C, cat0, dg0, b.v0}, {L1C, cat1, dg1, b.v1}, {L2B, a2, dh2, b.v2}, {L2A, x2, da2, b.v2}, {L1B, a1, dh1, b.v1}, {L1A, x1, da1, b.v1}, {L0B, a0, dh0, b.v0}, {L0A, x0, da0, b.v0}};
+    launch_prolong(u, dx2, b.v2, dh1, b.v1, C1, 0.125f, 1, h1);
+    if ((rc = layer_dgrad(u, L1B, b.v1, dh1, da1, a1))) return rc;
+    if ((rc = layer_dgrad(u, L1A, b.v1, da1, dx1, none))) return rc;
+    launch_prolong(u, dx1, b.v1, dh0, b.v0, C0, 0.125f, 1, h0);
+    if ((rc = layer_dgrad(u, L0B, b.v0, dh0, da0, a0))) return rc;
+    const WgItem items[] = {{LOUT, g0, dout, b.v0}, {L0C, cat0, dg0, b.v0}, {L1C, cat1, dg1, b.v1},
+                            {L2B, a2, dh2, b.v2},   {L2A, x2, da2, b.v2},   {L1B, a1, dh1, b.v1},
+                            {L1A, x1, da1, b.v1},   {L0B, a0, dh0, b.v0},   {L0A, x0, da0, b.v0}};
     if ((rc = unet_wgrad(u, items, NLAYERS))) return rc;
     CK(cudaGetLastError());
     return FG_OK;

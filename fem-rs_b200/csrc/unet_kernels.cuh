@@ -83,6 +83,18 @@ __device__ __forceinline__ uint32_t gather_pair(const TView &in, const Vol &V, c
     return ld_bf16x2(in.p + vv * in.cs + in.co + c.ci);
 }
 
+// Channels n, n+1 of voxel v, zero where mask (an activation of the same channels;
+// mask.p null: none) is not positive -- the ReLU backward of a gradient being stored.
+__device__ __forceinline__ bool mask_pos(__nv_bfloat16 y) { return __bfloat162float(y) > 0.f; }
+__device__ __forceinline__ void st_masked2(const TView &out, int64_t v, int n, float a, float b, const TView &mask) {
+    if (mask.p) {
+        const __nv_bfloat162 y = *reinterpret_cast<const __nv_bfloat162 *>(mask.p + v * mask.cs + mask.co + n);
+        a = mask_pos(y.x) ? a : 0.f;
+        b = mask_pos(y.y) ? b : 0.f;
+    }
+    *reinterpret_cast<__nv_bfloat162 *>(out.p + v * out.cs + out.co + n) = __floats2bfloat162_rn(a, b);
+}
+
 // One tile: 16 voxels x NT*8 output channels, computed by KS warps that split
 // the K loop (KS in {1, 2, 4}; a block of 4 warps holds 4/KS tiles) and sum
 // their accumulators in shared memory in warp order.  Small volumes use KS = 4
@@ -91,8 +103,8 @@ __device__ __forceinline__ uint32_t gather_pair(const TView &in, const Vol &V, c
 template <int NT, int KS>
 __global__ void __launch_bounds__(128) conv3_fwd_kernel(const TView in, const Vol V, int Cin,
                                                         const __nv_bfloat16 *__restrict__ W, int Kp,
-                                                        const float *__restrict__ bias, TView out,
-                                                        int relu) {
+                                                        const float *__restrict__ bias, TView out, int relu,
+                                                        const TView mask) {
     constexpr int TPB = 4 / KS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = warp / KS, part = warp % KS;
@@ -153,10 +165,8 @@ __global__ void __launch_bounds__(128) conv3_fwd_kernel(const TView in, const Vo
         if (relu) {
             r0 = fmaxf(r0, 0.f); r1 = fmaxf(r1, 0.f); r2 = fmaxf(r2, 0.f); r3 = fmaxf(r3, 0.f);
         }
-        if (ok0)
-            *reinterpret_cast<__nv_bfloat162 *>(out.p + v0 * out.cs + out.co + n) = __floats2bfloat162_rn(r0, r1);
-        if (ok1)
-            *reinterpret_cast<__nv_bfloat162 *>(out.p + v1 * out.cs + out.co + n) = __floats2bfloat162_rn(r2, r3);
+        if (ok0) st_masked2(out, v0, n, r0, r1, mask);
+        if (ok1) st_masked2(out, v1, n, r2, r3, mask);
     }
 }
 
@@ -174,8 +184,8 @@ __device__ __forceinline__ uint2 ld_bf16x4(const __nv_bfloat16 *p) {
 template <int NT, int KS>
 __global__ void __launch_bounds__(128) conv3_fwd16_kernel(const TView in, const Vol V, int Cin,
                                                           const __nv_bfloat16 *__restrict__ W, int Kp,
-                                                          const float *__restrict__ bias, TView out,
-                                                          int relu) {
+                                                          const float *__restrict__ bias, TView out, int relu,
+                                                          const TView mask) {
     constexpr int TPB = 4 / KS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = warp / KS, part = warp % KS;
@@ -193,31 +203,50 @@ __global__ void __launch_bounds__(128) conv3_fwd16_kernel(const TView in, const 
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
     if (active) {
         const __nv_bfloat16 *wl = W + (int64_t)gid * Kp + 4 * t4;
-        for (int tap = part; tap < 27; tap += KS) {
-            const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-            const __nv_bfloat16 *p0 = nullptr, *p1 = nullptr;
-            {
-                const int zz = z0 + dz, yy = y0 + dy, xx = x0 + dx;
-                if (ok0 && zz >= 0 && zz < V.Z && yy >= 0 && yy < V.Y && xx >= 0 && xx < V.X)
-                    p0 = in.p + ((((int64_t)b0 * V.Z + zz) * V.Y + yy) * V.X + xx) * in.cs + in.co + 4 * t4;
-            }
-            {
-                const int zz = z1 + dz, yy = y1 + dy, xx = x1 + dx;
-                if (ok1 && zz >= 0 && zz < V.Z && yy >= 0 && yy < V.Y && xx >= 0 && xx < V.X)
-                    p1 = in.p + ((((int64_t)b1 * V.Z + zz) * V.Y + yy) * V.X + xx) * in.cs + in.co + 4 * t4;
-            }
-            const __nv_bfloat16 *wt = wl + tap * Cin;
-#pragma unroll 2
-            for (int c0 = 0; c0 < Cin; c0 += 16) {
-                const uint2 a0 = p0 ? ld_bf16x4(p0 + c0) : make_uint2(0u, 0u);
-                const uint2 a1 = p1 ? ld_bf16x4(p1 + c0) : make_uint2(0u, 0u);
-                const uint32_t a[4] = {a0.x, a1.x, a0.y, a1.y};
+        // four steps of 16 channels at a time (taps in order, channel blocks in order), all
+        // their voxel loads issued before the first product: with one tap's loads in
+        // flight at a time a warp spent its time on seven L2 latencies; the products and
+        // their order are unchanged, so are the bits
+        int tap = part, c0 = 0;
+        while (tap < 27) {
+            uint2 a0[4], a1[4];
+            int wo[4];
 #pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    const uint2 bw = ld_bf16x4(wt + (int64_t)j * 8 * Kp + c0);
-                    mma_bf16_16816(acc[j], a, bw.x, bw.y);
+            for (int g = 0; g < 4; ++g) {
+                a0[g] = a1[g] = make_uint2(0u, 0u);
+                wo[g] = -1;
+                if (tap < 27) {
+                    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+                    {
+                        const int zz = z0 + dz, yy = y0 + dy, xx = x0 + dx;
+                        if (ok0 && zz >= 0 && zz < V.Z && yy >= 0 && yy < V.Y && xx >= 0 && xx < V.X)
+                            a0[g] = ld_bf16x4(in.p + ((((int64_t)b0 * V.Z + zz) * V.Y + yy) * V.X + xx) * in.cs + in.co +
+                                              4 * t4 + c0);
+                    }
+                    {
+                        const int zz = z1 + dz, yy = y1 + dy, xx = x1 + dx;
+                        if (ok1 && zz >= 0 && zz < V.Z && yy >= 0 && yy < V.Y && xx >= 0 && xx < V.X)
+                            a1[g] = ld_bf16x4(in.p + ((((int64_t)b1 * V.Z + zz) * V.Y + yy) * V.X + xx) * in.cs + in.co +
+                                              4 * t4 + c0);
+                    }
+                    wo[g] = tap * Cin + c0;
+                    c0 += 16;
+                    if (c0 == Cin) {
+                        c0 = 0;
+                        tap += KS;
+                    }
                 }
             }
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                if (wo[g] >= 0) {
+                    const uint32_t a[4] = {a0[g].x, a1[g].x, a0[g].y, a1[g].y};
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) {
+                        const uint2 bw = ld_bf16x4(wl + (int64_t)j * 8 * Kp + wo[g]);
+                        mma_bf16_16816(acc[j], a, bw.x, bw.y);
+                    }
+                }
         }
     }
     if constexpr (KS > 1) {
@@ -247,29 +276,31 @@ __global__ void __launch_bounds__(128) conv3_fwd16_kernel(const TView in, const 
         if (relu) {
             r0 = fmaxf(r0, 0.f); r1 = fmaxf(r1, 0.f); r2 = fmaxf(r2, 0.f); r3 = fmaxf(r3, 0.f);
         }
-        if (ok0)
-            *reinterpret_cast<__nv_bfloat162 *>(out.p + v0 * out.cs + out.co + n) = __floats2bfloat162_rn(r0, r1);
-        if (ok1)
-            *reinterpret_cast<__nv_bfloat162 *>(out.p + v1 * out.cs + out.co + n) = __floats2bfloat162_rn(r2, r3);
+        if (ok0) st_masked2(out, v0, n, r0, r1, mask);
+        if (ok1) st_masked2(out, v1, n, r2, r3, mask);
     }
 }
 
-// W'[ci][tap][co] = W[co][26 - tap][ci]  (input-gradient weights), padded rows
-__global__ void flip_weights_kernel(const __nv_bfloat16 *__restrict__ W, int Cout, int Cin, int Kp,
-                                    __nv_bfloat16 *__restrict__ Wt, int Kpt) {
-    const int total = Cin * Kpt;
+// W'[ci][tap][co] = W[co][26 - tap][ci] (input-gradient weights, padded rows) of
+// every layer with an input gradient, in one launch: blockIdx.y = layer.
+struct FlipArgs {
+    struct { const __nv_bfloat16 *W; __nv_bfloat16 *Wt; int Cout, Cin, Kp, Kpt; } L[9];
+};
+__global__ void flip_weights_kernel(const __grid_constant__ FlipArgs A) {
+    const auto &L = A.L[blockIdx.y];
+    const int total = L.Cin * L.Kpt;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int ci = i / Kpt, k = i % Kpt;
+        const int ci = i / L.Kpt, k = i % L.Kpt;
         __nv_bfloat16 v = __float2bfloat16(0.f);
-        if (k < 27 * Cout) {
-            const int tap = k / Cout, co = k % Cout;
-            v = W[(int64_t)co * Kp + (26 - tap) * Cin + ci];
+        if (k < 27 * L.Cout) {
+            const int tap = k / L.Cout, co = k % L.Cout;
+            v = L.W[(int64_t)co * L.Kp + (26 - tap) * L.Cin + ci];
         }
-        Wt[i] = v;
+        L.Wt[i] = v;
     }
 }
 
-// dy *= (y > 0)   (ReLU backward through the stored activation)
+// dy *= (y > 0)   (ReLU backward through the stored activation; the tcgen05 path)
 __global__ void relu_bwd_kernel(TView dy, const TView y, int64_t nv, int C) {
     const int64_t total = nv * C;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -317,7 +348,7 @@ template <> struct BVec<8> {
 // stride and offset multiples of VW)
 template <int VW>
 __global__ void prolong_kernel(const TView in, const Vol Vc, TView out, const Vol Vf, int C, float scale,
-                               int accumulate) {
+                               int accumulate, const TView mask) {
     const int G = C / VW;
     const int64_t total = Vf.nvox() * G;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -344,13 +375,20 @@ __global__ void prolong_kernel(const TView in, const Vol Vc, TView out, const Vo
         if (accumulate) BVec<VW>::ld(o, prev);
 #pragma unroll
         for (int k = 0; k < VW; ++k) s[k] = scale * s[k] + (accumulate ? prev[k] : 0.f);
+        if (mask.p) {
+            float m[VW];
+            BVec<VW>::ld(mask.p + v * mask.cs + mask.co + c, m);
+#pragma unroll
+            for (int k = 0; k < VW; ++k) s[k] = m[k] > 0.f ? s[k] : 0.f;
+        }
         BVec<VW>::st(o, s);
     }
 }
 
 // full-weighting restriction of C channels, VW channels per thread
 template <int VW>
-__global__ void restrict_kernel(const TView in, const Vol Vf, TView out, const Vol Vc, int C, float scale) {
+__global__ void restrict_kernel(const TView in, const Vol Vf, TView out, const Vol Vc, int C, float scale,
+                                const TView mask) {
     const int G = C / VW;
     const int64_t total = Vc.nvox() * G;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -378,6 +416,12 @@ __global__ void restrict_kernel(const TView in, const Vol Vf, TView out, const V
                 }
 #pragma unroll
         for (int k = 0; k < VW; ++k) s[k] *= scale;
+        if (mask.p) {
+            float m[VW];
+            BVec<VW>::ld(mask.p + v * mask.cs + mask.co + c, m);
+#pragma unroll
+            for (int k = 0; k < VW; ++k) s[k] = m[k] > 0.f ? s[k] : 0.f;
+        }
         BVec<VW>::st(out.p + v * out.cs + out.co + c, s);
     }
 }
@@ -414,6 +458,29 @@ __global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ g, 
         const float wi = w[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
         w[i] = wi;
         if (wb) wb[i] = __float2bfloat16(wi);
+    }
+}
+
+// All layers' parameters (or gradients) between their padded device arrays and one
+// flat array [per layer: W [cout][K], b [cout]]; unpacking refreshes the BF16 copies.
+struct PackArgs {
+    struct { float *w, *b; __nv_bfloat16 *wb; int cout, K, kp, off; } L[9];
+    int n, total;
+};
+__global__ void pack_params_kernel(const __grid_constant__ PackArgs A, float *__restrict__ flat, int unpack) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.total; i += gridDim.x * blockDim.x) {
+        int l = 0;
+        while (l + 1 < A.n && i >= A.L[l + 1].off) ++l;
+        const auto &L = A.L[l];
+        const int r = i - L.off, nw = L.cout * L.K;
+        const int64_t at = r < nw ? (int64_t)(r / L.K) * L.kp + r % L.K : 0;
+        float *p = r < nw ? L.w + at : L.b + (r - nw);
+        if (unpack) {
+            *p = flat[i];
+            if (r < nw) L.wb[at] = __float2bfloat16(flat[i]);
+        } else {
+            flat[i] = *p;
+        }
     }
 }
 
