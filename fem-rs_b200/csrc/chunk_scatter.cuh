@@ -73,14 +73,21 @@ __device__ __forceinline__ ChunkStage chunk_stage_lists(const ChunkLists &L, int
 __device__ __forceinline__ void chunk_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Block-wide: the chunk's values of x into xu (the caller places the barrier).
+// Eight DOFs of a thread at a time, so a chunk waits for its list and for x once
+// or twice instead of once per DOF of a thread.
 template <typename T, int BT>
 __device__ __forceinline__ void chunk_load_x(const ChunkLists &L, int c, const T *__restrict__ x, T *xu, int constrained) {
     const int u0 = __ldg(L.cu_off + c), nu = __ldg(L.cu_n + c);
-#pragma unroll 4
-    for (int k = threadIdx.x; k < nu; k += BT) {
-        const int32_t d = __ldg(L.cu_dof + u0 + k);
-        const T v = __ldg(x + (d & INT32_MAX));
-        xu[k] = constrained && d < 0 ? T(0) : v;
+    for (int k0 = threadIdx.x; k0 < nu; k0 += 8 * BT) {
+        int32_t d[8];
+        T v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) d[u] = k0 + u * BT < nu ? __ldg(L.cu_dof + u0 + k0 + u * BT) : 0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = k0 + u * BT < nu ? __ldg(x + (d[u] & INT32_MAX)) : T(0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (k0 + u * BT < nu) xu[k0 + u * BT] = constrained && d[u] < 0 ? T(0) : v[u];
     }
 }
 

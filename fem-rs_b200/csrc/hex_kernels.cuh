@@ -30,7 +30,7 @@
 //
 // What bounds it: the latency of one chunk's phases (gather, columns, sums) with
 // three CTAs per SM.  64^3 Q2 FP64, apply and shared DOFs: 159 us with a
-// 32-bit map and per-element x loads, 143 us as above.
+// 32-bit map and per-element x loads, 135 us as above (dependent launches included).
 //
 // Element math: slab sum factorisation (one qy slab of QH quadrature columns
 // at a time: y then x contraction of the element values, per column z, D, z^T,
