@@ -1446,11 +1446,16 @@ template <typename T> static int launch_pcg_fused(fg_op *op, const PcgBufs<T> &B
     if (!op->fused_pcg) return FG_OK;
     static int fits[64];  // per device: 1 fits, -1 does not, 0 not yet known
     if (op->device < 0 || op->device >= 64) return FG_OK;
-    auto kern = k_pcg_fused_jacobi<T>;
+    const unsigned grid = vec_grid(op->Nn);
+    // one block per SM: every vector is read once (ONE), whatever registers that takes
+    auto kern = grid <= 148u ? k_pcg_fused_jacobi<T, true> : k_pcg_fused_jacobi<T, false>;
     if (!fits[op->device]) {
         int per_sm = 0, sms = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, VEC_THREADS, 0));
+        int one = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_fused_jacobi<T, false>, VEC_THREADS, 0));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_pcg_fused_jacobi<T, true>, VEC_THREADS, 0));
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, op->device));
+        if (one < 1 || sms < 148) per_sm = 0;
         fits[op->device] = per_sm * sms >= VEC_GRID ? 1 : -1;
     }
     if (fits[op->device] < 0) return FG_OK;
@@ -1460,7 +1465,7 @@ template <typename T> static int launch_pcg_fused(fg_op *op, const PcgBufs<T> &B
         FG_LEGACY_FENCE();
     }
     cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(vec_grid(op->Nn));
+    lc.gridDim = dim3(grid);
     lc.blockDim = dim3(VEC_THREADS);
     lc.stream = op->stream;
     cudaLaunchAttribute at[1];

@@ -207,7 +207,7 @@ __device__ __forceinline__ void grid_barrier(unsigned *bar, int *err, bool &ok,
                     ok_s = 0;
                     break;
                 }
-                __nanosleep(64);
+                if (gridDim.x > 148) __nanosleep(64);  // few blocks: poll without a pause
             }
         }
         __threadfence();

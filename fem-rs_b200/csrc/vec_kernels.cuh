@@ -287,8 +287,13 @@ __device__ __forceinline__ void all_blocks_sum(double (&v)[NV], double *partials
 // 296-330) and of solve_cg_operator (dinv = 1, its own stopping rule).  The
 // state is read by every block at entry and written by block 0 only; the two
 // reductions use separate partial regions.  Same values as the separate kernels.
-template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_pcg_fused_jacobi(int64_t n, T *__restrict__ x, T *__restrict__ r,
+// ONE: the grid has a thread for every group of four (vec_grid below VEC_GRID).
+// All vectors are then read once, before the first barrier, and z stays in
+// registers, so an iteration waits for memory once instead of four times; the
+// kernel of a 24^3 Q1 solve is nothing but such waits and the two barriers.
+// Otherwise VEC_GRID blocks have to be resident, four per SM.
+template <typename T, bool ONE>
+__global__ void __launch_bounds__(VEC_THREADS, ONE ? 1 : 4) k_pcg_fused_jacobi(int64_t n, T *__restrict__ x, T *__restrict__ r,
                                                                   T *__restrict__ p, const T *__restrict__ ap,
                                                                   const T *__restrict__ dinv, T *__restrict__ z,
                                                                   double *partials, SolverState *st, unsigned *bar,
@@ -299,7 +304,18 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_fused_jacobi(int64_t n, T *
     const int iter0 = st->iter, max_iter = st->max_iter, cgop = st->cgop;
     bool ok = true;
     double v1[1] = {0.0};
-    FG_VEC4_LOOP(q, n) {
+    const int64_t q1 = (int64_t)blockIdx.x * VEC_THREADS + threadIdx.x;  // ONE: this thread's group
+    const bool have = q1 < (n >> 2);
+    V4<T> xo, ro, po, ao, dvo, zo;
+    if (ONE && have) {
+        po = ld4(p, q1);
+        ao = ld4(ap, q1);
+        xo = ld4(x, q1);
+        ro = ld4(r, q1);
+        dvo = ld4(dinv, q1);
+        FG_K4 v1[0] = fma((double)po.a[k], (double)ao.a[k], v1[0]);
+    }
+    if (!ONE) FG_VEC4_LOOP(q, n) {
         const V4<T> pv = ld4(p, q), av = ld4(ap, q);
         FG_K4 v1[0] = fma((double)pv.a[k], (double)av.a[k], v1[0]);
     }
@@ -316,7 +332,19 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_fused_jacobi(int64_t n, T *
     const double alpha_d = rz0 / pap[0];
     const T alpha = (T)alpha_d;
     double v2[2] = {0.0, 0.0};
-    FG_VEC4_LOOP(q, n) {
+    if (ONE && have) {
+        FG_K4 {
+            xo.a[k] += alpha * po.a[k];
+            ro.a[k] = ro.a[k] - alpha * ao.a[k];
+            v2[0] = fma((double)ro.a[k], (double)ro.a[k], v2[0]);
+            zo.a[k] = dvo.a[k] * ro.a[k];
+            v2[1] = fma((double)ro.a[k], (double)zo.a[k], v2[1]);
+        }
+        st4(x, q1, xo);
+        st4(r, q1, ro);
+        st4(z, q1, zo);
+    }
+    if (!ONE) FG_VEC4_LOOP(q, n) {
         V4<T> xv = ld4(x, q), rv = ld4(r, q), zv;
         const V4<T> pv = ld4(p, q), av = ld4(ap, q), dv = ld4(dinv, q);
         FG_K4 {
@@ -355,7 +383,11 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_fused_jacobi(int64_t n, T *
     }
     if (stop) return;
     const T beta = (T)beta_d;
-    FG_VEC4_LOOP(q, n) {
+    if (ONE && have) {
+        FG_K4 po.a[k] = zo.a[k] + beta * po.a[k];
+        st4(p, q1, po);
+    }
+    if (!ONE) FG_VEC4_LOOP(q, n) {
         const V4<T> zv = ld4(z, q);
         V4<T> pv = ld4(p, q);
         FG_K4 pv.a[k] = zv.a[k] + beta * pv.a[k];
