@@ -213,6 +213,11 @@ static int ensure_tables(int dev) {
             }
     }
     CK(cudaMemcpyToSymbol(c_DQ32, DQ, sizeof DQ));
+    float2 DD[FG_MAXP][FG_MAXP + 1][FG_MAXP + 1] = {};
+    for (int p = 0; p < FG_MAXP; ++p)
+        for (int q = 0; q <= FG_MAXP; ++q)
+            for (int k = 0; k <= FG_MAXP; ++k) DD[p][q][k] = make_float2(DQ[p][q][k], DQ[p][q][k]);
+    CK(cudaMemcpyToSymbol(c_DD32, DD, sizeof DD));
     CK(cudaMemcpyToSymbol(c_DQ64, DQd, sizeof DQd));
     g_tables_ready[dev] = true;
     return FG_OK;

@@ -39,6 +39,7 @@ __constant__ float2 c_BB32[FG_MAXP][FG_MAXP + 1][FG_MAXP + 1];
 // collocated derivative at the Gauss points, Dq = G B^-1: the derivative at
 // point q of the degree-p polynomial through the values at the p+1 points
 __constant__ float c_DQ32[FG_MAXP][FG_MAXP + 1][FG_MAXP + 1];
+__constant__ float2 c_DD32[FG_MAXP][FG_MAXP + 1][FG_MAXP + 1];  // (Dq, Dq) for packed FMAs
 __constant__ double c_DQ64[FG_MAXP][FG_MAXP + 1][FG_MAXP + 1];
 
 template <typename T> struct Tab;
