@@ -210,9 +210,13 @@ __device__ __forceinline__ void merge_and_store(T (&out)[P + 1][P + 1][P + 1], c
     const int I0 = tx * LX * P, J0 = ty * (WY * LY) * P, K0 = tz * g.TZ * P;
     const int ex = tx * LX + lx, ey = ty * (WY * LY) + row, ez = tz * g.TZ + lz;
     const int SX = LX * P + 1, SY = WY * LY * P + 1;
-    T *fxp = face + (int64_t)item * g.face_stride();
-    T *fyp = fxp + g.fx();
-    T *fzp = fyp + g.fy();
+    // g.fx(), fy(), fz() with the item's compile-time lanes and rows: from the grid's
+    // fields the sizes took registers that the Q3 FP64 forms spill for (1,330 against
+    // 1,154 bytes of stores in the affine one).
+    const int SZ = g.TZ * P + 1;
+    T *fxp = face + (int64_t)item * (SZ * (SX + SY) + SX * SY);
+    T *fyp = fxp + SZ * SY;
+    T *fzp = fyp + SZ * SX;
     const bool last_layer = (lz == nl - 1);
 #pragma unroll
     for (int c = 0; c < D; ++c) {
