@@ -471,9 +471,11 @@ static int launch_apply_t(fg_op *op, const Grid &g, const T *qd, T *face, const 
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) return fail(FG_CUDA_ERROR, "cuTensorMapEncodeTiled failed (%d)", (int)cr);
-    ApplyArgs<T> A{g, qd, y, face, accumulate, op->d_err, skip, fixcnt, op->wait_ns, item0, skip ? 0 : 1};
     const unsigned grid = (unsigned)(nitems < 0 ? g.n_items() : nitems);
-    CK(launch_dep(grid <= DEP_MAX_CTAS, kern, dim3(grid), C::WY * 32, SM::bytes, op->stream, tmap, A));
+    const bool dep = grid <= DEP_MAX_CTAS;
+    // in an ordinary launch the x tile, which the first layer waits for, goes first
+    ApplyArgs<T> A{g, qd, y, face, accumulate, op->d_err, skip, fixcnt, op->wait_ns, item0, dep && !skip ? 1 : 0};
+    CK(launch_dep(dep, kern, dim3(grid), C::WY * 32, SM::bytes, op->stream, tmap, A));
     return FG_OK;
 }
 
@@ -651,7 +653,7 @@ static void set_scratch_tiling(Grid &g) {
 // its SM or has it to itself (45 x 41 x 38 Q3 FP32 affine: 7.5 us a layer with one to four
 // CTAs per SM), so the time is the number of rounds of resident CTAs times the
 // layers of one, plus what a CTA spends before its first layer's data arrive
-// (about 0.8 layer).  Rounds count whole up to four (the last one leaves SMs
+// (about 0.8 layer).  Rounds count whole up to three (the last one leaves SMs
 // idle), above that half a round is lost on average; a small term counts the
 // warps that work at all, which separates the lane shapes when the rounds do
 // not.  32 lanes in x come first and a later candidate must win by a tenth of a
@@ -689,7 +691,7 @@ static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size
             set_depth(c, tz);
             if (face_limit && (size_t)c.n_items() * (size_t)c.face_stride() > face_limit) continue;
             const double w = c.n_items() / slots;
-            const double cost = shape * ((w >= 4.0 ? w + 0.5 : std::ceil(w)) * (tz + 0.8) + 0.25 * work);
+            const double cost = shape * ((w >= 3.0 ? w + 0.5 : std::ceil(w)) * (tz + 0.8) + 0.25 * work);
             if (cost < best_cost - 0.1) {
                 best_cost = cost;
                 best = c;
