@@ -666,7 +666,7 @@ static void set_scratch_tiling(Grid &g) {
 // affine 45.6 -> 34.8 us, 33x40x37 38.0 -> 24.8, 48x40x44 Q2 FP64 42.9 -> 34.1,
 // 45x41x38 Q3 FP64 121 -> 97, 100x90x80 Q1 FP64 76.9 -> 57.6, 64^3 Q2 FP32 affine
 // mass + diffusion 32.6 -> 30.6.  Over 767 random meshes of 6 to 192 elements a
-// side, all orders, kinds and forms: 2.4 % above the best of 18 shapes on average
+// side, all orders, kinds and forms: 2.6 % above the best of 18 shapes on average
 // (the old rule 13 %), 9 % below the old rule's time, at worst 20 % above it.
 static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size_t face_limit) {
     // CTAs per SM by registers and shared memory, [fp32][affine][order]
