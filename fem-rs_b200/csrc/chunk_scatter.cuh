@@ -74,9 +74,10 @@ __device__ __forceinline__ void chunk_wait() { asm volatile("cp.async.wait_group
 
 // Block-wide: the chunk's values of x into xu (the caller places the barrier).
 // Eight DOFs of a thread at a time, so a chunk waits for its list and for x once
-// or twice instead of once per DOF of a thread.
+// or twice instead of once per DOF of a thread.  x may be written by the kernel ahead
+// of a dependent launch, so it is read by ordinary loads (pdl_wait, fg_common.cuh).
 template <typename T, int BT>
-__device__ __forceinline__ void chunk_load_x(const ChunkLists &L, int c, const T *__restrict__ x, T *xu, int constrained) {
+__device__ __forceinline__ void chunk_load_x(const ChunkLists &L, int c, const T *x, T *xu, int constrained) {
     const int u0 = __ldg(L.cu_off + c), nu = __ldg(L.cu_n + c);
     for (int k0 = threadIdx.x; k0 < nu; k0 += 8 * BT) {
         int32_t d[8];
@@ -84,7 +85,7 @@ __device__ __forceinline__ void chunk_load_x(const ChunkLists &L, int c, const T
 #pragma unroll
         for (int u = 0; u < 8; ++u) d[u] = k0 + u * BT < nu ? __ldg(L.cu_dof + u0 + k0 + u * BT) : 0;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = k0 + u * BT < nu ? __ldg(x + (d[u] & INT32_MAX)) : T(0);
+        for (int u = 0; u < 8; ++u) v[u] = k0 + u * BT < nu ? x[d[u] & INT32_MAX] : T(0);
 #pragma unroll
         for (int u = 0; u < 8; ++u)
             if (k0 + u * BT < nu) xu[k0 + u * BT] = constrained && d[u] < 0 ? T(0) : v[u];
@@ -114,7 +115,7 @@ __device__ __forceinline__ void chunk_sums(const ChunkLists &L, const ChunkStage
 
 // DOFs not owned by a single chunk: the partials of their chunks in chunk order
 template <typename T>
-__global__ void chunk_shared_kernel(const ChunkLists L, const T *__restrict__ x, T *__restrict__ y, int accumulate,
+__global__ void chunk_shared_kernel(const ChunkLists L, const T *x, T *y, int accumulate,
                                     int constrained, int diag, const int *skip) {
     pdl_trigger();
     pdl_wait();

@@ -96,8 +96,15 @@ struct Grid {
 // predecessor in the stream is still running, once every CTA of the predecessor
 // has passed pdl_trigger (or exited).  It may touch nothing that an earlier
 // kernel writes or reads before pdl_wait, which returns when the predecessor has
-// completed -- and, as every kernel so launched waits, all before it.  Both are
-// no-ops in a kernel launched the ordinary way.
+// completed -- and, as every kernel so launched waits, all before it.  In a kernel
+// launched the ordinary way pdl_wait is a no-op, while pdl_trigger still releases a
+// dependent kernel behind it; a kernel that triggers therefore either waits or is
+// launched the ordinary way (then all before it has completed).
+// A kernel that waits is alive while its predecessor writes: data that any kernel
+// of a solve writes is no read-only data of it.  Such pointers are not __restrict__
+// (the compiler may move loads through them above the wait, or make them
+// non-coherent) and are not read by __ldg; matrices' data, lists and tables, which
+// are written before the first launch, may be.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {

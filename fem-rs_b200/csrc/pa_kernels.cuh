@@ -1405,7 +1405,7 @@ template <bool CG, typename T> __device__ __forceinline__ T ld_face(const T *p) 
 // fix-up reads slots other CTAs of the same launch wrote).
 template <typename T, bool CG = false>
 __device__ __forceinline__ T fixup_acc(const Grid &g, int I, int J, int K, int tx, int ty, int tz,
-                                       int sx, int sy, int sz, T own, const T *__restrict__ face) {
+                                       int sx, int sy, int sz, T own, const T *face) {
     const int SXe = g.LX * g.p, SYe = g.WY * g.p, SZe = g.TZ * g.p;
     const int fs = g.face_stride(), fxs = g.fx(), fys = g.fy();
     T sum = own;
@@ -1446,8 +1446,7 @@ __host__ __device__ inline int fixup_rows(const Grid &g) {
 // slower: batched, 16 instances, 46.9 against 44.9 us a launch; 8^3 Q2 apply and
 // fix-up 9.9 against 9.4.
 template <typename T, int P, int LX>
-__device__ __forceinline__ void fixup_row_t(const Grid &g, int r, T *__restrict__ y,
-                                            const T *__restrict__ face) {
+__device__ __forceinline__ void fixup_row_t(const Grid &g, int r, T *y, const T *face) {
     constexpr int SXe = LX * P;
     const int SYe = g.WY * P, SZe = g.TZ * P;
     const int rx = (g.ntx - 1) * g.NK, ry = (g.nty - 1) * g.NK;
@@ -1508,8 +1507,7 @@ __device__ __forceinline__ void fixup_row_t(const Grid &g, int r, T *__restrict_
 }
 
 template <typename T>
-__device__ __forceinline__ void fixup_row(const Grid &g, int r, T *__restrict__ y,
-                                          const T *__restrict__ face) {
+__device__ __forceinline__ void fixup_row(const Grid &g, int r, T *y, const T *face) {
     switch (g.LX + g.p) {
     case 32 + 1: fixup_row_t<T, 1, 32>(g, r, y, face); break;
     case 32 + 2: fixup_row_t<T, 2, 32>(g, r, y, face); break;
@@ -1600,8 +1598,7 @@ __device__ __forceinline__ void fused_fixup(const Grid &g, T *y, const T *face, 
 
 // One block per row of shared-face DOFs (grid = fixup_rows(g)).
 template <typename T>
-__global__ void __launch_bounds__(128) fixup_kernel(const Grid g, T *__restrict__ y,
-                                                    const T *__restrict__ face, const int *skip) {
+__global__ void __launch_bounds__(128) fixup_kernel(const Grid g, T *y, const T *face, const int *skip) {
     pdl_trigger();
     pdl_wait();
     if (skip && *skip) return;

@@ -268,9 +268,8 @@ __host__ __device__ inline size_t tet_chunk_smem(int NL, int CE, int max_nu) {
 // the identity row: y_d (+)= x_d (apply) or 1 (diagonal).  40^3 x 6 P2 tetrahedra:
 // 41.0 us with x gathered per element through a 32-bit map, 30.6 us this way (dependent launches included).
 template <int NL, int BT>
-__global__ void __launch_bounds__(BT, BT == 512 ? 2 : 3) tet_moment_kernel(const TetChunk C, const double *__restrict__ x,
-                                                                         double *__restrict__ y, int accumulate,
-                                                                         int constrained) {
+__global__ void __launch_bounds__(BT, BT == 512 ? 2 : 3) tet_moment_kernel(const TetChunk C, const double *x, double *y,
+                                                                         int accumulate, int constrained) {
     extern __shared__ __align__(16) unsigned char tsm_raw[];
     const int CE = C.CE;
     double *ys = reinterpret_cast<double *>(tsm_raw);  // [NL][CE] element results
@@ -301,8 +300,8 @@ __global__ void __launch_bounds__(BT, BT == 512 ? 2 : 3) tet_moment_kernel(const
 // eight-row tiles that share the table operand) at a time.
 template <int NL, int KIND, int BT>
 __global__ void __launch_bounds__(BT) tet_point_kernel(const TetChunk C, int nq, const double *__restrict__ TF,
-                                                       const double *__restrict__ TB, const double *__restrict__ x,
-                                                       double *__restrict__ y, int accumulate, int constrained) {
+                                                       const double *__restrict__ TB, const double *x, double *y,
+                                                       int accumulate, int constrained) {
     constexpr bool HM = (KIND & 1) != 0, HK = (KIND & 2) != 0;
     constexpr int NC = (HK ? 3 : 0) + (HM ? 1 : 0), KS = TetPoint<NL>::KS, IT = TetPoint<NL>::IT;
     extern __shared__ __align__(16) unsigned char tsm_raw[];

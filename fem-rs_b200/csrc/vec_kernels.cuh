@@ -124,11 +124,11 @@ template <typename T> __device__ __forceinline__ void st4(T *p, int64_t q, const
 
 // r = b - ap; z = dinv r (jacobi) ; p = z ; rz = r.z ; bb = b.b
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_pcg_init(int64_t n, const T *__restrict__ b,
-                                                          const T *__restrict__ ap,
-                                                          const T *__restrict__ dinv,
-                                                          T *__restrict__ r, T *__restrict__ z,
-                                                          T *__restrict__ p, int jacobi,
+__global__ void __launch_bounds__(VEC_THREADS) k_pcg_init(int64_t n, const T *b,
+                                                          const T *ap,
+                                                          const T *dinv,
+                                                          T *r, T *z,
+                                                          T *p, int jacobi,
                                                           double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -177,8 +177,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_init(int64_t n, const T *__
 
 // pap = p.ap ; alpha = rz / pap  (breakdown if |pap| < 1e-30)
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_pcg_pap(int64_t n, const T *__restrict__ p,
-                                                         const T *__restrict__ ap,
+__global__ void __launch_bounds__(VEC_THREADS) k_pcg_pap(int64_t n, const T *p,
+                                                         const T *ap,
                                                          double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -202,12 +202,12 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_pap(int64_t n, const T *__r
 
 // x += alpha p ; r -= alpha ap ; [jacobi: z = dinv r, rz_new] ; rr ; convergence
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_pcg_update(int64_t n, T *__restrict__ x,
-                                                            T *__restrict__ r,
-                                                            const T *__restrict__ p,
-                                                            const T *__restrict__ ap,
-                                                            const T *__restrict__ dinv,
-                                                            T *__restrict__ z, int jacobi,
+__global__ void __launch_bounds__(VEC_THREADS) k_pcg_update(int64_t n, T *x,
+                                                            T *r,
+                                                            const T *p,
+                                                            const T *ap,
+                                                            const T *dinv,
+                                                            T *z, int jacobi,
                                                             double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -397,8 +397,8 @@ __global__ void __launch_bounds__(VEC_THREADS, ONE ? 1 : 4) k_pcg_fused_jacobi(i
 
 // rz_new = r.z ; beta = rz_new / rz ; rz = rz_new   (non-Jacobi preconditioners)
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_pcg_rz(int64_t n, const T *__restrict__ r,
-                                                        const T *__restrict__ z,
+__global__ void __launch_bounds__(VEC_THREADS) k_pcg_rz(int64_t n, const T *r,
+                                                        const T *z,
                                                         double *partials, SolverState *st, int init) {
     pdl_trigger();
     pdl_wait();
@@ -417,8 +417,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_rz(int64_t n, const T *__re
 
 // p = z + beta p   (init: p = z)
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_pcg_pupdate(int64_t n, const T *__restrict__ z,
-                                                             T *__restrict__ p,
+__global__ void __launch_bounds__(VEC_THREADS) k_pcg_pupdate(int64_t n, const T *z,
+                                                             T *p,
                                                              const SolverState *st, int init) {
     pdl_trigger();
     pdl_wait();
@@ -438,11 +438,11 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_pupdate(int64_t n, const T 
 
 // Chebyshev sweep 1 from zero: res = dinv r ; d = res / theta ; z = d
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_cheb_first(int64_t n, const T *__restrict__ r,
-                                                            const T *__restrict__ dinv,
-                                                            T *__restrict__ res,
-                                                            T *__restrict__ d,
-                                                            T *__restrict__ z, double inv_theta,
+__global__ void __launch_bounds__(VEC_THREADS) k_cheb_first(int64_t n, const T *r,
+                                                            const T *dinv,
+                                                            T *res,
+                                                            T *d,
+                                                            T *z, double inv_theta,
                                                             const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -463,11 +463,11 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_first(int64_t n, const T *
 
 // Chebyshev sweep: res -= dinv t ; d = c1 d + c2 res ; z += d
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_cheb_step(int64_t n, const T *__restrict__ t,
-                                                           const T *__restrict__ dinv,
-                                                           T *__restrict__ res,
-                                                           T *__restrict__ d,
-                                                           T *__restrict__ z, double c1,
+__global__ void __launch_bounds__(VEC_THREADS) k_cheb_step(int64_t n, const T *t,
+                                                           const T *dinv,
+                                                           T *res,
+                                                           T *d,
+                                                           T *z, double c1,
                                                            double c2, const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -500,9 +500,9 @@ template <typename T> struct ChebSum {
 
 // sweep 1 from zero: res = dinv r ; d_0 = res / theta
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_cheb_first_d(int64_t n, const T *__restrict__ r,
-                                                              const T *__restrict__ dinv,
-                                                              T *__restrict__ res, T *__restrict__ d,
+__global__ void __launch_bounds__(VEC_THREADS) k_cheb_first_d(int64_t n, const T *r,
+                                                              const T *dinv,
+                                                              T *res, T *d,
                                                               double inv_theta, const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -522,11 +522,11 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_first_d(int64_t n, const T
 
 // middle sweep: res -= dinv t ; d_k = c1 d_{k-1} + c2 res
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_cheb_mid(int64_t n, const T *__restrict__ t,
-                                                          const T *__restrict__ dinv,
-                                                          T *__restrict__ res,
-                                                          const T *__restrict__ dprev,
-                                                          T *__restrict__ dnext, double c1, double c2,
+__global__ void __launch_bounds__(VEC_THREADS) k_cheb_mid(int64_t n, const T *t,
+                                                          const T *dinv,
+                                                          T *res,
+                                                          const T *dprev,
+                                                          T *dnext, double c1, double c2,
                                                           const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -546,11 +546,11 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_mid(int64_t n, const T *__
 
 // last sweep: d_s = c1 d_{s-1} + c2 (res - dinv t) ; z = d_0 + ... + d_{s-1} + d_s
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_cheb_last(int64_t n, const T *__restrict__ t,
-                                                           const T *__restrict__ dinv,
-                                                           const T *__restrict__ res,
-                                                           const T *__restrict__ dprev,
-                                                           const ChebSum<T> earlier, T *__restrict__ z,
+__global__ void __launch_bounds__(VEC_THREADS) k_cheb_last(int64_t n, const T *t,
+                                                           const T *dinv,
+                                                           const T *res,
+                                                           const T *dprev,
+                                                           const ChebSum<T> earlier, T *z,
                                                            double c1, double c2, const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -574,8 +574,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_last(int64_t n, const T *_
 }
 
 // ||b - ap|| / bnorm into st->tmp[0] (true residual)
-__global__ void __launch_bounds__(VEC_THREADS) k_true_residual(int64_t n, const double *__restrict__ b,
-                                                               const double *__restrict__ ap,
+__global__ void __launch_bounds__(VEC_THREADS) k_true_residual(int64_t n, const double *b,
+                                                               const double *ap,
                                                                double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -602,7 +602,7 @@ __device__ __forceinline__ double hash_unit(uint64_t i) {
     return (double)(z >> 11) * (2.0 / 9007199254740992.0) - 1.0;
 }
 
-__global__ void __launch_bounds__(VEC_THREADS) k_hash_vector(const Grid g, double *__restrict__ v,
+__global__ void __launch_bounds__(VEC_THREADS) k_hash_vector(const Grid g, double *v,
                                                              double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -621,8 +621,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_hash_vector(const Grid g, doubl
 }
 
 // v /= rho (if rho > 1e-14)
-__global__ void __launch_bounds__(VEC_THREADS) k_scale_by_rho(int64_t n, const double *__restrict__ w,
-                                                              double *__restrict__ v,
+__global__ void __launch_bounds__(VEC_THREADS) k_scale_by_rho(int64_t n, const double *w,
+                                                              double *v,
                                                               const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -637,8 +637,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_scale_by_rho(int64_t n, const d
 }
 
 // w = dinv * w ; rho = ||w||
-__global__ void __launch_bounds__(VEC_THREADS) k_dinv_norm(int64_t n, double *__restrict__ w,
-                                                           const double *__restrict__ dinv,
+__global__ void __launch_bounds__(VEC_THREADS) k_dinv_norm(int64_t n, double *w,
+                                                           const double *dinv,
                                                            double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -658,8 +658,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_dinv_norm(int64_t n, double *__
 
 // dinv = 1/d if |d| > 1e-30 else 1 on real DOFs (par_solver.rs:271-274); pads 0
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_invert_diag(const Grid g, const double *__restrict__ d,
-                                                             T *__restrict__ dinv) {
+__global__ void __launch_bounds__(VEC_THREADS) k_invert_diag(const Grid g, const double *d,
+                                                             T *dinv) {
     pdl_trigger();
     pdl_wait();
     const int64_t n = (int64_t)g.NIp * g.NJ * g.NK;
@@ -674,9 +674,9 @@ __global__ void __launch_bounds__(VEC_THREADS) k_invert_diag(const Grid g, const
 
 // r = b - ap (FP64); st->rr = ||r||^2, st->res = ||r|| / bnorm; on the first
 // call (init) also st->bnorm = ||b||.  Sets done/converged against rtol/atol.
-__global__ void __launch_bounds__(VEC_THREADS) k_ir_residual(int64_t n, const double *__restrict__ b,
-                                                             const double *__restrict__ ap,
-                                                             double *__restrict__ r, double *partials,
+__global__ void __launch_bounds__(VEC_THREADS) k_ir_residual(int64_t n, const double *b,
+                                                             const double *ap,
+                                                             double *r, double *partials,
                                                              SolverState *st, int init) {
     pdl_trigger();
     pdl_wait();
@@ -712,8 +712,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_residual(int64_t n, const do
 }
 
 // r32 = r / ||r|| (the inner solve sees a unit right-hand side)
-__global__ void __launch_bounds__(VEC_THREADS) k_ir_to_f32(int64_t n, const double *__restrict__ r,
-                                                           float *__restrict__ r32,
+__global__ void __launch_bounds__(VEC_THREADS) k_ir_to_f32(int64_t n, const double *r,
+                                                           float *r32,
                                                            const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -727,8 +727,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_to_f32(int64_t n, const doub
 }
 
 // x += ||r|| * e   (FP64 solution update)
-__global__ void __launch_bounds__(VEC_THREADS) k_ir_update(int64_t n, double *__restrict__ x,
-                                                           const float *__restrict__ e,
+__global__ void __launch_bounds__(VEC_THREADS) k_ir_update(int64_t n, double *x,
+                                                           const float *e,
                                                            const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -742,8 +742,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_update(int64_t n, double *__
 }
 
 // FP32 copy of an FP64 vector
-__global__ void __launch_bounds__(VEC_THREADS) k_to_f32(int64_t n, const double *__restrict__ a,
-                                                        float *__restrict__ b) {
+__global__ void __launch_bounds__(VEC_THREADS) k_to_f32(int64_t n, const double *a,
+                                                        float *b) {
     pdl_trigger();
     pdl_wait();
     FG_VEC_LOOP(i, n) b[i] = (float)a[i];
@@ -756,8 +756,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_to_f32(int64_t n, const double 
 template <typename T>
 __global__ void __launch_bounds__(256) k_repitch(const T *__restrict__ src, int64_t sp, T *__restrict__ dst,
                                                  int64_t dp, int w, int64_t rows) {
-    pdl_trigger();
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -776,10 +774,10 @@ __global__ void __launch_bounds__(256) k_repitch(const T *__restrict__ src, int6
 // search direction p is kept, so the Krylov space is not thrown away.
 
 // x_lo += alpha p ; r_lo -= alpha ap ; rr ; sets trigger
-__global__ void __launch_bounds__(VEC_THREADS) k_rel_step(int64_t n, float *__restrict__ xlo,
-                                                          float *__restrict__ r,
-                                                          const float *__restrict__ p,
-                                                          const float *__restrict__ ap,
+__global__ void __launch_bounds__(VEC_THREADS) k_rel_step(int64_t n, float *xlo,
+                                                          float *r,
+                                                          const float *p,
+                                                          const float *ap,
                                                           double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -810,8 +808,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_step(int64_t n, float *__re
 }
 
 // reliable update, part 1: x += x_lo ; x_lo = 0
-__global__ void __launch_bounds__(VEC_THREADS) k_rel_xupdate(int64_t n, double *__restrict__ x,
-                                                             float *__restrict__ xlo,
+__global__ void __launch_bounds__(VEC_THREADS) k_rel_xupdate(int64_t n, double *x,
+                                                             float *xlo,
                                                              const SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -827,9 +825,9 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_xupdate(int64_t n, double *
 
 // reliable update, part 2 (after ap = A x in FP64): r_lo = b - ap ; true residual
 // check; on init also bnorm.  init also runs when trigger is clear.
-__global__ void __launch_bounds__(VEC_THREADS) k_rel_residual(int64_t n, const double *__restrict__ b,
-                                                              const double *__restrict__ ap,
-                                                              float *__restrict__ r,
+__global__ void __launch_bounds__(VEC_THREADS) k_rel_residual(int64_t n, const double *b,
+                                                              const double *ap,
+                                                              float *r,
                                                               double *partials, SolverState *st,
                                                               int init) {
     pdl_trigger();
@@ -877,9 +875,9 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_residual(int64_t n, const d
 
 // z = dinv r ; rz_new = r.z ; beta (init: rz only)
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_jacobi_rz(int64_t n, const T *__restrict__ r,
-                                                           const T *__restrict__ dinv,
-                                                           T *__restrict__ z, double *partials,
+__global__ void __launch_bounds__(VEC_THREADS) k_jacobi_rz(int64_t n, const T *r,
+                                                           const T *dinv,
+                                                           T *z, double *partials,
                                                            SolverState *st, int init) {
     pdl_trigger();
     pdl_wait();
@@ -902,9 +900,9 @@ __global__ void __launch_bounds__(VEC_THREADS) k_jacobi_rz(int64_t n, const T *_
 }
 
 // out = a x + b y   (FP64; SDIRK stage combinations)
-__global__ void __launch_bounds__(VEC_THREADS) k_lincomb2(int64_t n, double *__restrict__ out, double a,
-                                                          const double *__restrict__ x, double b,
-                                                          const double *__restrict__ y) {
+__global__ void __launch_bounds__(VEC_THREADS) k_lincomb2(int64_t n, double *out, double a,
+                                                          const double *x, double b,
+                                                          const double *y) {
     pdl_trigger();
     pdl_wait();
     FG_VEC4_LOOP(q, n) {
@@ -1159,7 +1157,7 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_true_residual(const BatchVec *
 }
 
 // st->tmp[2] = ||v|| (FP64)
-__global__ void __launch_bounds__(VEC_THREADS) k_norm_tmp(int64_t n, const double *__restrict__ v,
+__global__ void __launch_bounds__(VEC_THREADS) k_norm_tmp(int64_t n, const double *v,
                                                           double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -1173,7 +1171,7 @@ __global__ void __launch_bounds__(VEC_THREADS) k_norm_tmp(int64_t n, const doubl
 }
 
 // v *= 1/tmp[2] (inverse = 1) or v *= tmp[2]; no-op when tmp[2] == 0
-__global__ void __launch_bounds__(VEC_THREADS) k_scale_tmp(int64_t n, double *__restrict__ v,
+__global__ void __launch_bounds__(VEC_THREADS) k_scale_tmp(int64_t n, double *v,
                                                            const SolverState *st, int inverse) {
     pdl_trigger();
     pdl_wait();
@@ -1189,8 +1187,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_scale_tmp(int64_t n, double *__
 
 // energy terms of a coarse correction c:  st->tmp[0] = c . (A c),
 // st->tmp[1] = c . r;  ac <- A c - r
-__global__ void __launch_bounds__(VEC_THREADS) k_energy_terms(int64_t n, const double *__restrict__ c,
-                                                              double *__restrict__ ac, const double *__restrict__ r,
+__global__ void __launch_bounds__(VEC_THREADS) k_energy_terms(int64_t n, const double *c,
+                                                              double *ac, const double *r,
                                                               double *partials, SolverState *st) {
     pdl_trigger();
     pdl_wait();
@@ -1215,8 +1213,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_energy_terms(int64_t n, const d
 // ---- flexible CG (Notay's FCG with one stored direction) -------------------
 // beta = -(z . A p_old) / (p_old . A p_old)  (0 on init);  then p = z + beta p
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_fcg_zap(int64_t n, const T *__restrict__ z,
-                                                         const T *__restrict__ ap, double *partials,
+__global__ void __launch_bounds__(VEC_THREADS) k_fcg_zap(int64_t n, const T *z,
+                                                         const T *ap, double *partials,
                                                          SolverState *st, int init) {
     pdl_trigger();
     pdl_wait();
@@ -1238,9 +1236,9 @@ __global__ void __launch_bounds__(VEC_THREADS) k_fcg_zap(int64_t n, const T *__r
 // one vector pass and one launch fewer.  rz is the FCG step numerator (alpha =
 // rz / pap in k_pcg_pap)
 template <typename T>
-__global__ void __launch_bounds__(VEC_THREADS) k_fcg_pupdate_pr(int64_t n, const T *__restrict__ z,
-                                                                T *__restrict__ p,
-                                                                const T *__restrict__ r, double *partials,
+__global__ void __launch_bounds__(VEC_THREADS) k_fcg_pupdate_pr(int64_t n, const T *z,
+                                                                T *p,
+                                                                const T *r, double *partials,
                                                                 SolverState *st, int init) {
     pdl_trigger();
     pdl_wait();
@@ -1298,10 +1296,10 @@ __global__ void __launch_bounds__(VEC_THREADS) k_sh_dots(int64_t n_own, const Ve
 // alpha = s[0] / s[1] (r.z / p.Ap after the allreduce); x += alpha p,
 // r -= alpha Ap, z = dinv r on the whole local vector; out = (r.r, r.z) over
 // the owned prefix
-__global__ void __launch_bounds__(VEC_THREADS) k_sh_update(int64_t n, int64_t n_own, double *__restrict__ x,
-                                                           double *__restrict__ r, const double *__restrict__ p,
-                                                           const double *__restrict__ ap,
-                                                           const double *__restrict__ dinv, double *__restrict__ z,
+__global__ void __launch_bounds__(VEC_THREADS) k_sh_update(int64_t n, int64_t n_own, double *x,
+                                                           double *r, const double *p,
+                                                           const double *ap,
+                                                           const double *dinv, double *z,
                                                            const double *s, double *partials, SolverState *st,
                                                            double *out) {
     pdl_trigger();
@@ -1334,8 +1332,8 @@ __global__ void __launch_bounds__(VEC_THREADS) k_sh_update(int64_t n, int64_t n_
 }
 
 // p = z + (num / den) p
-__global__ void __launch_bounds__(VEC_THREADS) k_sh_pupdate(int64_t n, const double *__restrict__ z,
-                                                            double *__restrict__ p, const double *num,
+__global__ void __launch_bounds__(VEC_THREADS) k_sh_pupdate(int64_t n, const double *z,
+                                                            double *p, const double *num,
                                                             const double *den) {
     pdl_trigger();
     pdl_wait();
