@@ -117,7 +117,6 @@ __device__ __forceinline__ void chunk_sums(const ChunkLists &L, const ChunkStage
 template <typename T>
 __global__ void chunk_shared_kernel(const ChunkLists L, const T *x, T *y, int accumulate,
                                     int constrained, int diag, const int *skip) {
-    pdl_trigger();
     pdl_wait();
     if (skip && *skip) return;
     const T *part = reinterpret_cast<const T *>(L.part);

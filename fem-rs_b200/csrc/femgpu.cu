@@ -63,15 +63,21 @@ static int fail(int status, const char *fmt, ...) {
             return fail(FG_UNSUPPORTED, "%s needs a structured hex box (fg_op_create)", what); \
     } while (0)
 
-// Launch that may start before the kernel ahead of it in the stream has ended
-// (pdl_trigger / pdl_wait, fg_common.cuh); the kernel must call pdl_wait.  It
-// hides the launch and the start-up of a CTA behind the tail of the kernel ahead:
-// 8^3 Q2 FP64 apply and fix-up 12.3 -> 10.0 us, 48^3 Q3 FP32 affine 43.0 -> 39.0, 40^3 P2
-// tetrahedra 37.0 -> 33.1, the Jacobi-PCG solve of 24^3 Q1 2.51 -> 2.11 ms (with
-// vec_grid).  dep = false: an ordinary launch.
+// Launch that may start once every CTA of the kernel ahead of it in the stream has
+// exited, while that kernel's writes are still on their way (pdl_wait, fg_common.cuh;
+// the kernel must call it).  It hides the launch: 8^3 Q2 FP64 apply and fix-up 14.4 ->
+// 10.2 us (10.6 -> 9.9 replayed from a graph), 24^3 Q1 10.3 -> 8.2, a Chebyshev iteration
+// of 24^3 Q1 FP64 108 -> 88, of 64^3 Q2 444 -> 432.
+// No kernel releases its successor earlier (griddepcontrol.launch_dependents).  With a
+// release at the start of each kernel the CTAs of the fix-up, and of the vector
+// kernel behind it, waited beside the running apply, slowed it and sat unevenly on the
+// SMs once they ran: per Chebyshev iteration of 64^3 Q3 FP64 1,450 us (1,330 without,
+// ordinary launches 1,335), 64^3 Q2 500 (432), 48^3 Q2 Jacobi-PCG 81 (71); 24^3 Q3 FP64 mass +
+// diffusion replayed from a graph 33.8 (29.6).  For the same reason the box applies
+// fetch nothing before pdl_wait: quadrature columns ahead of the x tile cost more than
+// they hid (48 x 40 x 30 Q2 33.1 against 31.2 us).
 template <typename... P, typename... A>
-static cudaError_t launch_dep(bool dep, void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
-                              A &&...args) {
+static cudaError_t launch_dep(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A &&...args) {
     cudaLaunchConfig_t lc{};
     lc.gridDim = grid;
     lc.blockDim = dim3((unsigned)threads);
@@ -81,17 +87,14 @@ static cudaError_t launch_dep(bool dep, void (*kern)(P...), dim3 grid, int threa
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at;
-    lc.numAttrs = dep ? 1 : 0;
+    lc.numAttrs = 1;
     return cudaLaunchKernelEx(&lc, kern, std::forward<A>(args)...);
 }
+// The solvers' vector kernels over n values (their first argument).
 template <typename... P, typename... A>
-static cudaError_t launch_dep(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A &&...args) {
-    return launch_dep(true, kern, grid, threads, smem, stream, std::forward<A>(args)...);
+static cudaError_t launch_vec(void (*kern)(int64_t, P...), cudaStream_t stream, int64_t n, A &&...args) {
+    return launch_dep(kern, dim3(vec_grid(n)), VEC_THREADS, 0, stream, n, std::forward<A>(args)...);
 }
-// Box applies and fix-ups of more CTAs than this are launched the ordinary way: in
-// a launch of many rounds the waiting CTAs of the next kernel take slots from the
-// last round (128^3 Q2 FP64, 2048 items: 549 us ordinary, 560 us dependent).
-constexpr unsigned DEP_MAX_CTAS = 148 * 8;
 
 #include "chunk_host.cuh"
 #include "unet_host.cuh"
@@ -472,10 +475,8 @@ static int launch_apply_t(fg_op *op, const Grid &g, const T *qd, T *face, const 
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) return fail(FG_CUDA_ERROR, "cuTensorMapEncodeTiled failed (%d)", (int)cr);
     const unsigned grid = (unsigned)(nitems < 0 ? g.n_items() : nitems);
-    const bool dep = grid <= DEP_MAX_CTAS;
-    // in an ordinary launch the x tile, which the first layer waits for, goes first
-    ApplyArgs<T> A{g, qd, y, face, accumulate, op->d_err, skip, fixcnt, op->wait_ns, item0, dep && !skip ? 1 : 0};
-    CK(launch_dep(dep, kern, dim3(grid), C::WY * 32, SM::bytes, op->stream, tmap, A));
+    ApplyArgs<T> A{g, qd, y, face, accumulate, op->d_err, skip, fixcnt, op->wait_ns, item0};
+    CK(launch_dep(kern, dim3(grid), C::WY * 32, SM::bytes, op->stream, tmap, A));
     return FG_OK;
 }
 
@@ -524,7 +525,7 @@ template <typename T>
 static int launch_fixup(fg_op *op, const Grid &g, T *y, const T *face, const int *skip) {
     const dim3 grid = fixup_grid(g);
     if (grid.x == 0) return FG_OK;
-    CK(launch_dep((unsigned)g.n_items() <= DEP_MAX_CTAS, fixup_kernel<T>, grid, 128, 0, op->stream, g, y, face, skip));
+    CK(launch_dep(fixup_kernel<T>, grid, 128, 0, op->stream, g, y, face, skip));
     return FG_OK;
 }
 
@@ -1279,13 +1280,12 @@ static int estimate_lmax(fg_op *op, int iters, double *out) {
     int rc;
     const int64_t n = op->Nn;
     k_hash_vector<<<VEC_GRID, VEC_THREADS, 0, op->stream>>>(op->g, op->cd, op->partials, op->st);
-    CK(launch_dep(k_scale_by_rho, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->cd, op->cd, op->st));
+    CK(launch_vec(k_scale_by_rho, op->stream, n, op->cd, op->cd, op->st));
     CK(cudaGetLastError());
     for (int it = 0; it < iters; ++it) {
         if ((rc = apply_native(op, op->cd, op->ct, 0, 1, nullptr))) return rc;
-        CK(launch_dep(k_dinv_norm, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->ct, op->dinv, op->partials,
-                      op->st));
-        CK(launch_dep(k_scale_by_rho, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->ct, op->cd, op->st));
+        CK(launch_vec(k_dinv_norm, op->stream, n, op->ct, op->dinv, op->partials, op->st));
+        CK(launch_vec(k_scale_by_rho, op->stream, n, op->ct, op->cd, op->st));
         CK(cudaGetLastError());
     }
     SolverState h;
@@ -1343,36 +1343,33 @@ static int cheb_apply(fg_op *op, const PcgBufs<T> &B, const ChebCoef &cc, const 
                 int rc = alloc_vec(&dk[k - 1], n);
                 if (rc) return rc;
             }
-        CK(launch_dep(k_cheb_first_d<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, r, B.dinv, B.cres, B.cd,
-                      cc.inv_theta, sst));
+        CK(launch_vec(k_cheb_first_d<T>, op->stream, n, r, B.dinv, B.cres, B.cd, cc.inv_theta, sst));
         CK(cudaGetLastError());
         const T *dprev = B.cd;
         for (int k = 1; k <= s; ++k) {
             int rc = apply_native_t<T>(op, B.qd, B.face, dprev, B.ct, 0, 1, skip);
             if (rc) return rc;
             if (k < s) {
-                CK(launch_dep(k_cheb_mid<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.ct, B.dinv, B.cres,
-                              dprev, dk[k - 1], cc.c1[k - 1], cc.c2[k - 1], sst));
+                CK(launch_vec(k_cheb_mid<T>, op->stream, n, B.ct, B.dinv, B.cres, dprev, dk[k - 1], cc.c1[k - 1],
+                              cc.c2[k - 1], sst));
                 dprev = dk[k - 1];
             } else {
                 ChebSum<T> earlier{};
                 earlier.n = s - 1;  // d_0 .. d_{s-2}
                 for (int j = 0; j < s - 1; ++j) earlier.d[j] = j == 0 ? B.cd : dk[j - 1];
-                CK(launch_dep(k_cheb_last<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.ct, B.dinv, B.cres,
-                              dprev, earlier, z, cc.c1[k - 1], cc.c2[k - 1], sst));
+                CK(launch_vec(k_cheb_last<T>, op->stream, n, B.ct, B.dinv, B.cres, dprev, earlier, z, cc.c1[k - 1],
+                              cc.c2[k - 1], sst));
             }
             CK(cudaGetLastError());
         }
         return FG_OK;
     }
-    CK(launch_dep(k_cheb_first<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, r, B.dinv, B.cres, B.cd, z,
-                  cc.inv_theta, sst));
+    CK(launch_vec(k_cheb_first<T>, op->stream, n, r, B.dinv, B.cres, B.cd, z, cc.inv_theta, sst));
     CK(cudaGetLastError());
     for (size_t s = 0; s < cc.c1.size(); ++s) {
         int rc = apply_native_t<T>(op, B.qd, B.face, B.cd, B.ct, 0, 1, skip);
         if (rc) return rc;
-        CK(launch_dep(k_cheb_step<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.ct, B.dinv, B.cres, B.cd, z,
-                      cc.c1[s], cc.c2[s], sst));
+        CK(launch_vec(k_cheb_step<T>, op->stream, n, B.ct, B.dinv, B.cres, B.cd, z, cc.c1[s], cc.c2[s], sst));
         CK(cudaGetLastError());
     }
     return FG_OK;
@@ -1501,13 +1498,13 @@ static int pcg_run(fg_op *op, const PcgBufs<T> &B, bool jacobi_like, const ChebC
         if ((rc = apply_native_t<T>(op, B.qd, B.face, B.x, B.ap, 0, 1, nullptr))) return rc;
         ++*applies;
     }
-    CK(launch_dep(k_pcg_init<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.b, B.ap, B.dinv, B.r, B.z, B.p,
-                  jacobi_like ? 1 : 0, op->partials, B.st));
+    CK(launch_vec(k_pcg_init<T>, op->stream, n, B.b, B.ap, B.dinv, B.r, B.z, B.p, jacobi_like ? 1 : 0, op->partials,
+                  B.st));
     CK(cudaGetLastError());
     if (cheb) {
         if ((rc = cheb_apply<T>(op, B, *cc, B.r, B.z, skip))) return rc;
-        CK(launch_dep(k_pcg_rz<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.r, B.z, op->partials, B.st, 1));
-        CK(launch_dep(k_pcg_pupdate<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.z, B.p, B.st, 1));
+        CK(launch_vec(k_pcg_rz<T>, op->stream, n, B.r, B.z, op->partials, B.st, 1));
+        CK(launch_vec(k_pcg_pupdate<T>, op->stream, n, B.z, B.p, B.st, 1));
         CK(cudaGetLastError());
     }
     int launched = 0;
@@ -1520,15 +1517,14 @@ static int pcg_run(fg_op *op, const PcgBufs<T> &B, bool jacobi_like, const ChebC
             if ((r2 = launch_pcg_fused<T>(op, B, &used))) return r2;
             if (used) return FG_OK;
         }
-        CK(launch_dep(k_pcg_pap<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.p, B.ap, op->partials, B.st));
-        CK(launch_dep(k_pcg_update<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream,  n, B.x, B.r, B.p, B.ap, B.dinv,
-                      B.z, cheb ? 0 : 1, op->partials, B.st));
+        CK(launch_vec(k_pcg_pap<T>, op->stream, n, B.p, B.ap, op->partials, B.st));
+        CK(launch_vec(k_pcg_update<T>, op->stream, n, B.x, B.r, B.p, B.ap, B.dinv, B.z, cheb ? 0 : 1, op->partials,
+                      B.st));
         if (cheb) {
             if ((r2 = cheb_apply<T>(op, B, *cc, B.r, B.z, skip))) return r2;
-            CK(launch_dep(k_pcg_rz<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.r, B.z, op->partials, B.st,
-                          0));
+            CK(launch_vec(k_pcg_rz<T>, op->stream, n, B.r, B.z, op->partials, B.st, 0));
         }
-        CK(launch_dep(k_pcg_pupdate<T>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.z, B.p, B.st, 0));
+        CK(launch_vec(k_pcg_pupdate<T>, op->stream, n, B.z, B.p, B.st, 0));
         CK(cudaGetLastError());
         return FG_OK;
     };
@@ -1723,18 +1719,15 @@ static int fcg_nn_run(fg_op *op, const PcgBufs<double> &B, const ChebCoef &cc, i
     *fell_back = 0;
     if ((rc = apply_native_t<double>(op, B.qd, B.face, B.x, B.ap, 0, 1, nullptr))) return rc;
     ++*applies;
-    CK(launch_dep(k_pcg_init<double>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.b, B.ap, B.dinv, B.r, B.z,
-                  B.p, 0, op->partials, B.st));
+    CK(launch_vec(k_pcg_init<double>, op->stream, n, B.b, B.ap, B.dinv, B.r, B.z, B.p, 0, op->partials, B.st));
     auto direction = [&](int init) -> int {
         const float *f1 = nullptr;
         int r2;
         if (nn_on && (r2 = nn_begin<double>(op, B.r, &f1))) return r2;
         if ((r2 = cheb_apply<double>(op, B, cc, B.r, B.z, skip))) return r2;
         if (nn_on && (r2 = nn_end<double>(op, f1, B.z))) return r2;
-        CK(launch_dep(k_fcg_zap<double>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.z, B.ap, op->partials,
-                      B.st, init));
-        CK(launch_dep(k_fcg_pupdate_pr<double>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.z, B.p, B.r,
-                      op->partials, B.st, init));
+        CK(launch_vec(k_fcg_zap<double>, op->stream, n, B.z, B.ap, op->partials, B.st, init));
+        CK(launch_vec(k_fcg_pupdate_pr<double>, op->stream, n, B.z, B.p, B.r, op->partials, B.st, init));
         CK(cudaGetLastError());
         return FG_OK;
     };
@@ -1744,10 +1737,8 @@ static int fcg_nn_run(fg_op *op, const PcgBufs<double> &B, const ChebCoef &cc, i
     auto iteration = [&]() -> int {
         int r2;
         if ((r2 = apply_native_t<double>(op, B.qd, B.face, B.p, B.ap, 0, 1, skip))) return r2;
-        CK(launch_dep(k_pcg_pap<double>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.p, B.ap, op->partials,
-                      B.st));
-        CK(launch_dep(k_pcg_update<double>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, B.x, B.r, B.p, B.ap,
-                      B.dinv, B.z, 0, op->partials, B.st));
+        CK(launch_vec(k_pcg_pap<double>, op->stream, n, B.p, B.ap, op->partials, B.st));
+        CK(launch_vec(k_pcg_update<double>, op->stream, n, B.x, B.r, B.p, B.ap, B.dinv, B.z, 0, op->partials, B.st));
         return direction(0);
     };
     while (launched < max_iter) {
@@ -1977,8 +1968,7 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
         // r = b - A x (FP64), r_lo = r
         if ((rc = apply_native(op, op->xw, op->ap, 0, 1, nullptr))) return rc;
         ++applies;
-        CK(launch_dep(k_rel_residual, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->bw, op->ap, op->r32,
-                      op->partials, op->st, 1));
+        CK(launch_vec(k_rel_residual, op->stream, n, op->bw, op->ap, op->r32, op->partials, op->st, 1));
         // z = M r_lo ; p = z ; rz
         bool nn_on = learned && use_nn;
         auto precond = [&](int init) -> int {
@@ -1988,24 +1978,20 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
                 if (nn_on && (rc2 = nn_begin<float>(op, op->r32, &f1))) return rc2;
                 if ((rc2 = cheb_apply<float>(op, B, cc, op->r32, op->z32, done))) return rc2;
                 if (nn_on && (rc2 = nn_end<float>(op, f1, op->z32))) return rc2;
-                CK(launch_dep(k_fcg_zap<float>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->z32, op->ap32,
-                              op->partials, op->st, init));
-                CK(launch_dep(k_fcg_pupdate_pr<float>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->z32,
-                              op->p32, op->r32, op->partials, op->st, init));
+                CK(launch_vec(k_fcg_zap<float>, op->stream, n, op->z32, op->ap32, op->partials, op->st, init));
+                CK(launch_vec(k_fcg_pupdate_pr<float>, op->stream, n, op->z32, op->p32, op->r32, op->partials, op->st,
+                              init));
                 CK(cudaGetLastError());
                 return FG_OK;
             }
             if (cheb) {
                 int rc2 = cheb_apply<float>(op, B, cc, op->r32, op->z32, done);
                 if (rc2) return rc2;
-                CK(launch_dep(k_pcg_rz<float>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->r32, op->z32,
-                              op->partials, op->st, init));
+                CK(launch_vec(k_pcg_rz<float>, op->stream, n, op->r32, op->z32, op->partials, op->st, init));
             } else {
-                CK(launch_dep(k_jacobi_rz<float>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->r32, dinv32,
-                              op->z32, op->partials, op->st, init));
+                CK(launch_vec(k_jacobi_rz<float>, op->stream, n, op->r32, dinv32, op->z32, op->partials, op->st, init));
             }
-            CK(launch_dep(k_pcg_pupdate<float>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->z32, op->p32,
-                          op->st, init));
+            CK(launch_vec(k_pcg_pupdate<float>, op->stream, n, op->z32, op->p32, op->st, init));
             CK(cudaGetLastError());
             return FG_OK;
         };
@@ -2015,15 +2001,12 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
         auto iteration = [&]() -> int {
             int r2;
             if ((r2 = apply_native_t<float>(op, op->qd32, op->face32, op->p32, op->ap32, 0, 1, done))) return r2;
-            CK(launch_dep(k_pcg_pap<float>, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->p32, op->ap32,
-                          op->partials, op->st));
-            CK(launch_dep(k_rel_step, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->e32, op->r32, op->p32,
-                          op->ap32, op->partials, op->st));
+            CK(launch_vec(k_pcg_pap<float>, op->stream, n, op->p32, op->ap32, op->partials, op->st));
+            CK(launch_vec(k_rel_step, op->stream, n, op->e32, op->r32, op->p32, op->ap32, op->partials, op->st));
             // reliable update (kernels return at once unless triggered)
-            CK(launch_dep(k_rel_xupdate, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->xw, op->e32, op->st));
+            CK(launch_vec(k_rel_xupdate, op->stream, n, op->xw, op->e32, op->st));
             if ((r2 = apply_native(op, op->xw, op->ap, 0, 1, skip_rel))) return r2;
-            CK(launch_dep(k_rel_residual, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->bw, op->ap, op->r32,
-                          op->partials, op->st, 0));
+            CK(launch_vec(k_rel_residual, op->stream, n, op->bw, op->ap, op->r32, op->partials, op->st, 0));
             return precond(0);
         };
         while (launched < cfg.max_iter) {
@@ -2047,8 +2030,7 @@ static int pcg_core(fg_op *op, const fg_cfg &cfg, fg_result *res) {
     CK(cudaEventRecord(op->ev1, op->stream));
     // true residual in FP64
     if ((rc = apply_native(op, op->xw, op->ap, 0, 1, nullptr))) return rc;
-    CK(launch_dep(k_true_residual, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->bw, op->ap, op->partials,
-                  op->st));
+    CK(launch_vec(k_true_residual, op->stream, n, op->bw, op->ap, op->partials, op->st));
     CK(cudaGetLastError());
     SolverState h2;
     if ((rc = read_state(op, &h2))) return rc;
@@ -2816,16 +2798,15 @@ FG_API int fg_sdirk2(fg_op *stiff, fg_op *stage, double *u, double dt, int n_ste
     double *scal = nullptr;  // ||b|| kept in a device scalar between the two calls
     auto normalise = [&](bool before) -> int {
         if (before) {
-            CK(launch_dep(k_norm_tmp, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->bw, stage->partials,
-                          stage->st));
-            CK(launch_dep(k_scale_tmp, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->bw, stage->st, 1));
-            CK(launch_dep(k_scale_tmp, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->xw, stage->st, 1));
+            CK(launch_vec(k_norm_tmp, stage->stream, n, stage->bw, stage->partials, stage->st));
+            CK(launch_vec(k_scale_tmp, stage->stream, n, stage->bw, stage->st, 1));
+            CK(launch_vec(k_scale_tmp, stage->stream, n, stage->xw, stage->st, 1));
             CK(cudaMemcpyAsync(scal, &stage->st->tmp[2], sizeof(double), cudaMemcpyDeviceToDevice,
                                stage->stream));
         } else {
             CK(cudaMemcpyAsync(&stage->st->tmp[2], scal, sizeof(double), cudaMemcpyDeviceToDevice,
                                stage->stream));
-            CK(launch_dep(k_scale_tmp, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->xw, stage->st, 0));
+            CK(launch_vec(k_scale_tmp, stage->stream, n, stage->xw, stage->st, 0));
         }
         CK(cudaGetLastError());
         return FG_OK;
@@ -2836,8 +2817,7 @@ FG_API int fg_sdirk2(fg_op *stiff, fg_op *stage, double *u, double dt, int n_ste
         int r2 = apply_native(stiff, ucur, stage->sd_w, 0, 1, nullptr);
         if (r2) return r2;
         ++applies;
-        CK(launch_dep(k_lincomb2, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->bw, -1.0, stage->sd_w,
-                      0.0, stage->sd_w));
+        CK(launch_vec(k_lincomb2, stage->stream, n, stage->bw, -1.0, stage->sd_w, 0.0, stage->sd_w));
         CK(cudaGetLastError());
         fg_result r{};
         int st = normalise(true);
@@ -2856,12 +2836,10 @@ FG_API int fg_sdirk2(fg_op *stiff, fg_op *stage, double *u, double dt, int n_ste
         CK(cudaMemcpyAsync(stage->sd_k1, stage->xw, sizeof(double) * n, cudaMemcpyDeviceToDevice,
                            stage->stream));
         // u2 = u + dt (1-g) k1 (held in the solver's r buffer until the stiff apply reads it)
-        CK(launch_dep(k_lincomb2, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->r, 1.0, stage->sd_u,
-                      dt * (1.0 - g), stage->sd_k1));
+        CK(launch_vec(k_lincomb2, stage->stream, n, stage->r, 1.0, stage->sd_u, dt * (1.0 - g), stage->sd_k1));
         if ((rc = apply_native(stiff, stage->r, stage->sd_w, 0, 1, nullptr))) return rc;
         ++applies;
-        CK(launch_dep(k_lincomb2, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->bw, -1.0, stage->sd_w,
-                      0.0, stage->sd_w));
+        CK(launch_vec(k_lincomb2, stage->stream, n, stage->bw, -1.0, stage->sd_w, 0.0, stage->sd_w));
         {
             fg_result r{};
             int st = normalise(true);
@@ -2875,10 +2853,8 @@ FG_API int fg_sdirk2(fg_op *stiff, fg_op *stage, double *u, double dt, int n_ste
             max_it = std::max(max_it, (int)r.iterations);
         }
         // u += dt (1-g) k1 + dt g k2
-        CK(launch_dep(k_lincomb2, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->sd_w, dt * (1.0 - g),
-                      stage->sd_k1, dt * g, stage->xw));
-        CK(launch_dep(k_lincomb2, dim3(vec_grid(n)), VEC_THREADS, 0, stage->stream, n, stage->sd_u, 1.0, stage->sd_u,
-                      1.0, stage->sd_w));
+        CK(launch_vec(k_lincomb2, stage->stream, n, stage->sd_w, dt * (1.0 - g), stage->sd_k1, dt * g, stage->xw));
+        CK(launch_vec(k_lincomb2, stage->stream, n, stage->sd_u, 1.0, stage->sd_u, 1.0, stage->sd_w));
         CK(cudaGetLastError());
     }
     CK(cudaEventRecord(e1, stage->stream));
@@ -3444,7 +3420,7 @@ FG_API int fg_op_collect_pairs(fg_op *op, const double *b, const fg_cfg *cfg_in,
     grid_launch(nv, blocks);
     for (size_t j = 0; j < stash.size(); ++j) {
         if ((rc = apply_native(op, stash[j], op->ap, 0, 1, nullptr))) return rc;
-        CK(launch_dep(k_lincomb2, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->r, 1.0, op->bw, -1.0, op->ap));
+        CK(launch_vec(k_lincomb2, op->stream, n, op->r, 1.0, op->bw, -1.0, op->ap));
         if ((rc = nn_restrict<double>(op, op->r, op->nn_rc))) return rc;
         rms_kernel<<<1, 1024, 0, op->stream>>>(op->nn_rc, nv, op->nn_scale);
         pack_input_f32_kernel<<<blocks, 256, 0, op->stream>>>(op->nn_rc, op->nn_lk, nv, op->nn_scale,
@@ -3552,8 +3528,7 @@ FG_API int fg_unet_train_energy(fg_unet *u, fg_op *op, const double *d_res, int 
                                                            op->nn_oc);
         if ((rc = nn_prolong<double>(op, op->nn_oc, op->pv, tb + 4 * b, mult, 0))) return rc;
         if ((rc = apply_native(op, op->pv, op->ap, 0, 1, nullptr))) return rc;
-        CK(launch_dep(k_energy_terms, dim3(vec_grid(n)), VEC_THREADS, 0, op->stream, n, op->pv, op->ap, r,
-                      op->partials, op->st));
+        CK(launch_vec(k_energy_terms, op->stream, n, op->pv, op->ap, r, op->partials, op->st));
         CK(cudaMemcpyAsync(tb + 4 * b + 1, &op->st->tmp[0], 2 * sizeof(double), cudaMemcpyDeviceToDevice,
                            op->stream));
         if ((rc = nn_restrict<double>(op, op->ap, op->nn_rc))) return rc;

@@ -92,20 +92,17 @@ struct Grid {
 // ---------------------------------------------------------------------------
 // PTX helpers: dependent launches, mbarrier, bulk async copies (TMA), timers.
 // ---------------------------------------------------------------------------
-// Dependent launches: a kernel launched with launch_dep may start while its
-// predecessor in the stream is still running, once every CTA of the predecessor
-// has passed pdl_trigger (or exited).  It may touch nothing that an earlier
+// Dependent launches: a kernel launched with launch_dep may start once every CTA
+// of its predecessor in the stream has exited.  It may touch nothing that an earlier
 // kernel writes or reads before pdl_wait, which returns when the predecessor has
-// completed -- and, as every kernel so launched waits, all before it.  In a kernel
-// launched the ordinary way pdl_wait is a no-op, while pdl_trigger still releases a
-// dependent kernel behind it; a kernel that triggers therefore either waits or is
-// launched the ordinary way (then all before it has completed).
-// A kernel that waits is alive while its predecessor writes: data that any kernel
+// completed and its writes are visible -- and, as every kernel so launched waits, all
+// before it.  In a kernel launched the ordinary way pdl_wait does nothing.  No kernel
+// releases its successor before it exits (griddepcontrol.launch_dependents): see launch_dep.
+// A kernel that waits may be alive while its predecessor writes: data that any kernel
 // of a solve writes is no read-only data of it.  Such pointers are not __restrict__
 // (the compiler may move loads through them above the wait, or make them
 // non-coherent) and are not read by __ldg; matrices' data, lists and tables, which
 // are written before the first launch, may be.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);

@@ -117,7 +117,6 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
                 q_issued = j + 1;
             }
     };
-    pdl_trigger();
     if (!A.skip) issue_first();  // quadrature data and maps do not depend on earlier kernels
     // gather (E): the chunk's DOFs once, zero on the essential ones; padding
     // elements take position 0 (their quadrature data are zero and no slot names them)

@@ -86,8 +86,6 @@ template <typename T> struct ApplyArgs {
                       // between launches); null: fixup_kernel runs after the apply
     uint64_t wait_ns; // limit of each wait for a copy into shared memory; 0: 1 s
     int item0;        // first item of this launch (block b works on item item0 + b)
-    int early;        // 1: the first quadrature columns may be fetched before the kernels before this one
-                      // are done (only without a skip flag: a skipped launch must not read them)
 };
 
 template <typename T, int P>
@@ -306,16 +304,6 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
     }
     __syncthreads();
     int x_issued = 0, q_issued = 0;  // thread 0 / lane 0 bookkeeping
-    auto issue_first = [&]() {
-        if (lane == 0)
-            for (int j = 0; j < S && j < total_cols; ++j) {
-                mbar_arrive_expect_tx(&qbw[j], QBYTES);
-                bulk_g2s(qsw + j * STAGE, qdw + (int64_t)j * STAGE, QBYTES, &qbw[j]);
-                q_issued = j + 1;
-            }
-    };
-    pdl_trigger();
-    if (A.early) issue_first();
     pdl_wait();
     if (A.skip && *A.skip) return;
     if (threadIdx.x == 0) {
@@ -323,7 +311,13 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
         tma_load_3d(xs, &xmap, I0, J0, K0, &xbar[0]);
         x_issued = 1;
     }
-    if (!A.early) issue_first();
+    if (lane == 0) {
+        for (int j = 0; j < S && j < total_cols; ++j) {
+            mbar_arrive_expect_tx(&qbw[j], QBYTES);
+            bulk_g2s(qsw + j * STAGE, qdw + (int64_t)j * STAGE, QBYTES, &qbw[j]);
+            q_issued = j + 1;
+        }
+    }
     const int ess = g.ess;
     const bool fx0 = (ess & 16) && ex == 0, fx1 = (ess & 32) && ex == g.nx - 1;
     const bool fy0 = (ess & 4) && ey == 0, fy1 = (ess & 8) && ey == g.ny - 1;
@@ -1599,7 +1593,6 @@ __device__ __forceinline__ void fused_fixup(const Grid &g, T *y, const T *face, 
 // One block per row of shared-face DOFs (grid = fixup_rows(g)).
 template <typename T>
 __global__ void __launch_bounds__(128) fixup_kernel(const Grid g, T *y, const T *face, const int *skip) {
-    pdl_trigger();
     pdl_wait();
     if (skip && *skip) return;
     fixup_row<T>(g, blockIdx.x, y, face);

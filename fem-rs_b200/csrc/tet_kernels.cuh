@@ -277,7 +277,6 @@ __global__ void __launch_bounds__(BT, BT == 512 ? 2 : 3) tet_moment_kernel(const
     double *xu = reinterpret_cast<double *>(tsm_raw + sizeof(double) * NL * CE + chunk_list_smem(NL, CE, C.L.max_nu));
     const int64_t e0 = (int64_t)blockIdx.x * CE;
     const int ne = (int)(C.E - e0 < CE ? C.E - e0 : CE);
-    pdl_trigger();
     pdl_wait();  // the slot lists do not depend on earlier kernels
     chunk_load_x<double, BT>(C.L, blockIdx.x, x, xu, constrained);
     __syncthreads();
@@ -314,7 +313,6 @@ __global__ void __launch_bounds__(BT) tet_point_kernel(const TetChunk C, int nq,
     const int ne = (int)(E - e0 < CE ? E - e0 : CE);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r8 = lane >> 2, l4 = lane & 3;
     const int QT = (nq + 7) / 8;
-    pdl_trigger();
     pdl_wait();
     chunk_load_x<double, BT>(C.L, blockIdx.x, x, xu, constrained);
     __syncthreads();

@@ -130,7 +130,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_init(int64_t n, const T *b,
                                                           T *r, T *z,
                                                           T *p, int jacobi,
                                                           double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     double v[2] = {0.0, 0.0};
     FG_VEC4_LOOP(q, n) {
@@ -180,7 +179,6 @@ template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_pcg_pap(int64_t n, const T *p,
                                                          const T *ap,
                                                          double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (st->done) return;
     double v[1] = {0.0};
@@ -209,7 +207,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_pcg_update(int64_t n, T *x,
                                                             const T *dinv,
                                                             T *z, int jacobi,
                                                             double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (st->done) return;
     const T alpha = (T)st->alpha;
@@ -298,7 +295,6 @@ __global__ void __launch_bounds__(VEC_THREADS, ONE ? 1 : 4) k_pcg_fused_jacobi(i
                                                                   const T *__restrict__ dinv, T *__restrict__ z,
                                                                   double *partials, SolverState *st, unsigned *bar,
                                                                   int *err) {
-    pdl_trigger();
     if (st->done) return;
     const double rz0 = st->rz, bnorm = st->bnorm, rtol = st->rtol, atol = st->atol, stop_abs = st->stop_abs;
     const int iter0 = st->iter, max_iter = st->max_iter, cgop = st->cgop;
@@ -400,7 +396,6 @@ template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_pcg_rz(int64_t n, const T *r,
                                                         const T *z,
                                                         double *partials, SolverState *st, int init) {
-    pdl_trigger();
     pdl_wait();
     if (st->done) return;
     double v[1] = {0.0};
@@ -420,7 +415,6 @@ template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_pcg_pupdate(int64_t n, const T *z,
                                                              T *p,
                                                              const SolverState *st, int init) {
-    pdl_trigger();
     pdl_wait();
     if (st->done) return;
     const T beta = init ? T(0) : (T)st->beta;
@@ -444,7 +438,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_first(int64_t n, const T *
                                                             T *d,
                                                             T *z, double inv_theta,
                                                             const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (st && st->done) return;
     const T it = (T)inv_theta;
@@ -469,7 +462,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_step(int64_t n, const T *t
                                                            T *d,
                                                            T *z, double c1,
                                                            double c2, const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (st && st->done) return;
     const T a1 = (T)c1, a2 = (T)c2;
@@ -504,7 +496,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_first_d(int64_t n, const T
                                                               const T *dinv,
                                                               T *res, T *d,
                                                               double inv_theta, const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (st && st->done) return;
     const T it = (T)inv_theta;
@@ -528,7 +519,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_mid(int64_t n, const T *t,
                                                           const T *dprev,
                                                           T *dnext, double c1, double c2,
                                                           const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (st && st->done) return;
     const T a1 = (T)c1, a2 = (T)c2;
@@ -552,7 +542,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_last(int64_t n, const T *t
                                                            const T *dprev,
                                                            const ChebSum<T> earlier, T *z,
                                                            double c1, double c2, const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (st && st->done) return;
     const T a1 = (T)c1, a2 = (T)c2;
@@ -577,7 +566,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cheb_last(int64_t n, const T *t
 __global__ void __launch_bounds__(VEC_THREADS) k_true_residual(int64_t n, const double *b,
                                                                const double *ap,
                                                                double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     double v[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
@@ -604,7 +592,6 @@ __device__ __forceinline__ double hash_unit(uint64_t i) {
 
 __global__ void __launch_bounds__(VEC_THREADS) k_hash_vector(const Grid g, double *v,
                                                              double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     const int64_t n = (int64_t)g.NIp * g.NJ * g.NK;
     double acc[1] = {0.0};
@@ -624,7 +611,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_hash_vector(const Grid g, doubl
 __global__ void __launch_bounds__(VEC_THREADS) k_scale_by_rho(int64_t n, const double *w,
                                                               double *v,
                                                               const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     const double rho = st->rho;
     if (!(rho > 1e-14)) return;
@@ -640,7 +626,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_scale_by_rho(int64_t n, const d
 __global__ void __launch_bounds__(VEC_THREADS) k_dinv_norm(int64_t n, double *w,
                                                            const double *dinv,
                                                            double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     double acc[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
@@ -660,7 +645,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_dinv_norm(int64_t n, double *w,
 template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_invert_diag(const Grid g, const double *d,
                                                              T *dinv) {
-    pdl_trigger();
     pdl_wait();
     const int64_t n = (int64_t)g.NIp * g.NJ * g.NK;
     FG_VEC_LOOP(i, n) {
@@ -678,7 +662,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_residual(int64_t n, const do
                                                              const double *ap,
                                                              double *r, double *partials,
                                                              SolverState *st, int init) {
-    pdl_trigger();
     pdl_wait();
     double v[2] = {0.0, 0.0};
     FG_VEC4_LOOP(q, n) {
@@ -715,7 +698,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_residual(int64_t n, const do
 __global__ void __launch_bounds__(VEC_THREADS) k_ir_to_f32(int64_t n, const double *r,
                                                            float *r32,
                                                            const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     const double s = st->rr > 0.0 ? 1.0 / sqrt(st->rr) : 0.0;
     FG_VEC4_LOOP(q, n) {
@@ -730,7 +712,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_to_f32(int64_t n, const doub
 __global__ void __launch_bounds__(VEC_THREADS) k_ir_update(int64_t n, double *x,
                                                            const float *e,
                                                            const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     const double s = sqrt(st->rr);
     FG_VEC4_LOOP(q, n) {
@@ -744,7 +725,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_ir_update(int64_t n, double *x,
 // FP32 copy of an FP64 vector
 __global__ void __launch_bounds__(VEC_THREADS) k_to_f32(int64_t n, const double *a,
                                                         float *b) {
-    pdl_trigger();
     pdl_wait();
     FG_VEC_LOOP(i, n) b[i] = (float)a[i];
 }
@@ -779,7 +759,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_step(int64_t n, float *xlo,
                                                           const float *p,
                                                           const float *ap,
                                                           double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (st->done) return;
     const float alpha = (float)st->alpha;
@@ -811,7 +790,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_step(int64_t n, float *xlo,
 __global__ void __launch_bounds__(VEC_THREADS) k_rel_xupdate(int64_t n, double *x,
                                                              float *xlo,
                                                              const SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     if (!st->trigger) return;
     FG_VEC4_LOOP(q, n) {
@@ -830,7 +808,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_rel_residual(int64_t n, const d
                                                               float *r,
                                                               double *partials, SolverState *st,
                                                               int init) {
-    pdl_trigger();
     pdl_wait();
     if (!init && !st->trigger) return;
     double v[2] = {0.0, 0.0};
@@ -879,7 +856,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_jacobi_rz(int64_t n, const T *r
                                                            const T *dinv,
                                                            T *z, double *partials,
                                                            SolverState *st, int init) {
-    pdl_trigger();
     pdl_wait();
     if (st->done) return;
     double v[1] = {0.0};
@@ -903,7 +879,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_jacobi_rz(int64_t n, const T *r
 __global__ void __launch_bounds__(VEC_THREADS) k_lincomb2(int64_t n, double *out, double a,
                                                           const double *x, double b,
                                                           const double *y) {
-    pdl_trigger();
     pdl_wait();
     FG_VEC4_LOOP(q, n) {
         const V4<double> xv = ld4(x, q), yv = ld4(y, q);
@@ -1159,7 +1134,6 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_true_residual(const BatchVec *
 // st->tmp[2] = ||v|| (FP64)
 __global__ void __launch_bounds__(VEC_THREADS) k_norm_tmp(int64_t n, const double *v,
                                                           double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     double a[1] = {0.0};
     FG_VEC4_LOOP(q, n) {
@@ -1173,7 +1147,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_norm_tmp(int64_t n, const doubl
 // v *= 1/tmp[2] (inverse = 1) or v *= tmp[2]; no-op when tmp[2] == 0
 __global__ void __launch_bounds__(VEC_THREADS) k_scale_tmp(int64_t n, double *v,
                                                            const SolverState *st, int inverse) {
-    pdl_trigger();
     pdl_wait();
     const double s = st->tmp[2];
     if (!(s > 0.0)) return;
@@ -1190,7 +1163,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_scale_tmp(int64_t n, double *v,
 __global__ void __launch_bounds__(VEC_THREADS) k_energy_terms(int64_t n, const double *c,
                                                               double *ac, const double *r,
                                                               double *partials, SolverState *st) {
-    pdl_trigger();
     pdl_wait();
     double a[2] = {0.0, 0.0};
     FG_VEC4_LOOP(q, n) {
@@ -1216,7 +1188,6 @@ template <typename T>
 __global__ void __launch_bounds__(VEC_THREADS) k_fcg_zap(int64_t n, const T *z,
                                                          const T *ap, double *partials,
                                                          SolverState *st, int init) {
-    pdl_trigger();
     pdl_wait();
     if (st->done) return;
     double v[1] = {0.0};
@@ -1240,7 +1211,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_fcg_pupdate_pr(int64_t n, const
                                                                 T *p,
                                                                 const T *r, double *partials,
                                                                 SolverState *st, int init) {
-    pdl_trigger();
     pdl_wait();
     if (st->done) return;
     const T beta = init ? T(0) : (T)st->beta;
@@ -1275,7 +1245,6 @@ struct VecPairs {
 template <int NV>
 __global__ void __launch_bounds__(VEC_THREADS) k_sh_dots(int64_t n_own, const VecPairs P, double *partials,
                                                          SolverState *st, double *out) {
-    pdl_trigger();
     pdl_wait();
     double v[NV];
 #pragma unroll
@@ -1302,7 +1271,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_sh_update(int64_t n, int64_t n_
                                                            const double *dinv, double *z,
                                                            const double *s, double *partials, SolverState *st,
                                                            double *out) {
-    pdl_trigger();
     pdl_wait();
     const double alpha = s[0] / s[1];
     double v[2] = {0.0, 0.0};
@@ -1335,7 +1303,6 @@ __global__ void __launch_bounds__(VEC_THREADS) k_sh_update(int64_t n, int64_t n_
 __global__ void __launch_bounds__(VEC_THREADS) k_sh_pupdate(int64_t n, const double *z,
                                                             double *p, const double *num,
                                                             const double *den) {
-    pdl_trigger();
     pdl_wait();
     const double beta = *num / *den;
     FG_VEC4_LOOP(q, n) {

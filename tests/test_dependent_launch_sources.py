@@ -60,3 +60,11 @@ def test_no_read_only_loads_of_vectors(name):
             assert CONSTANT.match(p), f"{f}: {name}: {p} is __restrict__"
         for a in re.findall(r"__ldg\(\s*([\w.]+)", body):
             assert CONSTANT.match(a), f"{f}: {name}: __ldg({a})"
+
+
+@pytest.mark.parametrize("name", FILES + ("fg_common.cuh", "femgpu.cu"))
+def test_no_kernel_releases_its_successor_early(name):
+    """CTAs that wait beside a running kernel slow it, and take SMs unevenly: a
+    dependent kernel starts when the CTAs ahead of it have exited."""
+    with open(os.path.join(CSRC, name)) as h:
+        assert "launch_dependents" not in re.sub(r"//[^\n]*", "", h.read())
