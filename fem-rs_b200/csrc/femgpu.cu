@@ -659,21 +659,24 @@ static void set_scratch_tiling(Grid &g) {
 // warps that work at all, which separates the lane shapes when the rounds do
 // not.  32 lanes in x come first and a later candidate must win by a tenth of a
 // layer: the 8 x 4 shape pays for its shuffles and shorter rows of stores (128^3 Q2
-// FP64 517 against 552 us; a few microseconds where one round holds everything),
-// except in the Q3 FP64 full format (0.9 of the cost), where it has
-// the deeper ring (64^3: 245 against 275 us).  The rule before this one took 32 lanes
-// in x and halved the depth until there were 592 items, which left a nearly empty
-// last round or lane padding: apply and fix-up on a B200, then -> now: 48^3 Q3 FP32
-// affine 45.6 -> 34.8 us, 33x40x37 38.0 -> 24.8, 48x40x44 Q2 FP64 42.9 -> 34.1,
-// 45x41x38 Q3 FP64 121 -> 97, 100x90x80 Q1 FP64 76.9 -> 57.6, 64^3 Q2 FP32 affine
-// mass + diffusion 32.6 -> 30.6.  Over 767 random meshes of 6 to 192 elements a
-// side, all orders, kinds and forms: 2.6 % above the best of 18 shapes on average
-// (the old rule 13 %), 9 % below the old rule's time, at worst 20 % above it.
+// FP64 508 against 534 us), except where it has the deeper ring, in the Q3 FP64 full
+// format (0.9 of the cost; 64^3: 229 against 273 us).  Its mass kernel gains less from the
+// ring than the lanes cost (29 x 52 x 6: 18.9 against 16.2 us) and is left out.
+// The resident CTAs are those of each kind's kernel: with the diffusion kernels' for
+// all kinds, 62 x 63 x 17 Q3 FP64 mass + diffusion took 102 us where 83 were to be had,
+// 104 x 54 x 101 Q1 FP32 affine mass + diffusion 28.1 for 21.4.
+// The rule before this one took 32 lanes in x and halved the depth until there were
+// 592 items, which left a nearly empty last round or lane padding.  Over 2,900 random
+// meshes of 6 to 192 elements a side, all orders, kinds and forms, replayed from a
+// graph: 1.7 % above the best of 22 shapes on average (the old rule 12 %), on none
+// more than 9 % above the time of the old rule and the kernels of its time.
 static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size_t face_limit) {
-    // CTAs per SM by registers and shared memory, [fp32][affine][order]
-    static const int resident[2][2][3] = {{{3, 2, 4}, {3, 2, 2}}, {{5, 3, 4}, {5, 5, 4}}};
-    const int R = (fp32 && affine && g.p == 2 && (kind & FG_MASS)) ? 4 : resident[fp32][affine][g.p - 1];
-    const double slots = 148.0 * R;
+    // CTAs per SM by registers and shared memory, [lanes 32, 8][fp32][affine][kind][order]
+    static const int resident[2][2][2][3][3] = {
+        {{{{5, 2, 4}, {3, 2, 4}, {3, 2, 4}}, {{4, 2, 2}, {3, 2, 2}, {3, 1, 1}}},
+         {{{6, 4, 6}, {5, 3, 4}, {4, 3, 4}}, {{6, 5, 4}, {5, 5, 4}, {5, 4, 3}}}},
+        {{{{5, 2, 4}, {3, 2, 4}, {3, 2, 3}}, {{4, 2, 2}, {3, 2, 2}, {3, 1, 1}}},
+         {{{5, 4, 6}, {5, 3, 4}, {4, 3, 4}}, {{5, 5, 4}, {5, 5, 4}, {4, 4, 3}}}}};
     Grid best = g;
     double best_cost = 1e300;
     int warps32 = 0;  // warps per layer of the 32-wide shape
@@ -686,7 +689,8 @@ static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size
         // 8-wide items may not outnumber the 32-wide ones by more than a tenth: a warp
         // without elements still holds its registers, and the face slots grow
         else if (!lanes && 10 * warps > 11 * warps32) continue;
-        const double shape = LX == 8 && g.p == 3 && !fp32 && !affine ? 0.9 : 1.0;
+        const double slots = 148.0 * resident[LX == 8][fp32][affine][kind - 1][g.p - 1];
+        const double shape = LX == 8 && g.p == 3 && !fp32 && !affine && kind != FG_MASS ? 0.9 : 1.0;
         const double work = (double)(LX == 32 ? warps : live) * c.nz / (c.NW * slots);
         for (int tz = 1; tz <= std::min(g.nz, 16); ++tz) {
             set_depth(c, tz);
