@@ -647,6 +647,25 @@ static void set_scratch_tiling(Grid &g) {
 
 #define FG_NOALLOC_FACE_DOUBLES (4u << 20)  // 4 Mi doubles = 32 MiB of static face scratch
 
+// Layers' time of xy columns of items of TZ of nz layers (the last one shallower) on
+// slots = 148 R resident CTAs, where a layer takes k / S as long with k > S CTAs on an
+// SM; in layers at full residency.  c: start-up of an item in layers.
+static double item_rounds(int64_t xy, int nz, int TZ, int R, double S, double c) {
+    const int64_t slots = 148 * (int64_t)R;
+    auto layer = [&](int64_t k) { return std::max(1.0, (double)k / S); };
+    const int64_t deep = xy * (nz / TZ);
+    int64_t shallow = nz % TZ ? xy : 0;
+    const double d = TZ + c, e = nz % TZ + c;
+    double t = (double)(deep / slots) * d * layer(R);
+    if (const int64_t last = deep % slots) {  // the slots left over take shallow items
+        t += d * layer((last + 147) / 148);
+        shallow = std::max<int64_t>(0, shallow - (slots - last) * (int64_t)(d / e));
+    }
+    t += (double)(shallow / slots) * e * layer(R);
+    if (const int64_t last = shallow % slots) t += e * layer((last + 147) / 148);
+    return t / layer(R);
+}
+
 // Tile shape of one form (precision, format) of the apply: the lane shape, 32
 // elements in x or 8 in x by 4 in y, and the layers TZ per item.
 //
@@ -665,6 +684,10 @@ static void set_scratch_tiling(Grid &g) {
 // The resident CTAs are those of each kind's kernel: with the diffusion kernels' for
 // all kinds, 62 x 63 x 17 Q3 FP64 mass + diffusion took 102 us where 83 were to be had,
 // 104 x 54 x 101 Q1 FP32 affine mass + diffusion 28.1 for 21.4.
+// The Q3 FP64 affine kernels with two CTAs per SM are bound by the FP64 pipe: two
+// CTAs on an SM take 2 / 1.7 as long per layer as one, so a half-filled round is not
+// lost, and the depth of the last item counts (item_rounds): 64^3 297 us at the 4 layers
+// of the rule before this one, 323 at the 16 that whole rounds ask for, 281 at 7.
 // The rule before this one took 32 lanes in x and halved the depth until there were
 // 592 items, which left a nearly empty last round or lane padding.  Over 2,900 random
 // meshes of 6 to 192 elements a side, all orders, kinds and forms, replayed from a
@@ -689,14 +712,17 @@ static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size
         // 8-wide items may not outnumber the 32-wide ones by more than a tenth: a warp
         // without elements still holds its registers, and the face slots grow
         else if (!lanes && 10 * warps > 11 * warps32) continue;
-        const double slots = 148.0 * resident[LX == 8][fp32][affine][kind - 1][g.p - 1];
+        const int R = resident[LX == 8][fp32][affine][kind - 1][g.p - 1];
+        const double slots = 148.0 * R;
+        const bool pipe = g.p == 3 && !fp32 && affine && R > 1;
         const double shape = LX == 8 && g.p == 3 && !fp32 && !affine && kind != FG_MASS ? 0.9 : 1.0;
         const double work = (double)(LX == 32 ? warps : live) * c.nz / (c.NW * slots);
         for (int tz = 1; tz <= std::min(g.nz, 16); ++tz) {
             set_depth(c, tz);
             if (face_limit && (size_t)c.n_items() * (size_t)c.face_stride() > face_limit) continue;
             const double w = c.n_items() / slots;
-            const double cost = shape * ((w >= 3.0 ? w + 0.5 : std::ceil(w)) * (tz + 0.8) + 0.25 * work);
+            const double cost = pipe ? item_rounds((int64_t)c.ntx * c.nty, c.nz, tz, R, 1.7, 0.8)
+                                     : shape * ((w >= 3.0 ? w + 0.5 : std::ceil(w)) * (tz + 0.8) + 0.25 * work);
             if (cost < best_cost - 0.1) {
                 best_cost = cost;
                 best = c;
