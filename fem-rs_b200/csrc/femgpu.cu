@@ -1261,20 +1261,27 @@ template <typename T> static int relayout(fg_op *op, const Grid &gn, T **dst, in
     }
 }
 
-// FP32 copy of the quadrature data (in its own tile shape) and the FP32 work vectors.
-static int ensure_fp32(fg_op *op) {
+// Full-format FP32 quadrature data, in their own tile shape (an affine handle reads none).
+static int ensure_qd32(fg_op *op) {
+    if (op->qd32) return FG_OK;
+    const Grid &a = op->gv[0][0], &b = op->gv[1][0];
     int rc;
-    if (!op->qd32 && op->unstr) {
+    if (op->unstr || (a.LX == b.LX && a.TZ == b.TZ)) {  // the same layout: a straight conversion
         if ((rc = alloc_vec(&op->qd32, op->qsize))) return rc;
         k_to_f32<<<VEC_GRID * 4, VEC_THREADS, 0, op->stream>>>(op->qsize, op->qd, op->qd32);
         CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(op->stream));  // as below
+        // an unstructured apply fetches its first columns ahead of its stream order
+        if (op->unstr) CK(cudaStreamSynchronize(op->stream));
+        return FG_OK;
     }
     int64_t n32 = 0;
-    if (!op->qd32) {
-        if ((rc = relayout<float>(op, op->gv[1][0], &op->qd32, &n32))) return rc;
-        CK(cudaStreamSynchronize(op->stream));  // an apply may read the data ahead of its stream order
-    }
+    return relayout<float>(op, b, &op->qd32, &n32);
+}
+
+// FP32 quadrature data of the handle's format and the FP32 work vectors.
+static int ensure_fp32(fg_op *op) {
+    int rc;
+    if (op->fmt == 0 && (rc = ensure_qd32(op))) return rc;
     if (!op->face32 && (rc = alloc_vec(&op->face32, op->unstr ? 1 : face_words(op, 1)))) return rc;
     if (op->fmt == 1 && !op->qa32 && (rc = build_affine<float>(op, &op->qa32))) return rc;
     float **v[] = {&op->r32, &op->z32, &op->p32, &op->ap32, &op->e32, &op->b32, &op->cres32,
@@ -1816,7 +1823,10 @@ FG_API int fg_op_set_qdata_format(fg_op *op, int format) {
     if (format == FG_QDATA_AFFINE) {
         int rc;
         if (!op->qa64 && (rc = build_affine<double>(op, &op->qa64))) return rc;
-        if (op->qd32 && !op->qa32 && (rc = build_affine<float>(op, &op->qa32))) return rc;
+        if (op->face32 && !op->qa32 && (rc = build_affine<float>(op, &op->qa32))) return rc;
+    } else if (op->face32) {
+        int rc;
+        if ((rc = ensure_qd32(op))) return rc;
     }
     op->fmt = format;
     return FG_OK;
