@@ -2275,17 +2275,20 @@ static std::vector<FixBlk> fix_blocks(const std::vector<Grid> &g) {
 }
 
 // Blocks of the batched vector kernels: about 16 per SM over all instances, in
-// proportion to their lengths (at least one, at most one per 256 groups of
-// four); first[i]: the first block of instance i.
-static std::vector<BatchBlk> vec_blocks(const std::vector<int64_t> &n, std::vector<int> &first) {
+// proportion to their lengths (at least one, at most one per piece); first[i]: the
+// first partial of instance i, first[n]: their number.
+static std::vector<BatchBlk> vec_blocks(const std::vector<int64_t> &n, std::vector<int64_t> &first) {
     double total = 0.0;
     for (int64_t v : n) total += (double)v;
     std::vector<BatchBlk> m;
+    first.assign(1, 0);
     for (size_t i = 0; i < n.size(); ++i) {
-        const int most = (int)std::max<int64_t>(1, (n[i] / 4 + VEC_THREADS - 1) / VEC_THREADS);
-        const int nb = std::max(1, std::min(most, (int)(148.0 * 16.0 * (double)n[i] / total + 0.5)));
-        first.push_back((int)m.size());
-        for (int b = 0; b < nb; ++b) m.push_back(BatchBlk{(int)i, b, nb});
+        const int piece = batch_piece(n[i]), np = (int)std::max<int64_t>(1, (n[i] / 4 + piece - 1) / piece);
+        const int nb = std::max(1, std::min(np, (int)(148.0 * 16.0 * (double)n[i] / total + 0.5)));
+        for (int b = 0; b < nb; ++b)
+            m.push_back(BatchBlk{(int)i, (int)((int64_t)np * b / nb), (int)((int64_t)np * (b + 1) / nb), np, nb,
+                                 piece});
+        first.push_back(first.back() + np);
     }
     return m;
 }
@@ -2627,10 +2630,10 @@ FG_API int fg_batch_pcg(fg_op *const *ops, int n, const double *const *b, double
         g32[i] = grid_of<float>(ops[i]);
         g64[i] = grid_of<double>(ops[i]);
     }
-    std::vector<int> vfirst;
+    std::vector<int64_t> vfirst;
     const std::vector<BatchBlk> vmap = vec_blocks(len, vfirst);
     const std::vector<FixBlk> fmap = fix_blocks(g32), fmap64 = fix_blocks(g64);
-    CK(cudaMalloc(&d_part, sizeof(double) * 2 * vmap.size()));
+    CK(cudaMalloc(&d_part, sizeof(double) * 2 * vfirst.back()));
     std::vector<SolverState> hst(n);
     for (int i = 0; i < n; ++i) {
         fg_op *o = ops[i];

@@ -65,18 +65,13 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *sm) {
     __syncthreads();
 }
 
-// Writes this block's partials; returns true in the last of the sum's nb
-// blocks, whose thread 0 then holds the grand totals in `tot` (summed in block
-// order).  bid: this block's place among them.
+// The last of nb blocks to arrive (an atomic ticket) returns true; its thread 0
+// then holds in `tot` the sum of the np partials, in their order.
 template <int NV>
-__device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, SolverState *st,
-                                         double (&tot)[NV], int bid, int nb) {
-    __shared__ double sm[NV * (VEC_THREADS / 32)];
+__device__ __forceinline__ bool sum_partials(const double *partials, SolverState *st, double (&tot)[NV], double *sm,
+                                             int np, int nb) {
     __shared__ int last;
-    block_sum<NV>(v, sm);
     if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) partials[bid * NV + k] = v[k];
         __threadfence();
         const unsigned t = atomicAdd(&st->ticket, 1u);
         last = (t == (unsigned)nb - 1);
@@ -87,8 +82,8 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, Solv
     double acc[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-    // fixed order: thread i sums blocks i, i+256, ... then a fixed tree
-    for (int b = threadIdx.x; b < nb; b += VEC_THREADS)
+    // fixed order: thread i sums partials i, i+256, ... then a fixed tree
+    for (int b = threadIdx.x; b < np; b += VEC_THREADS)
 #pragma unroll
         for (int k = 0; k < NV; ++k) acc[k] += __ldcg(&partials[b * NV + k]);
     block_sum<NV>(acc, sm);
@@ -100,9 +95,17 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, Solv
     return true;
 }
 
+// Writes this block's partials; returns true in the last block, whose thread 0
+// then holds the grand totals in `tot` (summed in block order).
 template <int NV>
-__device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, SolverState *st, double (&tot)[NV]) {
-    return grid_sum<NV>(v, partials, st, tot, (int)blockIdx.x, (int)gridDim.x);
+__device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, SolverState *st,
+                                         double (&tot)[NV]) {
+    __shared__ double sm[NV * (VEC_THREADS / 32)];
+    block_sum<NV>(v, sm);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) partials[blockIdx.x * NV + k] = v[k];
+    return sum_partials<NV>(partials, st, tot, sm, (int)gridDim.x, (int)gridDim.x);
 }
 
 #define FG_VEC_LOOP(i, n) \
@@ -888,9 +891,9 @@ __global__ void __launch_bounds__(VEC_THREADS) k_lincomb2(int64_t n, double *out
     }
 }
 
-// ---- batched solves: blockIdx.y = instance ---------------------------------
+// ---- batched solves ---------------------------------------------------------
 // Per-instance pointers, state and Chebyshev coefficients; reductions use the
-// instance's own partials and ticket (grid_sum over gridDim.x blocks).
+// instance's own partials and ticket.  Block b works where map[b] says (BatchBlk).
 constexpr int BATCH_MAXK = 16;
 struct BatchVec {
     int64_t n;
@@ -903,30 +906,64 @@ struct BatchVec {
     double c1[BATCH_MAXK], c2[BATCH_MAXK];
 };
 
-// One block of a batched vector kernel: the instance it works on, its place
-// among that instance's blocks and their number.  An instance gets blocks in
-// proportion to its length: with the same 64 for every instance (the form
-// before), the largest of 16 uneven ones (3M DOFs) set the time of each launch,
-// 42 us for a sweep that takes 9 us of bandwidth.
+// One block of a batched vector kernel: its instance and the pieces [p0, p1) of that
+// instance's np that it works on, as one of the instance's nb blocks.  A piece is a
+// number of groups of four that follows from the instance's length alone, and one
+// partial of a sum, so the sums of an instance, and with them its iterations and its
+// solution, do not depend on the rest of the batch.  An instance gets blocks in
+// proportion to its length: with the same 64 for every instance the largest of 16
+// uneven ones (3M DOFs) set the time of each launch, 42 us for a sweep that takes 9 us
+// of bandwidth.  Four groups a thread and piece cost 7 % of a batch of small instances
+// (one 24^3 Q2 solve 3.9 -> 4.2 ms), one to two cost 3 % of one of large (two 48^3 Q3
+// 110 -> 113 ms): one up to 128 pieces, four above.
 struct BatchBlk {
-    int inst, bid, nb;
+    int inst, p0, p1, np, nb, piece;
 };
-#define FG_BVEC4_LOOP(q, n)                                                                \
-    for (int64_t q = (int64_t)K.bid * VEC_THREADS + threadIdx.x; q < ((n) >> 2);           \
-         q += (int64_t)K.nb * VEC_THREADS)
+inline int batch_piece(int64_t n) { return n <= 4 * 128 * VEC_THREADS ? VEC_THREADS : 4 * VEC_THREADS; }
+#define FG_BVEC4_LOOP(q, n)                                                                       \
+    for (int64_t q = (int64_t)K.p0 * K.piece + threadIdx.x,                                       \
+                 q##_end = min((int64_t)K.p1 * K.piece, (n) >> 2); q < q##_end; q += VEC_THREADS)
+
+// body(q, v) over this block's groups, v summed piece by piece; as grid_sum
+template <int NV, int PIECE, class Body>
+__device__ __forceinline__ void batch_pieces(const BatchBlk &K, int64_t n, double *partials, double *sm, Body &body) {
+    for (int p = K.p0; p < K.p1; ++p) {
+        double v[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] = 0.0;
+        const int64_t q0 = (int64_t)p * PIECE + threadIdx.x, end = n >> 2;
+        if (q0 - threadIdx.x + PIECE <= end) {
+#pragma unroll
+            for (int u = 0; u < PIECE; u += VEC_THREADS) body(q0 + u, v);
+        } else {
+            for (int64_t q = q0; q < end; q += VEC_THREADS) body(q, v);
+        }
+        block_sum<NV>(v, sm);
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) partials[p * NV + k] = v[k];
+    }
+}
+template <int NV, class Body>
+__device__ __forceinline__ bool batch_sum(const BatchBlk &K, int64_t n, double *partials, SolverState *st,
+                                          double (&tot)[NV], Body body) {
+    __shared__ double sm[NV * (VEC_THREADS / 32)];
+    if (K.piece == VEC_THREADS) batch_pieces<NV, VEC_THREADS>(K, n, partials, sm, body);
+    else batch_pieces<NV, 4 * VEC_THREADS>(K, n, partials, sm, body);
+    return sum_partials<NV>(partials, st, tot, sm, K.np, K.nb);
+}
 
 __global__ void __launch_bounds__(VEC_THREADS) kb_pap(const BatchVec *bv, const BatchBlk *map) {
     const BatchBlk K = map[blockIdx.x];
     const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
     if (st->done) return;
-    double v[1] = {0.0};
-    FG_BVEC4_LOOP(q, B.n) {
+    double tot[1];
+    const bool last = batch_sum<1>(K, B.n, B.partials, st, tot, [&](int64_t q, double (&v)[1]) {
         const V4<float> pv = ld4(B.p, q), av = ld4(B.ap, q);
         FG_K4 v[0] += (double)pv.a[k] * (double)av.a[k];
-    }
-    double tot[1];
-    if (grid_sum<1>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0) {
+    });
+    if (last && threadIdx.x == 0) {
         st->pap = tot[0];
         if (fabs(tot[0]) < 1e-30) {
             st->breakdown = 1;
@@ -944,8 +981,8 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_step(const BatchVec *bv, c
     SolverState *st = B.st;
     if (st->done) return;
     const float alpha = (float)st->alpha;
-    double v[1] = {0.0};
-    FG_BVEC4_LOOP(q, B.n) {
+    double tot[1];
+    const bool last = batch_sum<1>(K, B.n, B.partials, st, tot, [&](int64_t q, double (&v)[1]) {
         V4<float> xv = ld4(B.e, q), rv = ld4(B.r, q);
         const V4<float> pv = ld4(B.p, q), av = ld4(B.ap, q);
         FG_K4 {
@@ -955,9 +992,8 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_step(const BatchVec *bv, c
         }
         st4(B.e, q, xv);
         st4(B.r, q, rv);
-    }
-    double tot[1];
-    if (grid_sum<1>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0) {
+    });
+    if (last && threadIdx.x == 0) {
         st->iter += 1;
         st->rr = tot[0];
         const double rn = sqrt(tot[0]);
@@ -986,8 +1022,8 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_residual(const BatchVec *b
     const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
     if (!init && !st->trigger) return;
-    double v[2] = {0.0, 0.0};
-    FG_BVEC4_LOOP(q, B.n) {
+    double tot[2];
+    const bool last = batch_sum<2>(K, B.n, B.partials, st, tot, [&](int64_t q, double (&v)[2]) {
         const V4<double> bb = ld4(B.b64, q), av = ld4(B.ap64, q);
         V4<float> rv;
         FG_K4 {
@@ -997,9 +1033,8 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rel_residual(const BatchVec *b
             if (init) v[1] += bb.a[k] * bb.a[k];
         }
         st4(B.r, q, rv);
-    }
-    double tot[2];
-    if (grid_sum<2>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0) {
+    });
+    if (last && threadIdx.x == 0) {
         if (init) {
             st->bb = tot[1];
             st->bnorm = sqrt(tot[1]);
@@ -1073,8 +1108,8 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rz(const BatchVec *bv, const B
     const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
     if (st->done) return;
-    double v[1] = {0.0};
-    FG_BVEC4_LOOP(q, B.n) {
+    double tot[1];
+    const bool last = batch_sum<1>(K, B.n, B.partials, st, tot, [&](int64_t q, double (&v)[1]) {
         const V4<float> rv = ld4(B.r, q);
         V4<float> zv;
         if (jacobi) {
@@ -1085,9 +1120,8 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_rz(const BatchVec *bv, const B
             zv = ld4(B.z, q);
         }
         FG_K4 v[0] += (double)rv.a[k] * (double)zv.a[k];
-    }
-    double tot[1];
-    if (grid_sum<1>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0) {
+    });
+    if (last && threadIdx.x == 0) {
         if (!init) st->beta = tot[0] / st->rz;
         st->rz = tot[0];
     }
@@ -1118,16 +1152,15 @@ __global__ void __launch_bounds__(VEC_THREADS) kb_true_residual(const BatchVec *
     const BatchBlk K = map[blockIdx.x];
     const BatchVec &B = bv[K.inst];
     SolverState *st = B.st;
-    double v[1] = {0.0};
-    FG_BVEC4_LOOP(q, B.n) {
+    double tot[1];
+    const bool last = batch_sum<1>(K, B.n, B.partials, st, tot, [&](int64_t q, double (&v)[1]) {
         const V4<double> bb = ld4(B.b64, q), av = ld4(B.ap64, q);
         FG_K4 {
             const double s = bb.a[k] - av.a[k];
             v[0] += s * s;
         }
-    }
-    double tot[1];
-    if (grid_sum<1>(v, B.partials, st, tot, K.bid, K.nb) && threadIdx.x == 0)
+    });
+    if (last && threadIdx.x == 0)
         st->tmp[0] = st->bnorm == 0.0 ? 0.0 : sqrt(tot[0]) / st->bnorm;
 }
 
