@@ -357,12 +357,14 @@ static int unet_wgrad(fg_unet *u, const WgItem *items, int n) {
         work[k] = (double)L.ntiles * (2 + nt / 8 * wg_co16(l.cout));
         sum += work[k];
     }
-    // voxel splits: two waves' worth of blocks over all layers, in proportion to their work
+    // voxel splits: two waves' worth of blocks over all layers, in proportion to their
+    // work, and none longer than WG_CHAIN voxels
     int64_t blocks = 0, part = 0, red = 0;
     for (int k = 0; k < n; ++k) {
         WgLayer &L = A.L[k];
         const double want = 148.0 * 4 * work[k] / sum / (3 * L.groups);
-        L.splits = std::max(1, std::min(L.ntiles, (int)(want + 0.5)));
+        const int tiles = std::max(1, WG_CHAIN / (L.TX * L.TY));  // of one split, at most
+        L.splits = std::min(L.ntiles, std::max((int)(want + 0.5), (L.ntiles + tiles - 1) / tiles));
         L.blk0 = (int)blocks;
         L.part0 = part;
         L.red0 = (int)red;
