@@ -3182,6 +3182,7 @@ static int unet_copy_params(fg_unet *u, float *host, bool to_host, bool grads) {
         A.L[l] = {grads ? L.gw : L.w, grads ? L.gb : L.b, L.wb, L.cout, 27 * L.cin, L.kp, A.total};
         A.total += L.cout * (27 * L.cin + 1);
     }
+    std::lock_guard<std::mutex> lk(u->flat_mu);
     if (!u->flat) CK(cudaMalloc(&u->flat, sizeof(float) * A.total));
     const size_t nb = sizeof(float) * A.total;
     if (!to_host) CK(cudaMemcpy(u->flat, host, nb, cudaMemcpyHostToDevice));

@@ -56,6 +56,7 @@ struct fg_unet {
     fg::UnetBufs buf;
     __nv_bfloat16 *wflip = nullptr;
     size_t wflip_n = 0;
+    std::mutex flat_mu;     // readers of parameters and gradients may run on several threads
     float *flat = nullptr;  // all parameters or gradients on their way to or from the host
     int step = 0;
     cudaStream_t stream = nullptr;
