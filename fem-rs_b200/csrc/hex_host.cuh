@@ -47,17 +47,36 @@ template <typename K> static int hex_smem_limit(K kern, int device, int bytes, s
     return FG_OK;
 }
 
-template <int P, int OPK, typename T>
-static int hex_apply_t(fg_op *op, const HexApply<T> &A) {
+template <int P, int OPK, typename T, int FIRST>
+static int hex_launch(fg_op *op, const HexApply<T> &A) {
     constexpr int WARPS = HexCfg<P>::WARPS, S = HexCfg<P>::S, BS = WARPS * 32;
-    using SM = HexSmem<P, OPK, T, WARPS, S>;
-    auto kern = hex_apply_kernel<P, OPK, T, WARPS, S, HexCfg<P>::MINB>;
+    auto kern = hex_apply_kernel<P, OPK, T, WARPS, S, HexCfg<P>::MINB, FIRST>;
     static std::atomic<int> lim[64];
-    const int bytes = SM::bytes(op->u_lists.max_nu);
+    const int bytes = HexSmem<P, OPK, T, WARPS, S, FIRST>::bytes(op->u_lists.max_nu);
     int rc;
     if ((rc = hex_smem_limit(kern, op->device, bytes, lim))) return rc;
     CK(launch_dep(kern, dim3((unsigned)op->u_chunks), BS, bytes, op->stream, A));
     return FG_OK;
+}
+// Q3 FP64: the second ring stage waits for the gather where the x values in its place let
+// another CTA onto the SM (228 KB, 1 KB of each CTA the system's) and that saves a round
+// of CTAs.  The chunks of a Morton order hold more DOFs when the extents are no powers of
+// two: 48^3 297 -> 250 us, 40^3 194 -> 169, mass + diffusion 203 -> 179 (277, 189 and 194 with
+// 32-bit lists and no values of x in shared memory).  With as many rounds either way the
+// early fetch is better: 32^3 103 against 106, mass + diffusion 105 against 112.
+template <int P, int OPK, typename T>
+static int hex_apply_t(fg_op *op, const HexApply<T> &A) {
+    constexpr int WARPS = HexCfg<P>::WARPS, S = HexCfg<P>::S;
+    if constexpr (P == 3 && std::is_same<T, double>::value) {
+        const int nu = op->u_lists.max_nu;
+        auto rounds = [&](int bytes) {
+            const int64_t slots = 148 * std::max(1, std::min(HexCfg<P>::MINB, 228 * 1024 / (bytes + 1024)));
+            return (op->u_chunks + slots - 1) / slots;
+        };
+        if (rounds(HexSmem<P, OPK, T, WARPS, S, 1>::bytes(nu)) < rounds(HexSmem<P, OPK, T, WARPS, S, S>::bytes(nu)))
+            return hex_launch<P, OPK, T, 1>(op, A);
+    }
+    return hex_launch<P, OPK, T, S>(op, A);
 }
 
 template <typename T> static int hex_shared(fg_op *op, const HexApply<T> &A, int diag) {

@@ -61,37 +61,40 @@ template <int P, int OPK> __host__ __device__ inline int64_t hex_qd_index(int64_
     return (((e >> 5) * (Q * Q) + col) * Q + qz) * (NC * 32) + comp * 32 + (e & 31);
 }
 
-// Shared memory (bytes): the per-warp quadrature-data rings; the element values
-// (then results), one column per thread; a region holding first the chunk's x
-// values and, once the elements have taken them, the chunk's slot lists; the
-// ring barriers.
-template <int P, int OPK, typename T, int WARPS, int S> struct HexSmem {
+// Shared memory (bytes): the element values (then results), one column per thread; the
+// quadrature-data rings, stage by stage, each holding all warps; the chunk's slot lists;
+// the ring barriers.  The chunk's x values lie where the lists go once the elements have
+// taken them (FIRST = S), or begin at the second ring stage, which is then fetched after
+// that (FIRST = 1).  The second way takes less and is chosen where another CTA fits on the
+// SM by it (hex_apply_t).
+template <int P, int OPK, typename T, int WARPS, int S, int FIRST> struct HexSmem {
     static constexpr int Q = P + 1, NL = (P + 1) * (P + 1) * (P + 1), BS = WARPS * 32;
     static constexpr int STAGE = Q * NComp<OPK>::v * 32;  // elements of one column stage
-    static constexpr int off_x = WARPS * S * STAGE * (int)sizeof(T);
-    static constexpr int off_l = off_x + NL * BS * (int)sizeof(T);
+    static constexpr int off_q = NL * BS * (int)sizeof(T);
+    static constexpr int off_u = off_q + FIRST * WARPS * STAGE * (int)sizeof(T);
+    static constexpr int off_l = off_q + S * WARPS * STAGE * (int)sizeof(T);
     static __host__ __device__ int off_b(int max_nu) {
-        const int l = chunk_list_smem(NL, BS, max_nu), u = max_nu * (int)sizeof(T);
-        return off_l + round_up(l > u ? l : u, 16);
+        const int l = off_l + chunk_list_smem(NL, BS, max_nu), u = off_u + max_nu * (int)sizeof(T);
+        return round_up(l > u ? l : u, 16);
     }
     static __host__ __device__ int bytes(int max_nu) { return off_b(max_nu) + WARPS * S * 8; }
 };
 
-template <int P, int OPK, typename T, int WARPS, int S, int MINB>
+template <int P, int OPK, typename T, int WARPS, int S, int MINB, int FIRST>
 __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexApply<T> A) {
     constexpr int D = P + 1, Q = P + 1, NL = D * D * D, NC = NComp<OPK>::v, BS = WARPS * 32;
     constexpr bool HM = (OPK & 1) != 0, HK = (OPK & 2) != 0;
     constexpr int QH = (P == 3 && sizeof(T) == 8) ? 2 : Q;  // half slabs bound the Q3 FP64 state
     constexpr int COLS = Q * Q;
-    using SM = HexSmem<P, OPK, T, WARPS, S>;
+    using SM = HexSmem<P, OPK, T, WARPS, S, FIRST>;
     constexpr int STAGE = SM::STAGE;
     constexpr uint32_t QBYTES = (uint32_t)(STAGE * sizeof(T));
     using TB = Tab<T>;
     extern __shared__ __align__(128) unsigned char hex_smem[];
     const int MU = A.L.max_nu;
-    T *ring = reinterpret_cast<T *>(hex_smem);
-    T *xs = reinterpret_cast<T *>(hex_smem + SM::off_x);
-    T *xu = reinterpret_cast<T *>(hex_smem + SM::off_l);
+    T *xs = reinterpret_cast<T *>(hex_smem);
+    T *ring = reinterpret_cast<T *>(hex_smem + SM::off_q);
+    T *xu = reinterpret_cast<T *>(hex_smem + SM::off_u);
     uint64_t *bars = reinterpret_cast<uint64_t *>(hex_smem + SM::off_b(MU));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
     const int64_t E = A.E;
@@ -104,20 +107,21 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
         fence_barrier_init();
     }
     __syncthreads();
-    T *qsw = ring + warp * S * STAGE;
+    T *qsw = ring + warp * STAGE;  // this warp's part of stage 0
+    constexpr int NEXT = WARPS * STAGE;  // to its part of the next stage
     uint64_t *qbw = bars + warp * S;
     const T *qdw = A.qd + group * COLS * STAGE;
     int q_issued = 0, q_waited = 0;
     bool ok = true;
-    auto issue_first = [&]() {
+    auto issue = [&](int j0, int j1) {
         if (wvalid && lane == 0)
-            for (int j = 0; j < S && j < COLS; ++j) {
+            for (int j = j0; j < j1 && j < COLS; ++j) {
                 mbar_arrive_expect_tx(&qbw[j], QBYTES);
-                bulk_g2s(qsw + j * STAGE, qdw + (int64_t)j * STAGE, QBYTES, &qbw[j]);
+                bulk_g2s(qsw + j * NEXT, qdw + (int64_t)j * STAGE, QBYTES, &qbw[j]);
                 q_issued = j + 1;
             }
     };
-    if (!A.skip) issue_first();  // quadrature data and maps do not depend on earlier kernels
+    if (!A.skip) issue(0, FIRST);  // quadrature data and maps do not depend on earlier kernels
     // gather (E): the chunk's DOFs once, zero on the essential ones; padding
     // elements take position 0 (their quadrature data are zero and no slot names them)
     uint32_t lm[(NL + 1) / 2];
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
     pdl_wait();
     if (A.skip) {
         if (*A.skip) return;
-        issue_first();
+        issue(0, FIRST);
     }
     chunk_load_x<T, BS>(A.L, blockIdx.x, A.x, xu, A.constrained);
     __syncthreads();
@@ -138,7 +142,11 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
 #pragma unroll
         for (int k = 0; k < NL; ++k) xs[k * BS + tid] = xu[(lm[k / 2] >> (16 * (k & 1))) & 0xffffu];
     }
-    __syncthreads();  // the chunk's x values are free: the slot lists take their place
+    __syncthreads();  // the chunk's x values are free: later stages and the slot lists take their place
+    if (FIRST < S) {
+        fence_proxy_async();
+        issue(FIRST, S);
+    }
     const ChunkStage cst = chunk_stage_lists<BS>(A.L, blockIdx.x, hex_smem + SM::off_l);
     if (wvalid) {
         auto uval = [&](int c, int b, int a) -> T { return xs[((c * D + b) * D + a) * BS + tid]; };
@@ -197,7 +205,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
                     const int j = qy * Q + h0 + k;  // column = stream stage
                     const int st = j % S;
                     wait_stage(&qbw[st], (j / S) & 1, A.err, wlim, ok, q_waited, j + 1);
-                    const T *qc = qsw + st * STAGE + lane;
+                    const T *qc = qsw + st * NEXT + lane;
                     T vx[Q], vy[Q], vz[Q], vu[Q];
 #pragma unroll
                     for (int qz = 0; qz < Q; ++qz) {
@@ -225,7 +233,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) hex_apply_kernel(const HexAp
                     if (lane == 0 && ok && j + S < COLS) {
                         fence_proxy_async();
                         mbar_arrive_expect_tx(&qbw[st], QBYTES);
-                        bulk_g2s(qsw + st * STAGE, qdw + (int64_t)(j + S) * STAGE, QBYTES, &qbw[st]);
+                        bulk_g2s(qsw + st * NEXT, qdw + (int64_t)(j + S) * STAGE, QBYTES, &qbw[st]);
                         q_issued = j + S + 1;
                     }
 #pragma unroll
