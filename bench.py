@@ -15,8 +15,7 @@ reliable updates, affine-compressed quadrature data, the learned coarse
 correction), for 128^3 Q2 and 64^3 Q3.
 
 The JSON line carries summaries; the full record (per-form iteration counts,
-autotuner table, heat, batch, tet details) goes to --detail (default
-gpurun_out/bench_detail.json when that folder exists).
+autotuner table, heat, batch, tet details) goes to the file --detail names.
 
 --impl reference times the reference's algorithm (the oracle port of
 crates/assembly/src/partial.rs's element loop with the Hex8 isoparametric
@@ -829,8 +828,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=5)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--workload", default="q2_128", choices=sorted(WORKLOADS))
-    ap.add_argument("--detail", default=None, help="file for the full record (default: gpurun_out/bench_detail.json "
-                                                   "if that folder exists)")
+    ap.add_argument("--detail", default=None, help="file for the full record (default: none)")
     for opt in ("solve", "q3", "cpu", "heat", "batch", "tet", "ex1", "hex"):
         ap.add_argument(f"--no-{opt}", action="store_true")
     ap.add_argument("--mode", default=None, choices=["replicas", "sharded"],
@@ -1009,11 +1007,8 @@ def main():
             "ex1": ex1,
         }
         print(json.dumps(out), flush=True)
-        path = args.detail
-        if path is None and os.path.isdir(os.path.join(ROOT, "gpurun_out")):
-            path = os.path.join(ROOT, "gpurun_out", "bench_detail.json")
-        if path:
-            with open(path, "w") as f:
+        if args.detail:
+            with open(args.detail, "w") as f:
                 json.dump(dict(out, detail=detail), f, indent=1)
     op.close()
     if world > 1:

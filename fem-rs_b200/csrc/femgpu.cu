@@ -678,8 +678,8 @@ static double item_rounds(int64_t xy, int nz, int TZ, int R, double S, double c)
 // warps that work at all, which separates the lane shapes when the rounds do
 // not.  32 lanes in x come first and a later candidate must win by a tenth of a
 // layer: the 8 x 4 shape pays for its shuffles and shorter rows of stores (128^3 Q2
-// FP64 508 against 534 us), except where it has the deeper ring, in the Q3 FP64 full
-// format (0.9 of the cost; 64^3: 229 against 273 us).  Its mass kernel gains less from the
+// FP64 497 against 533 us), except where it has the deeper ring, in the Q3 FP64 full
+// format (0.9 of the cost; 64^3: 239 against 274 us).  Its mass kernel gains less from the
 // ring than the lanes cost (29 x 52 x 6: 18.9 against 16.2 us) and is left out.
 // The resident CTAs are those of each kind's kernel: with the diffusion kernels' for
 // all kinds, 62 x 63 x 17 Q3 FP64 mass + diffusion took 102 us where 83 were to be had,

@@ -209,8 +209,8 @@ __device__ __forceinline__ void merge_and_store(T (&out)[P + 1][P + 1][P + 1], c
     const int ex = tx * LX + lx, ey = ty * (WY * LY) + row, ez = tz * g.TZ + lz;
     const int SX = LX * P + 1, SY = WY * LY * P + 1;
     // g.fx(), fy(), fz() with the item's compile-time lanes and rows: from the grid's
-    // fields the sizes took registers that the Q3 FP64 forms spill for (1,330 against
-    // 1,154 bytes of stores in the affine one): 45 x 41 x 38 Q3 FP64 102 -> 93 us.
+    // fields the sizes took registers that the Q3 FP64 forms spill for (1,346 against
+    // 1,186 bytes of stores in the affine one): 45 x 41 x 38 Q3 FP64 102 -> 93 us.
     const int SZ = g.TZ * P + 1;
     T *fxp = face + (int64_t)item * (SZ * (SX + SY) + SX * SY);
     T *fyp = fxp + SZ * SY;
@@ -534,8 +534,9 @@ __device__ __forceinline__ void pa_apply_body(const CUtensorMap *xmap_ptr, const
                 // Pairs of points (qx, qx+1) in packed FMAs: the y and z derivatives, D and
                 // the transposed y and z derivatives, 22 instructions a point instead of
                 // 36 (the x derivatives stay scalar: a pair would have to be duplicated).
-                // These kernels are bound by instruction issue: 48^3 Q3 38.8 -> 37.8 us, 64^3 Q2
-                // mass + diffusion 33.4 -> 32.1, a batch of 16 instances 259 -> 248 ms.
+                // These kernels are bound by instruction issue: with new vectors each pass 48^3 Q3
+                // 38.8 -> 37.8 us, 64^3 Q2 mass + diffusion 33.4 -> 32.1, a batch of 16 instances
+                // 259 -> 248 ms.
                 float2 Gd[6];
 #pragma unroll
                 for (int k = 0; k < 6; ++k) Gd[k] = make_float2(Ge[k], Ge[k]);

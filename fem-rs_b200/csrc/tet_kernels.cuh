@@ -261,12 +261,12 @@ __host__ __device__ inline size_t tet_chunk_smem(int NL, int CE, int max_nu) {
 }
 
 // One CTA (BT threads) per chunk; diffusion by the moment form (P1, P2).  The
-// copies of the chunk's slot lists are started and its values of x read once into shared memory; then the element
-// results are computed into shared memory, each element taking its values by
-// its 16-bit positions.  After a barrier each DOF's slots are summed.  MOM:
-// diffusion-only apply by the moment form.  On essential DOFs of a constrained call
-// the identity row: y_d (+)= x_d (apply) or 1 (diagonal).  40^3 x 6 P2 tetrahedra:
-// 41.0 us with x gathered per element through a 32-bit map, 30.6 us this way (dependent launches included).
+// copies of the chunk's slot lists are started and its values of x read once into
+// shared memory; then the element results are computed into shared memory, each element
+// taking its values by its 16-bit positions.  After a barrier each DOF's slots are
+// summed.  On essential DOFs of a constrained call the identity row: y_d (+)= x_d (apply)
+// or 1 (diagonal).  40^3 x 6 P2 tetrahedra, new vectors each pass: 41.0 us with x gathered
+// per element through a 32-bit map, 30.9 us this way (with dependent launches).
 template <int NL, int BT>
 __global__ void __launch_bounds__(BT, BT == 512 ? 2 : 3) tet_moment_kernel(const TetChunk C, const double *x, double *y,
                                                                          int accumulate, int constrained) {
