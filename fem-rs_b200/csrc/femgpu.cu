@@ -267,7 +267,7 @@ struct fg_op {
     Grid g{};              // FP64 full format; the other forms' tiles in gv
     Grid gv[2][2];         // [FP32][affine]: the same mesh, each form with its own tile shape
     int ess_tags = 0, kind = 0, p = 0;
-    bool tile_set = false;  // item depth chosen by fg_op_set_tile or the autotuner
+    int limit_tz = 0;  // item depth last asked for by fg_op_set_tile or the autotuner; 0: none
     int64_t N = 0, Nn = 0;
     double *qd = nullptr, *face = nullptr;
     double *xs = nullptr, *ys = nullptr;
@@ -2195,7 +2195,10 @@ static int set_tile_locked(fg_op *op, int tz) {
         same = same && gv[k >> 1][k & 1].TZ == tz;
         set_depth(gv[k >> 1][k & 1], tz);
     }
-    if (same) return FG_OK;
+    if (same) {
+        op->limit_tz = tz;
+        return FG_OK;
+    }
     double *nq = nullptr, *nface = nullptr;
     int64_t nsize = 0;
     int rc = relayout<double>(op, gv[0][0], &nq, &nsize);
@@ -2220,8 +2223,22 @@ static int set_tile_locked(fg_op *op, int tz) {
     op->qsize = nsize;
     for (int k = 0; k < 4; ++k) op->gv[k >> 1][k & 1] = gv[k >> 1][k & 1];
     op->g = gv[0][0];
-    op->tile_set = true;
+    op->limit_tz = tz;
     if (op->fmt == 1 && (rc = build_affine<double>(op, &op->qa64))) return rc;
+    return FG_OK;
+}
+
+// Give the FP32 forms the tile shapes gv32 (full, affine); their data and face slots
+// are dropped and rebuilt on next use (caller holds op->mu).
+static int set_tiles32(fg_op *op, const Grid (&gv32)[2]) {
+    bool same = true;
+    for (int f = 0; f < 2; ++f) same = same && op->gv[1][f].TZ == gv32[f].TZ;
+    if (same) return FG_OK;
+    CK(cudaStreamSynchronize(op->stream));
+    float **f32[] = {&op->qd32, &op->face32, &op->qa32};
+    for (float **b : f32)
+        if (*b) { cudaFree(*b); *b = nullptr; }
+    for (int f = 0; f < 2; ++f) op->gv[1][f] = gv32[f];
     return FG_OK;
 }
 
@@ -2441,12 +2458,25 @@ FG_API int fg_batch_autotune(fg_op *const *ops, int n, int reps, fg_tune_entry *
         }
         return true;
     };
+    // FP32 tiles of member j of a class: as it came (k < 0) or all at candidate k's depth
+    struct Tiles { Grid g[2]; };
+    auto tiles = [&](const fg_op *o, const Tiles &came, int k) {
+        Tiles t = came;
+        if (k >= 0)
+            for (Grid &g : t.g) set_depth(g, depth(o, kTuneTZ[k]));
+        return t;
+    };
     int count = 0;
     for (const Cls &c : cls) {
         double us[2][FG_TUNE_CANDIDATES];
         int best_f = -1, best_k = -1;
+        double best_us = 0.0;
         int maxnz = 1;
-        for (int i : c.inst) maxnz = std::max(maxnz, ops[i]->g.nz);
+        std::vector<Tiles> came;
+        for (int i : c.inst) {
+            maxnz = std::max(maxnz, ops[i]->g.nz);
+            came.push_back(Tiles{{ops[i]->gv[1][0], ops[i]->gv[1][1]}});
+        }
         for (int f = 0; f < 2; ++f) {
             for (int k = 0; k < FG_TUNE_CANDIDATES; ++k) us[f][k] = -1.0;
             int err;
@@ -2454,12 +2484,20 @@ FG_API int fg_batch_autotune(fg_op *const *ops, int n, int reps, fg_tune_entry *
                 if (err) return err;
                 continue;
             }
-            for (int k = 0; k < FG_TUNE_CANDIDATES; ++k) {
+            for (int k = -1; k < FG_TUNE_CANDIDATES; ++k) {
                 if (k > 0 && kTuneTZ[k] > maxnz) continue;  // same shapes as a smaller candidate
-                for (int i : c.inst)
-                    if ((rc = set_tile_locked(ops[i], depth(ops[i], kTuneTZ[k])))) return rc;
-                if ((rc = time_batched_apply(ops, c.inst, bs, reps, &us[f][k]))) return rc;
-                if (best_k < 0 || us[f][k] < us[best_f][best_k]) {
+                for (size_t j = 0; j < c.inst.size(); ++j)
+                    if ((rc = set_tiles32(ops[c.inst[j]], tiles(ops[c.inst[j]], came[j], k).g))) return rc;
+                double t;
+                if ((rc = time_batched_apply(ops, c.inst, bs, reps, &t))) return rc;
+                // the tiles as they came are reported under the depth nearest the first member's
+                int r = k;
+                if (k < 0)
+                    for (r = 0; r + 1 < FG_TUNE_CANDIDATES && kTuneTZ[r + 1] <= maxnz &&
+                                2 * came[0].g[f].TZ >= 3 * kTuneTZ[r];) ++r;
+                us[f][r] = us[f][r] < 0 ? t : std::min(us[f][r], t);
+                if (best_f < 0 || t < best_us) {
+                    best_us = t;
                     best_f = f;
                     best_k = k;
                 }
@@ -2467,18 +2505,22 @@ FG_API int fg_batch_autotune(fg_op *const *ops, int n, int reps, fg_tune_entry *
         }
         int err;
         if (!set_format(c, best_f, err)) return err ? err : fail(FG_CUDA_ERROR, "autotune: format lost");
-        for (int i : c.inst) {
-            if ((rc = set_tile_locked(ops[i], depth(ops[i], kTuneTZ[best_k]))) || (rc = ensure_fp32(ops[i])))
-                return rc;
-            CK(cudaStreamSynchronize(ops[i]->stream));
+        for (size_t j = 0; j < c.inst.size(); ++j) {
+            fg_op *o = ops[c.inst[j]];
+            if ((rc = set_tiles32(o, tiles(o, came[j], best_k).g)) || (rc = ensure_fp32(o))) return rc;
+            if (best_k >= 0) o->limit_tz = depth(o, kTuneTZ[best_k]);
+            CK(cudaStreamSynchronize(o->stream));
         }
+        int best_r = 0;  // the reported candidate
+        for (int k = 1; k < FG_TUNE_CANDIDATES; ++k)
+            if (us[best_f][k] >= 0 && us[best_f][k] < us[best_f][best_r]) best_r = k;
         if (out && count < max_out) {
             fg_tune_entry &e = out[count];
             e.order = c.p;
             e.kind = c.kind;
             e.size_class = c.sc;
             e.instances = (int)c.inst.size();
-            e.tz = kTuneTZ[best_k];
+            e.tz = kTuneTZ[best_r];
             e.format = best_f;
             for (int k = 0; k < FG_TUNE_CANDIDATES; ++k) {
                 e.us[k] = us[best_f][k];
@@ -3090,7 +3132,7 @@ extern "C" FG_API int fg_op_apply_native_noalloc(fg_op *op, const double *x, dou
     // operator uses (choose_tile keeps the chosen one inside it)
     Grid w = g;
     set_scratch_tiling(w);
-    if (op->tile_set) set_depth(w, g.TZ);
+    if (op->limit_tz) set_depth(w, op->limit_tz);
     const size_t need = std::max((size_t)g.n_items() * (size_t)g.face_stride(),
                                  (size_t)w.n_items() * (size_t)w.face_stride());
     if (need > FG_NOALLOC_FACE_DOUBLES)

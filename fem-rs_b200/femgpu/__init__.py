@@ -379,7 +379,7 @@ class PAOperator:
 
     @property
     def tile(self):
-        """(32, WY, TZ): elements per apply work item in x, y, z."""
+        """(LX, WY, TZ): elements per work item of the FP64 apply in x (32 or 8), y, z."""
         d = (C.c_int * 3)()
         _check(lib().fg_op_tile(self._h, d))
         return tuple(d)
@@ -556,9 +556,9 @@ def batch_pcg(ops, bs, xs, cfg=None, precond=PC_CHEBYSHEV):
 
 
 def batch_autotune(ops, reps=5):
-    """Choose each batch class's quadrature-data format and item depth TZ by
-    timing the batched FP32 apply (fg_batch_autotune); the choice stays on the
-    operators.  Returns one dict per (order, kind, size class): ``format`` and
+    """Choose each batch class's quadrature-data format and the depth TZ of its FP32
+    items by timing the batched FP32 apply (fg_batch_autotune); the choice stays on
+    the operators, whose own FP32 tiles are a candidate too.  Returns one dict per (order, kind, size class): ``format`` and
     ``tz`` chosen, ``us`` the times per TZ in that format, ``us_other`` in the
     other format (None: not tried)."""
     n = len(ops)

@@ -390,10 +390,13 @@ typedef struct {
  * class); for each group every candidate (quadrature-data format, TZ) -- the
  * affine format only when every member's elements have constant Jacobians;
  * TZ clamped per instance to the largest power of two <= nz -- is applied to
- * all members, the group's batched FP32 apply (one launch + fix-up) is timed
- * over `reps` launches with CUDA events, and the fastest pair is kept on the
- * operators (the FP64 reliable-update applies of the mixed solve use the same
- * format).  Results per group in out[0 .. min(*n_out, max_out)). */
+ * the FP32 tiles of all members, the group's batched FP32 apply (one launch +
+ * fix-up) is timed over `reps` launches with CUDA events, and the fastest pair is
+ * kept on the operators.  The FP32 tiles that the operators came with are a candidate
+ * too (timed in both formats, reported under the TZ nearest the first member's
+ * depth) and are given back when they are the fastest; the FP64 tiles stay as they
+ * are (the FP64 reliable-update applies of the mixed solve use the same format).
+ * Results per group in out[0 .. min(*n_out, max_out)). */
 FG_API int fg_batch_autotune(fg_op *const *ops, int n, int reps, fg_tune_entry *out, int max_out,
                              int *n_out);
 
