@@ -689,10 +689,12 @@ static double item_rounds(int64_t xy, int nz, int TZ, int R, double S, double c)
 // lost, and the depth of the last item counts (item_rounds): 64^3 297 us at the 4 layers
 // of the rule before this one, 323 at the 16 that whole rounds ask for, 281 at 7.
 // The rule before this one took 32 lanes in x and halved the depth until there were
-// 592 items, which left a nearly empty last round or lane padding.  Over 2,900 random
-// meshes of 6 to 192 elements a side, all orders, kinds and forms, replayed from a
-// graph: 1.7 % above the best of 22 shapes on average (the old rule 12 %), on none
-// more than 9 % above the time of the old rule and the kernels of its time.
+// 592 items, which left a nearly empty last round of CTAs or lane padding.  Over 2,900
+// random meshes of 6 to 192 elements a side, all orders, kinds and forms, replayed from a
+// graph: 1.7 % above the best of 22 shapes on average (the old rule 12 %).  Against the old
+// rule and the kernels of its time, over 9,554 meshes: 13 % less time on average, on 47 more
+// than 5 % more, most of them Q1 FP32 full ones whose data just fit L2 and whose times move by
+// 10 % between runs of one tile.
 static void choose_tile(Grid &g, int kind, int fp32, int affine, int lanes, size_t face_limit) {
     // CTAs per SM by registers and shared memory, [lanes 32, 8][fp32][affine][kind][order]
     static const int resident[2][2][2][3][3] = {
